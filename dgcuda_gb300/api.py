@@ -296,7 +296,7 @@ def probe_reciprocal(x, device=0):
 
 def oz_table_image(p):
     """(words uint32[2240, 2], colexp int32[3, 16], dense float64[5, 16, 16])
-    of the tensor-core digit tables of order p: the digit words, the column
+    of the digit tables of order p: the digit words, the column
     exponents and the tables they were split from (host-built; no GPU
     needed)."""
     L = load_library()
@@ -498,8 +498,9 @@ class Solver:
 
     @property
     def tensor_contractions(self):
-        """True when the fused element stage runs its contractions on the
-        tensor cores (Euler, p = 1..4; on by default from p = 2)."""
+        """True when the Euler element stage computes its contractions as exact
+        integer slices (p = 1..4; on by default from p = 2; the other
+        equations always do at these orders)."""
         v = np.zeros(1, dtype=np.int32)
         _check(self._L.dg_get_tensor_contractions(self._h, _iptr(v)))
         return bool(v[0])
@@ -590,7 +591,7 @@ class Solver:
     def autotune_stage(self):
         """(block size, threads per element): the stage kernels' block size
         and, where the solver has both, the element stage (1: FP64 FMAs, one
-        thread per element; 2: tensor cores, a lane quad per two elements),
+        thread per element; 2: fixed point, one thread per element and variable),
         chosen by timing SSP-RK3 steps; the state is restored."""
         b, tpe = C.c_int(), C.c_int()
         _check(self._L.dg_autotune_stage(self._h, C.byref(b), C.byref(tpe)))

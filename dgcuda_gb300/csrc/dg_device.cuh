@@ -140,6 +140,21 @@ __device__ __forceinline__ float f32_of_hi(double x) {
   return __uint_as_float(ex == 0u ? (hi & 0x80000000u) : ex - 897u < 253u ? b : 0x7FC00000u);
 }
 
+// true only if the Euler state U (rho, m_x, m_y, E) is physical, from the
+// high words alone.  As an integer the high word of 2^k (1 + f) is 2^20 (k +
+// 1023 + f), and k + f <= log2 <= k + f + 0.0861: with L the high words and
+// L_m the larger one of |m_x|, |m_y|, L_rho + L_E > 2 L_m + 0.18 proves rho E
+// > max(m_x^2, m_y^2) by a margin of 2^0.007, hence 2 rho E > |m|^2 with far
+// more room than the FP64 test's rounding needs.  rho and E must be positive
+// and normal; an infinite or NaN rho or E passes, as the FP64 test passes it.
+// Eight integer instructions; false means "not settled here"
+__device__ __forceinline__ bool physical_log(const double *U) {
+  const int r = __double2hiint(U[0]), E = __double2hiint(U[3]);
+  const unsigned m = (unsigned)max(__double2hiint(U[1]) & 0x7FFFFFFF,
+                                   __double2hiint(U[2]) & 0x7FFFFFFF);
+  return min(r, E) >= 0x00100000 && (unsigned)r + (unsigned)E > 2u * m + 188744u;
+}
+
 // true only if the Euler state U (rho, m_x, m_y, E) is physical (rho >= 0,
 // 2 rho E >= |m|^2): with rho > 0 and a = 2 rho E in the normal range, a
 // and b = |m|^2 formed in single precision from 20-bit copies are each
@@ -336,6 +351,7 @@ struct Advection {  // advection/advection.cu
   static constexpr int N = 1;
   static constexpr bool kBathymetry = false;
   // the velocity may vary in space (q.field): fluxes then take the position
+  static constexpr bool kFusedLimiter = false;  // the limiter in the element epilogue
   static constexpr bool kField = true;
   static constexpr bool kFolded = false;
   DG_HD static bool physical(const EqP &, const double *) { return true; }
@@ -385,6 +401,7 @@ struct Advection {  // advection/advection.cu
 struct Euler {  // euler/euler.cu
   static constexpr int N = 4;
   static constexpr bool kBathymetry = false;
+  static constexpr bool kFusedLimiter = true;  // the limiter in the element epilogue
   static constexpr bool kField = false;
   // rho >= 0 and p >= 0 (is_physical, euler.cu:76-86); with rho > 0,
   // p < 0 <=> 2 rho E < |rho u|^2, which needs no FP64 division.  On the
@@ -397,7 +414,7 @@ struct Euler {  // euler/euler.cu
   }
   DG_HD static bool physical(const EqP &, const double *U) {
 #ifdef __CUDA_ARCH__
-    if (physical_f32(U)) return true;
+    if (physical_log(U) || physical_f32(U)) return true;
 #endif
     return physical_fp64(U);
   }
@@ -419,7 +436,7 @@ struct Euler {  // euler/euler.cu
   // the physical flux folded with the element metric, g = F . (ys, -xs) and
   // h = F . (-yr, xr), the two integrands of the volume term (eval_volume,
   // conserv_kernels.cu:1066-1074), formed from the momentum components
-  // along those directions without F_x and F_y: 26 FP64 operations where
+  // along those directions without F_x and F_y: 24 FP64 operations where
   // the flux and the fold take 33
   static constexpr bool kFolded = true;
   DG_HD static void flux_folded(const EqP &q, const double *U, double xr, double yr, double xs,
@@ -428,16 +445,17 @@ struct Euler {  // euler/euler.cu
     const double ma = fma(U[1], ys, -U[2] * xs), mb = fma(U[2], xr, -U[1] * yr);
     const double ua = ma * ir, ub = mb * ir;
     const double m2 = fma(U[1], U[1], U[2] * U[2]);
-    // p is reused as an addend: round it explicitly (never fused into an FMA)
-    const double p = mul_rn(q.gamma - 1., fma(-0.5 * m2, ir, U[3]));
-    const double H = U[3] + p;
+    // k = |m|^2/rho - 2E = -2 p / (gamma - 1): with k2 = (1 - gamma)/2, p = k2 k
+    // enters through the products k2 ys, k2 xs, ... formed once per element
+    const double k2 = 0.5 * (1. - q.gamma), k = fma(m2, ir, -2.0 * U[3]);
+    const double H = fma(k2, k, U[3]);
     g[0] = ma;
-    g[1] = fma(U[1], ua, p * ys);
-    g[2] = fma(U[2], ua, -p * xs);
+    g[1] = fma(U[1], ua, k * (k2 * ys));
+    g[2] = fma(U[2], ua, -k * (k2 * xs));
     g[3] = H * ua;
     h[0] = mb;
-    h[1] = fma(U[1], ub, -p * yr);
-    h[2] = fma(U[2], ub, p * xr);
+    h[1] = fma(U[1], ub, -k * (k2 * yr));
+    h[2] = fma(U[2], ub, k * (k2 * xr));
     h[3] = H * ub;
   }
   // local Lax-Friedrichs (euler.cu:170-237)
@@ -501,6 +519,7 @@ struct Euler {  // euler/euler.cu
 struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
   static constexpr int N = 3;
   static constexpr bool kBathymetry = true;  // optional bed b(x, y): source -g h grad b
+  static constexpr bool kFusedLimiter = false;  // the limiter in the element epilogue
   static constexpr bool kField = false;
   static constexpr bool kFolded = false;
   DG_HD static bool physical(const EqP &, const double *U) { return U[0] >= 0.; }
@@ -547,6 +566,7 @@ struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
 struct Maxwell {  // maxwells/maxwells.cu, U = (Hx, Hy, Ez)
   static constexpr int N = 3;
   static constexpr bool kBathymetry = false;
+  static constexpr bool kFusedLimiter = false;  // the limiter in the element epilogue
   static constexpr bool kField = false;
   static constexpr bool kFolded = false;
   DG_HD static bool physical(const EqP &, const double *) { return true; }

@@ -1,0 +1,89 @@
+// dg_fixed.cu -- host side of the fixed-point contractions: the limb tables
+// of the element stage's basis tables.
+#include <cmath>
+#include <cstring>
+
+#include "dg_fixed.cuh"
+
+namespace dg {
+namespace fx {
+namespace {
+
+int host_bexp(double x) {
+  unsigned long long b;
+  std::memcpy(&b, &x, 8);
+  return (int)((b >> 52) & 0x7FF);
+}
+
+// t in units of 2^(M - 1078), M the table's largest biased exponent: a
+// signed integer below 2^56, as h 2^28 + l with l in [-2^27, 2^27)
+Limb limb(double t, int M) {
+  const long long T = std::llrint(std::ldexp(t, 1078 - M));
+  Limb r;
+  r.h = (int)((T + (1ll << (kLow - 1))) >> kLow);
+  r.l = (int)(T - ((long long)r.h << kLow));
+  return r;
+}
+
+template <int P>
+void build(const Tab<P> &t, FxTab<P> *o) {
+  constexpr int NP = Tab<P>::NP, NQ = Tab<P>::NQ, N1 = Tab<P>::N1, NF = 3 * N1;
+  int mB = 1, mG = 1, mE = 1;
+  for (int q = 0; q < NQ; q++)
+    for (int i = 0; i < NP; i++) {
+      mB = std::max(mB, host_bexp(t.B[q][i]));
+      mG = std::max(mG, std::max(host_bexp(t.GR[q][i]), host_bexp(t.GS[q][i])));
+    }
+  for (int k = 0; k < NF; k++)
+    for (int i = 0; i < NP; i++) mE = std::max(mE, host_bexp(t.E[k / N1][k % N1][i]));
+  o->eB = mB;
+  o->eP = std::max(mB, std::max(mG, mE));
+  o->eE = mE;
+  o->c0 = 1;
+  for (int q = 1; q < NQ; q++)
+    if (t.B[q][0] != t.B[0][0]) o->c0 = 0;
+  for (int q = 0; q < NQ; q++) {
+    for (int i = 0; i < NP; i++) {
+      o->B[q][i] = limb(t.B[q][i], o->eB);
+      o->G[q][0][i] = limb(t.GR[q][i], o->eP);
+      o->G[q][1][i] = limb(t.GS[q][i], o->eP);
+      o->Q[q][i] = limb(t.B[q][i], o->eP);
+    }
+    o->r[q] = t.r[q];
+    o->s[q] = t.s[q];
+    o->B0[q] = t.B[q][0];
+  }
+  for (int k = 0; k < NF; k++) {
+    const double *E = t.E[k / N1][k % N1];
+    for (int i = 0; i < NP; i++) {
+      o->S[k][i] = limb(E[i], o->eP);
+      o->E[k][i] = limb(E[i], o->eE);
+    }
+  }
+  o->phi0 = t.B[0][0];
+  o->e0 = t.E[0][0][0];
+}
+
+}  // namespace
+}  // namespace fx
+
+size_t fx_tab_bytes(int p) {
+  switch (p) {
+    case 1: return sizeof(fx::FxTab<1>);
+    case 2: return sizeof(fx::FxTab<2>);
+    case 3: return sizeof(fx::FxTab<3>);
+    case 4: return sizeof(fx::FxTab<4>);
+  }
+  return 0;
+}
+
+void build_fx_tab(int p, const void *tabimg, void *out) {
+  switch (p) {
+    case 1: fx::build(*static_cast<const Tab<1> *>(tabimg), static_cast<fx::FxTab<1> *>(out)); break;
+    case 2: fx::build(*static_cast<const Tab<2> *>(tabimg), static_cast<fx::FxTab<2> *>(out)); break;
+    case 3: fx::build(*static_cast<const Tab<3> *>(tabimg), static_cast<fx::FxTab<3> *>(out)); break;
+    case 4: fx::build(*static_cast<const Tab<4> *>(tabimg), static_cast<fx::FxTab<4> *>(out)); break;
+  }
+}
+
+}  // namespace dg

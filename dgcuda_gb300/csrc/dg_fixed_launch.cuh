@@ -1,0 +1,78 @@
+// dg_fixed_launch.cuh -- launchers of the fixed-point element stage and
+// traces (dg_fixed.cuh), p = 1..4; each equation is instantiated in a
+// translation unit of its own (dg_fixed_<equation>.cu).
+#pragma once
+#include "dg_fixed.cuh"
+
+namespace dg {
+namespace fx {
+
+template <class Eq, int P>
+void run_element(const Ctx &c, const ElemArgs &a, int mode) {
+  using S = Shape<Eq, P>;
+  const FxTab<P> &tab = *static_cast<const FxTab<P> *>(c.fx);
+  const unsigned blocks = nblk(c.m.K, kTile);
+  if (mode == 0) {
+    k_element_fx<Eq, P, 0><<<blocks, S::kThreads, 0, c.st>>>(tab, *c.q, a);
+  } else if (mode == 1) {
+    k_element_fx<Eq, P, 1><<<blocks, S::kThreads, 0, c.st>>>(tab, *c.q, a);
+  } else {
+    if constexpr (Eq::kFusedLimiter)
+      k_element_fx<Eq, P, 2><<<blocks, S::kThreads, 0, c.st>>>(tab, *c.q, a);
+  }
+}
+
+template <class Eq, int P>
+void run_trace(const Ctx &c, double *u) {
+  k_trace_fx<Eq, P><<<nblk(c.m.K, kTile), Shape<Eq, P>::kThreads, 0, c.st>>>(
+      *static_cast<const FxTab<P> *>(c.fx), *c.q, u, c.T, c.m.K, c.m.Kp);
+}
+
+template <class Eq>
+void element(const Ctx &c, const ElemArgs &a, int mode) {
+  switch (c.p) {
+    case 1: run_element<Eq, 1>(c, a, mode); break;
+    case 2: run_element<Eq, 2>(c, a, mode); break;
+    case 3: run_element<Eq, 3>(c, a, mode); break;
+    case 4: run_element<Eq, 4>(c, a, mode); break;
+  }
+}
+
+template <class Eq>
+void trace(const Ctx &c, double *u) {
+  switch (c.p) {
+    case 1: run_trace<Eq, 1>(c, u); break;
+    case 2: run_trace<Eq, 2>(c, u); break;
+    case 3: run_trace<Eq, 3>(c, u); break;
+    case 4: run_trace<Eq, 4>(c, u); break;
+  }
+}
+
+// the element stage, and the start-of-run traces, of n blocks of blk elements
+// from block lo of a batch's map, all of order p
+template <class Eq, int P>
+void run_batch(const BatchLaunch &b, cudaStream_t st, int lo, int n, int blk, int stage,
+               int check) {
+  using S = Shape<Eq, P>;
+  const FxTab<P> &tab = *static_cast<const FxTab<P> *>(b.fx[P]);
+  const int sub = blk / kTile;
+  if (stage < 0)
+    k_trace_batch_fx<Eq, P><<<n * sub, S::kThreads, 0, st>>>(tab, b.probs, b.eblk2prob, b.eblk0,
+                                                             lo, sub);
+  else
+    k_element_batch_fx<Eq, P><<<n * sub, S::kThreads, 0, st>>>(
+        tab, b.probs, b.eblk2prob, b.eblk0, lo, sub, stage, check);
+}
+
+template <class Eq>
+void batch_element(const BatchLaunch &b, cudaStream_t st, int p, int lo, int n, int blk,
+                   int stage, int check) {
+  switch (p) {
+    case 1: run_batch<Eq, 1>(b, st, lo, n, blk, stage, check); break;
+    case 2: run_batch<Eq, 2>(b, st, lo, n, blk, stage, check); break;
+    case 3: run_batch<Eq, 3>(b, st, lo, n, blk, stage, check); break;
+  }
+}
+
+}  // namespace fx
+}  // namespace dg

@@ -26,7 +26,7 @@
 // writes the traces of its output as it stores it, so T always holds what
 // k_trace would have computed from the next stage's input.  With the limiter
 // on, the limiter runs on those traces: for Euler in the element kernel's own
-// epilogue (k_element<TR, LIM>, or k_element_oz<LIM> on the tensor path),
+// epilogue (k_element<TR, LIM>, or the fixed-point stage of dg_fixed.cuh),
 // with the neighbours' new cell means found before the element stage by
 // k_means from the per-side flux sums k_face<FS> leaves; for the other
 // equations as the pass k_limit_tr.  Either way a limited element's traces
@@ -312,12 +312,14 @@ struct ElemArgs {
   const double *geo;        // metric
   const double *dtp;        // time step
   const double *bathy;      // bed modes [mode][Kp] (shallow water) or null
+  const double *bslope;     // its slopes at the area points (fixed-point stage) or null
   const double *vtx;        // element vertices (rows of Kp): positions for a velocity field
   double *T;                // traces of out (TR)
   const double *M;          // fused limiter: the means of out (k_means), rows of Kp
   const int *nbr;           // fused limiter: neighbours across faces 0..2, rows of Kp
   double ca, cb, cc;
   int K, Kp, check;
+  int has_un, unit_cb;      // ca != 0; cb == 1
 };
 
 // TR: also write the edge traces of `out` into T (what k_trace would compute
@@ -446,6 +448,36 @@ __global__ void __launch_bounds__(kMaxBlock) k_element(const __grid_constant__ T
                                                        const __grid_constant__ ElemArgs a) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < a.K) element_body<Eq, P, TR, LIM>(tab, q, a, e);
+}
+
+// ---------------------------------------------------------------------------
+// The bed's slopes at the area points: volume()'s source per -g h, w J b_x in
+// rows 0..NQ-1 and w J b_y in rows NQ..2NQ-1 of Kp
+template <int P>
+__global__ void __launch_bounds__(kMaxBlock) k_bed_slopes(const __grid_constant__ Tab<P> tab,
+                                                          const double *__restrict__ bathy,
+                                                          const double *__restrict__ geo,
+                                                          double *__restrict__ out, int K,
+                                                          int Kp) {
+  constexpr int NP = Tab<P>::NP, NQ = Tab<P>::NQ;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= K) return;
+  double bz[NP];
+#pragma unroll
+  for (int i = 0; i < NP; i++) bz[i] = bathy[(size_t)i * Kp + e];
+  const double xr = geo[e], yr = geo[(size_t)Kp + e], xs = geo[2 * (size_t)Kp + e],
+               ys = geo[3 * (size_t)Kp + e];
+#pragma unroll
+  for (int k = 0; k < NQ; k++) {
+    double br = 0.0, bs = 0.0;
+#pragma unroll
+    for (int i = 1; i < NP; i++) {
+      br = fma(bz[i], tab.GR[k][i], br);
+      bs = fma(bz[i], tab.GS[k][i], bs);
+    }
+    out[(size_t)k * Kp + e] = fma(ys, br, -yr * bs);
+    out[(size_t)(NQ + k) * Kp + e] = fma(xr, bs, -xs * br);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -890,6 +922,7 @@ __device__ __forceinline__ ElemArgs batch_elem_args(const BatchProb &pr, int sta
   a.geo = pr.geo;
   a.dtp = &pr.ds->dt;
   a.bathy = pr.bathy;
+  a.bslope = pr.bslope;
   a.vtx = pr.vtx;
   a.T = pr.T;
   a.M = pr.M;
@@ -900,6 +933,8 @@ __device__ __forceinline__ ElemArgs batch_elem_args(const BatchProb &pr, int sta
   a.K = pr.K;
   a.Kp = pr.Kp;
   a.check = check;
+  a.has_un = stage != 0;
+  a.unit_cb = stage == 0;
   return a;
 }
 
@@ -1016,6 +1051,19 @@ __global__ void __launch_bounds__(kBlock)
 // ---------------------------------------------------------------------------
 // launchers: dispatch on p to the template instance
 // ---------------------------------------------------------------------------
+namespace fx {
+// the fixed-point element stage and traces (dg_fixed.cuh), where Ctx::fx
+// holds the tables
+template <class Eq>
+void element(const Ctx &c, const ElemArgs &a, int mode);
+template <class Eq>
+void trace(const Ctx &c, double *u);
+// of a batch's blocks of one order: the element stage, or with stage < 0 the
+// start-of-run traces
+template <class Eq>
+void batch_element(const BatchLaunch &b, cudaStream_t st, int p, int lo, int n, int blk,
+                   int stage, int check);
+}  // namespace fx
 inline unsigned nblk(int n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
 
 template <class Eq>
@@ -1035,6 +1083,11 @@ struct Launch {
     case 5: { constexpr int P = 5; expr; } break; \
   }
 
+  // orders whose FP64 traces and element stage are reachable: all of Euler's
+  // (its fixed-point stage can be switched off, and its batch contracts in
+  // FP64), elsewhere only those without a fixed-point stage
+  static constexpr bool fp64(int P) { return Eq::kFusedLimiter || P < 1 || P > 4; }
+
   static ElemArgs eargs(const Ctx &c, double *us, const double *un, double *out, double ca,
                         double cb, double cc, const double *dtp, double *T, int check) {
     ElemArgs a;
@@ -1046,6 +1099,7 @@ struct Launch {
     a.geo = c.m.geo;
     a.dtp = dtp;
     a.bathy = c.m.bathy;
+    a.bslope = c.m.bslope;
     a.vtx = c.m.vtx;
     a.T = T;
     a.M = c.M;
@@ -1056,13 +1110,17 @@ struct Launch {
     a.K = c.m.K;
     a.Kp = c.m.Kp;
     a.check = check;
+    a.has_un = ca != 0.0;
+    a.unit_cb = cb == 1.0;
     return a;
   }
 
   static void trace(const Ctx &c, double *u) {
     if (!c.m.K) return;
-    DG_DISPATCH_P((k_trace<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, u,
-                                                                          c.T, c.m.K, c.m.Kp)));
+    if (c.fx) return fx::trace<Eq>(c, u);
+    DG_DISPATCH_P(if constexpr (fp64(P)) (
+        k_trace<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, u, c.T, c.m.K,
+                                                               c.m.Kp)));
   }
   template <bool FS>
   static void face_args(const Ctx &c, const double *t, double tcoef, double *Fs) {
@@ -1104,8 +1162,9 @@ struct Launch {
                       double cb, double cc, const double *dtp) {
     if (!c.m.K) return;
     const ElemArgs a = eargs(c, us, un, out, ca, cb, cc, dtp, nullptr, 0);
-    DG_DISPATCH_P((k_element<Eq, P, false><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c),
-                                                                                   *c.q, a)));
+    if (c.fx) return fx::element<Eq>(c, a, 0);
+    DG_DISPATCH_P(if constexpr (fp64(P)) (
+        k_element<Eq, P, false><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, a)));
   }
   // element_tr() with the limiter in the epilogue (c.M holds the output's
   // means from k_means)
@@ -1113,6 +1172,7 @@ struct Launch {
                           double cb, double cc, const double *dtp) {
     if (!c.m.K) return;
     const ElemArgs a = eargs(c, us, un, out, ca, cb, cc, dtp, c.T, 0);
+    if (c.fx) return fx::element<Eq>(c, a, 2);
     DG_DISPATCH_P((k_element<Eq, P, true, true><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(
         tab<P>(c), *c.q, a)));
   }
@@ -1120,8 +1180,14 @@ struct Launch {
                          double cb, double cc, const double *dtp, int check) {
     if (!c.m.K) return;
     const ElemArgs a = eargs(c, us, un, out, ca, cb, cc, dtp, c.T, check);
-    DG_DISPATCH_P((k_element<Eq, P, true><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c),
-                                                                                  *c.q, a)));
+    if (c.fx) return fx::element<Eq>(c, a, 1);
+    DG_DISPATCH_P(if constexpr (fp64(P)) (
+        k_element<Eq, P, true><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, a)));
+  }
+  static void bed_slopes(const Ctx &c, double *out) {
+    if (!c.m.K) return;
+    DG_DISPATCH_P((k_bed_slopes<P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(
+        tab<P>(c), c.m.bathy, c.m.geo, out, c.m.K, c.m.Kp)));
   }
   static void limit_tr(const Ctx &c, double *u) {
     if (!c.m.K || c.p < 1) return;
@@ -1156,7 +1222,7 @@ struct Launch {
 
   static const Ops &ops() {
     static const Ops o = {trace,  face,       element,  limit,  lambda,  init,    l2err,
-                          element_tr, limit_tr, vertex, nullptr, nullptr, nullptr};
+                          element_tr, limit_tr, vertex, nullptr, nullptr, nullptr, nullptr};
     return o;
   }
 
@@ -1165,7 +1231,14 @@ struct Launch {
     return *reinterpret_cast<const BatchTabs *>(b.tabs);
   }
   static void b_trace(const BatchLaunch &b) {
-    k_trace_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0);
+    if constexpr (Eq::kFusedLimiter) {
+      k_trace_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0);
+    } else {
+      for (int g = 0; g < BatchLaunch::kGroups; g++) {
+        const int lo = b.eblk_g[g], n = b.eblk_g[g + 1] - lo;
+        if (n > 0) fx::batch_element<Eq>(b, b.st, 1 + g / 2, lo, n, b.blk_g[g], -1, 1);
+      }
+    }
   }
   static void b_face(const BatchLaunch &b, double tcoef) {
     k_face_batch<Eq><<<b.nsblk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.sblk2prob, b.sblk0,
@@ -1186,15 +1259,18 @@ struct Launch {
       const cudaStream_t st = side ? b.gst[g] : b.st;
       first = false;
       if (side) cudaStreamWaitEvent(st, b.fork, 0);
-      if (p == 1)
+      if constexpr (!Eq::kFusedLimiter) {
+        fx::batch_element<Eq>(b, st, p, lo, n, blk, stage, check);
+      } else if (p == 1) {
         k_element_batch_p<Eq, 1, LIM><<<n, blk, 0, st>>>(tb.t1, b.probs, b.eblk2prob, b.eblk0,
                                                            lo, stage, check);
-      else if (p == 2)
+      } else if (p == 2) {
         k_element_batch_p<Eq, 2, LIM><<<n, blk, 0, st>>>(tb.t2, b.probs, b.eblk2prob, b.eblk0,
                                                            lo, stage, check);
-      else
+      } else {
         k_element_batch_p<Eq, 3, LIM><<<n, blk, 0, st>>>(tb.t3, b.probs, b.eblk2prob, b.eblk0,
                                                            lo, stage, check);
+      }
       if (side) {
         cudaEventRecord(b.join[g], st);
         cudaStreamWaitEvent(b.st, b.join[g], 0);

@@ -2,6 +2,13 @@
 #include "dg_kernels.cuh"
 
 namespace dg {
-const Ops &ops_shallow_water() { return Launch<ShallowWater>::ops(); }
+const Ops &ops_shallow_water() {
+  static const Ops o = [] {
+    Ops v = Launch<ShallowWater>::ops();
+    v.bed_slopes = Launch<ShallowWater>::bed_slopes;
+    return v;
+  }();
+  return o;
+}
 const BatchOps &batch_ops_shallow_water() { return Launch<ShallowWater>::batch_ops(); }
 }  // namespace dg

@@ -38,6 +38,7 @@ struct DevMesh {
   double *bxy = nullptr;  // 4 rows of Sb: start and end vertex of the left face (boundary sides)
   int *perm = nullptr;    // K: internal index -> caller's (.pmsh) index
   double *bathy = nullptr; // shallow water bed modes [mode][Kp], null = flat
+  double *bslope = nullptr; // its slopes at the area points (fixed-point stage), rows of Kp
 };
 
 // device scalars used by graph-captured steps
@@ -68,7 +69,7 @@ struct Ctx {
   double *Fs = nullptr;           // per-side sums of Fh over the edge points [side][var]
   double *M = nullptr;            // means of the stage output [var][Kp] (fused limiter)
   DevScalars *ds = nullptr;       // device scalars
-  const void *oz = nullptr;       // tensor-core tables of order p (null: FP64 contractions)
+  const void *fx = nullptr;       // host FxTab<p> image (null: FP64 contractions)
 };
 
 // one problem of a batched ensemble (device resident)
@@ -79,7 +80,7 @@ struct BatchProb {
   const double *geo;
   const int *esd, *nbr;
   const int4 *side;
-  const double *sgeo, *bxy, *bathy;
+  const double *sgeo, *bxy, *bathy, *bslope;
   const double *vtx;
   DevScalars *ds;
   EqP q;
@@ -88,6 +89,9 @@ struct BatchProb {
 struct BatchLaunch {
   cudaStream_t st = nullptr;
   const void *tabs = nullptr;       // BatchTabs image (Tab<1>, Tab<2>, Tab<3>)
+  // host FxTab<p> images of p = 1..3 where the members' own steps contract in
+  // fixed point (null: FP64, as the Euler batch)
+  const void *fx[4] = {nullptr, nullptr, nullptr, nullptr};
   BatchProb *probs = nullptr;       // device array
   int nprob = 0, blk = 128, limiter = 0;
   int fused = 0;  // limiter in the element epilogue (face_fs, means, element_lim)
@@ -168,15 +172,17 @@ struct Ops {
                 const double *dtp);
   void (*element_lim)(const Ctx &, double *us, const double *un, double *out, double ca,
                       double cb, double cc, const double *dtp);
+  // slopes of the bed c.m.bathy at the area points into rows of Kp (null where
+  // an equation has no bed): w J times the source per -g h, x then y
+  void (*bed_slopes)(const Ctx &, double *out);
 };
 
 const Ops &ops_advection();
 const Ops &ops_euler();
-// tensor-core element stage (Euler, p = 1..4): table image size, builder
-// from the host Tab<p> image, and the per-device kernel attribute
-size_t oz_tabs_bytes();
-bool oz_build_tabs(int p, const void *tabimg, void *out, double *dense = nullptr);
-cudaError_t oz_prepare_euler(int p);
+// fixed-point element stage (p = 1..4): table image size and builder from the
+// host Tab<p> image
+size_t fx_tab_bytes(int p);
+void build_fx_tab(int p, const void *tabimg, void *out);
 const Ops &ops_shallow_water();
 const Ops &ops_maxwell();
 

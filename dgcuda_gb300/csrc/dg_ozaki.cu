@@ -1,5 +1,5 @@
-// dg_ozaki.cu -- host side of the tensor-core contractions: the f16 digit
-// words and column exponents of the element kernel's four basis tables.
+// dg_ozaki.cu -- the f16 digit words and column exponents of the basis tables
+// (dg_ozaki.cuh).
 #include <cstring>
 #include <vector>
 
@@ -102,9 +102,7 @@ void build_tabs(const Tab<P> &tb, Tabs *out, double *dense) {
 
 }  // namespace oz
 
-size_t oz_tabs_bytes() { return sizeof(oz::Tabs); }
-
-bool oz_build_tabs(int p, const void *tabimg, void *out, double *dense) {
+static bool oz_build_tabs(int p, const void *tabimg, void *out, double *dense) {
   oz::Tabs *o = static_cast<oz::Tabs *>(out);
   switch (p) {
     case 1: oz::build_tabs<1>(*static_cast<const Tab<1> *>(tabimg), o, dense); return true;

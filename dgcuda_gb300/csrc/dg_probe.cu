@@ -40,7 +40,7 @@ __global__ void k_physical(const double *U, int *fast, int *exact, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     const double *u = U + 4 * (size_t)i;
-    fast[i] = dg::physical_f32(u) ? 1 : 0;
+    fast[i] = dg::physical_log(u) || dg::physical_f32(u) ? 1 : 0;
     exact[i] = dg::Euler::physical_fp64(u) ? 1 : 0;
   }
 }

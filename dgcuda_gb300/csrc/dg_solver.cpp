@@ -40,7 +40,7 @@ struct dg_solver {
   dg_params prm{};
   dg::EqP q{};
   dg_order_tables tables{};
-  std::vector<char> tabimg;
+  std::vector<char> tabimg, fximg;  // Tab<p>; FxTab<p> (p = 1..4)
   dg::DevMesh m;
   dg::Ctx ctx;
   const dg::Ops *ops = nullptr;
@@ -48,15 +48,15 @@ struct dg_solver {
   double *ubuf = nullptr, *partial = nullptr, *T = nullptr, *Fh = nullptr, *vbuf = nullptr;
   double *Fs = nullptr, *M = nullptr;  // side-flux sums and output means (fused limiter)
   double *bathy = nullptr;        // bed modes (shallow water), internal order
+  double *bslope = nullptr;       // bed slopes at the area points (fixed-point stage)
   double *lin_tv = nullptr, *lin_f0 = nullptr, *lin_f1 = nullptr;  // adjoint work
   bool has_inout_bc = false;      // a side with an inflow or outflow code
-  void *oz = nullptr;             // tensor-core tables (Euler, p = 1..4)
   int *flag = nullptr;            // device flag of put_state
   // host transfers of the state: a copy stream and one event per chunk of
   // rows, so that the permutation of one chunk overlaps the copy of the next
   cudaStream_t cst = nullptr;
   std::vector<cudaEvent_t> cev;
-  bool tensor = true;             // use them in the fused element stage
+  bool tensor = true;             // Euler: fixed-point contractions (dg_set_tensor_contractions)
   // T holds the traces of U as the last fused SSP-RK3 stage left them (and U
   // is already limited): the next dg_step continues without recomputing
   // them, so a run split over several calls is the uninterrupted run
@@ -160,19 +160,14 @@ void collect_profile(dg_solver *s) {
 
 enum { K_TRACE = 0, K_FACE = 1, K_ELEMENT = 2, K_LIMIT = 3, K_CFL = 4, K_RK = 5, K_MEANS = 6 };
 
-// one RK stage of the DG operator: out = ca*un + cb*us + cc*dt*L(us).
-// With the tensor-core contractions on, the element stage is the one the
-// fused SSP-RK3 step runs (k_element_oz; the traces of `out` it also leaves
-// in T are not used, and no positivity rule is applied to them), so dg_rhs
-// and the RK4 / RK2 loops evaluate the operator the SSP-RK3 step evaluates.
+// one RK stage of the DG operator: out = ca*un + cb*us + cc*dt*L(us), by the
+// element stage the SSP-RK3 step runs without the traces it leaves, so dg_rhs
+// and the RK4 / RK2 loops evaluate the operator the SSP-RK3 step evaluates
 void stage(dg_solver *s, double *us, const double *un, double *out, double ca, double cb,
            double cc, double tcoef, const double *dtp) {
   run(s, K_TRACE, [&] { s->ops->trace(s->ctx, us); });
   run(s, K_FACE, [&] { s->ops->face(s->ctx, &s->ds->t, tcoef); });
-  if (s->ctx.oz)
-    run(s, K_ELEMENT, [&] { s->ops->element_tr(s->ctx, us, un, out, ca, cb, cc, dtp, 0); });
-  else
-    run(s, K_ELEMENT, [&] { s->ops->element(s->ctx, us, un, out, ca, cb, cc, dtp); });
+  run(s, K_ELEMENT, [&] { s->ops->element(s->ctx, us, un, out, ca, cb, cc, dtp); });
 }
 
 void limit(dg_solver *s, double *u) {
@@ -286,25 +281,21 @@ void drop_graphs(dg_solver *s) {
   s->graph_launches.clear();
 }
 
-// (re)builds the tensor-core tables from the current basis tables and
-// points the fused element stage at them (or back at the FP64 kernel)
-dg_status oz_refresh(dg_solver *s) {
-  s->ctx.oz = nullptr;
-  if (s->eq != DG_EULER || s->p < 1 || s->p > 4) return DG_OK;
-  // at p = 1 (3 modes, 3 area points) the FP64 kernel is the faster one:
-  // the tensor path is built but off until asked for
-  if (!s->oz) s->tensor = s->p >= 2;
-  std::vector<char> img(dg::oz_tabs_bytes());
-  if (!dg::oz_build_tabs(s->p, s->tabimg.data(), img.data()))
-    return fail(DG_UNSUPPORTED, "no tensor-core tables for this order");
-  if (!s->oz) {
-    dg_status st = dalloc(s, reinterpret_cast<char **>(&s->oz), img.size());
-    if (st != DG_OK) return st;
-    CK(dg::oz_prepare_euler(s->p));
-  }
-  CK(cudaMemcpy(s->oz, img.data(), img.size(), cudaMemcpyHostToDevice));
-  if (s->tensor) s->ctx.oz = s->oz;
-  return DG_OK;
+// the element stage's contractions: fixed point at p = 1..4, for Euler only
+// where it is switched on
+void fx_select(dg_solver *s) {
+  const bool on = !s->fximg.empty() && (s->eq != DG_EULER || s->tensor);
+  s->ctx.fx = on ? s->fximg.data() : nullptr;
+}
+
+// (re)builds the fixed-point tables from the current basis tables and points
+// the element stage at them where it uses them
+void fx_refresh(dg_solver *s) {
+  s->ctx.fx = nullptr;
+  s->fximg.resize(dg::fx_tab_bytes(s->p));
+  if (s->fximg.empty()) return;
+  dg::build_fx_tab(s->p, s->tabimg.data(), s->fximg.data());
+  fx_select(s);
 }
 
 dg_status get_graph(dg_solver *s, int scheme, cudaGraphExec_t *out) {
@@ -643,8 +634,8 @@ extern "C" dg_status dg_solver_create(const dg_mesh *mesh, dg_equation eq, int p
   c.Fs = s->Fs;
   c.M = s->M;
   c.ds = s->ds;
-  dg_status ozs = oz_refresh(s);
-  if (ozs != DG_OK) return bail(ozs);
+  s->tensor = p >= 2;
+  fx_refresh(s);
   *out = s;
   return DG_OK;
 }
@@ -677,6 +668,23 @@ extern "C" dg_status dg_solver_sizes(const dg_solver *s, int *N, int *n_p, int *
 }
 
 extern "C" void *dg_solver_stream(dg_solver *s) { return s ? (void *)s->st : nullptr; }
+
+// ---- shallow-water bed ---------------------------------------------------
+// the bed's slopes at the area points, which the fixed-point stage reads in
+// place of the bed's modes (they change only with the bed and the tables)
+static dg_status set_bed_slopes(dg_solver *s) {
+  s->m.bslope = nullptr;
+  if (s->m.bathy && s->ctx.fx) {
+    if (!s->bslope) {
+      dg_status st = dalloc(s, &s->bslope, (size_t)2 * dg::nq_of(s->p) * s->m.Kp);
+      if (st != DG_OK) return st;
+    }
+    s->ops->bed_slopes(s->ctx, s->bslope);
+    s->m.bslope = s->bslope;
+  }
+  s->ctx.m.bslope = s->m.bslope;
+  return sync_check(s);
+}
 
 extern "C" dg_status dg_solver_set_tables(dg_solver *s, int n_q, int n_1, const double *basis,
                                           const double *grad_x, const double *grad_y,
@@ -724,10 +732,8 @@ extern "C" dg_status dg_solver_set_tables(dg_solver *s, int n_q, int n_1, const 
   dg::build_tab(s->p, s->tables, s->tabimg.data());
   field_refresh(s);
   drop_graphs(s);
-  {
-    dg_status ozs = oz_refresh(s);
-    if (ozs != DG_OK) return ozs;
-  }
+  fx_refresh(s);
+  if (s->bathy && s->m.bathy) return set_bed_slopes(s);
   return DG_OK;
 }
 
@@ -957,7 +963,6 @@ extern "C" dg_status dg_l2_error(dg_solver *s, double t, double *err) {
   return DG_OK;
 }
 
-// ---- shallow-water bed ---------------------------------------------------
 extern "C" dg_status dg_set_bathymetry(dg_solver *s, const double *b) {
   if (!s) return fail(DG_BAD_ARG, "null solver");
   s->tr_valid = false;
@@ -977,7 +982,7 @@ extern "C" dg_status dg_set_bathymetry(dg_solver *s, const double *b) {
   }
   s->ctx.m.bathy = s->m.bathy;
   drop_graphs(s);
-  return sync_check(s);
+  return set_bed_slopes(s);
 }
 
 extern "C" dg_status dg_get_bathymetry(dg_solver *s, double *b) {
@@ -1079,14 +1084,15 @@ extern "C" dg_status dg_autotune_stage(dg_solver *s, int *block, int *threads_pe
   double *save = nullptr;
   CK(cudaMalloc(&save, s->ndof_p * sizeof(double)));
   CK(cudaMemcpyAsync(save, s->U, s->ndof_p * sizeof(double), cudaMemcpyDeviceToDevice, s->st));
-  std::vector<int> variants;  // 1: the FP64 element stage, 2: the tensor-core one
-  if (threads_per_element && s->oz) variants = {1, 2};
-  else variants = {s->ctx.oz ? 2 : 1};
+  std::vector<int> variants;  // 1: the FP64 element stage, 2: the fixed-point one
+  const bool two = s->eq == DG_EULER && !s->fximg.empty();
+  if (threads_per_element && two) variants = {1, 2};
+  else variants = {two && s->tensor ? 2 : 1};
   int best_blk = s->ctx.blk, best_v = variants[0];
   float best_ms = 1e30f;
   for (int v : variants) {
-    s->tensor = v == 2;
-    s->ctx.oz = s->tensor ? s->oz : nullptr;
+    if (two) s->tensor = v == 2;
+    fx_select(s);
     int blk = s->ctx.blk;
     float ms = 0;
     dg_status st = tune_blocks(s, save, &blk, &ms);
@@ -1103,8 +1109,8 @@ extern "C" dg_status dg_autotune_stage(dg_solver *s, int *block, int *threads_pe
   }
   cudaStreamSynchronize(s->st);
   cudaFree(save);
-  s->tensor = best_v == 2;
-  s->ctx.oz = s->tensor ? s->oz : nullptr;
+  if (two) s->tensor = best_v == 2;
+  fx_select(s);
   s->ctx.blk = best_blk;
   drop_graphs(s);
   if (block) *block = best_blk;
@@ -1119,7 +1125,7 @@ struct dg_batch {
   dg_equation eq = DG_SHALLOW_WATER;
   cudaStream_t st = nullptr;
   const dg::BatchOps *ops = nullptr;
-  std::vector<char> tabs;
+  std::vector<char> tabs, fximg[4];
   dg::BatchProb *probs = nullptr;
   int *maps = nullptr;  // device: element/side/lambda block maps
   dg::BatchLaunch bl;
@@ -1318,6 +1324,21 @@ extern "C" dg_status dg_batch_create(int n, dg_solver *const *members, dg_batch 
   b->ops = batch_ops_for(b->eq);
   b->tabs.resize(dg::batch_tabs_bytes());
   dg::build_batch_tabs(timg[1], timg[2], timg[3], b->tabs.data());
+  // members that contract in fixed point (every equation but Euler, whose
+  // batch contracts in FP64): the default tables or the first member's of
+  // each order, as the FP64 tables above
+  if (b->eq != DG_EULER)
+    for (int p = 1; p <= 3; p++) {
+      b->fximg[p].resize(dg::fx_tab_bytes(p));
+      if (!timg[p]) {
+        std::vector<char> t(dg::tab_bytes(p));
+        dg::build_tab(p, DG_TABLES[p], t.data());
+        dg::build_fx_tab(p, t.data(), b->fximg[p].data());
+      } else {
+        dg::build_fx_tab(p, timg[p], b->fximg[p].data());
+      }
+      b->bl.fx[p] = b->fximg[p].data();
+    }
   std::vector<dg::BatchProb> hp(n);
   for (int i = 0; i < n; i++) {
     dg_solver *s = b->m[i];
@@ -1341,6 +1362,7 @@ extern "C" dg_status dg_batch_create(int n, dg_solver *const *members, dg_batch 
     q.sgeo = s->m.sgeo;
     q.bxy = s->m.bxy;
     q.bathy = s->m.bathy;
+    q.bslope = s->m.bslope;
     q.vtx = s->m.vtx;
     q.ds = s->ds;
     q.q = s->q;
@@ -2113,23 +2135,24 @@ extern "C" dg_status dg_load_checkpoint(dg_solver *s, const char *path, double *
   return DG_OK;
 }
 
-// the fused element stage's basis contractions on the tensor cores (exact
-// slices, FP64 accuracy) or in FP64 FMAs; Euler p = 1..4 have the former
+// the Euler element stage's basis contractions in fixed point (dg_fixed.cuh) or
+// in FP64 FMAs, p = 1..4
 extern "C" dg_status dg_set_tensor_contractions(dg_solver *s, int on) {
   if (!s) return fail(DG_BAD_ARG, "null solver");
   s->tr_valid = false;
-  if (on && !s->oz) return fail(DG_UNSUPPORTED, "tensor-core contractions are for Euler, p = 1..4");
+  if (on && (s->eq != DG_EULER || s->fximg.empty()))
+    return fail(DG_UNSUPPORTED, "exact-slice contractions are switched for Euler, p = 1..4");
   CK(cudaSetDevice(s->device));
   CK(cudaStreamSynchronize(s->st));
   s->tensor = on != 0;
-  s->ctx.oz = s->tensor ? s->oz : nullptr;
+  fx_select(s);
   drop_graphs(s);
   return DG_OK;
 }
 
 extern "C" dg_status dg_get_tensor_contractions(dg_solver *s, int *on) {
   if (!s || !on) return fail(DG_BAD_ARG, "null argument");
-  *on = s->ctx.oz != nullptr;
+  *on = s->eq == DG_EULER && s->ctx.fx != nullptr;
   return DG_OK;
 }
 

@@ -223,15 +223,16 @@ dg_status dg_get_velocity_field(const dg_solver *s, double out[7]);
 dg_status dg_set_inflow_series(dg_solver *s, int n, const double *amp, const double *omega,
                                const double *phase, double t0);
 
-/* The fused SSP-RK3 element stage computes its basis contractions (area
- * values, volume and surface projections, next-stage traces) either with
- * FP64 FMAs or on the tensor cores as exact integer slices (Ozaki-style
- * FP64 emulation; per-output error of the order of an FP64 dot product's
- * rounding).  The tensor path exists for Euler at p = 1..4 and is on by
- * default at p = 2..4 (at p = 1 the FP64 kernel is faster); DG_UNSUPPORTED
- * elsewhere.  No reference counterpart. */
+/* The element stage computes its basis contractions (area values, volume
+ * and surface projections, next-stage traces) at p = 1..4 as exact integer
+ * slices off the FP64 pipe (56-bit fixed point, per-output error below an
+ * FP64 dot product's rounding).  For Euler this can be switched: off, the
+ * contractions are FP64 FMAs; it is on by default at p = 2..4 and off at
+ * p = 1; DG_UNSUPPORTED for other equations and orders.  (The name is from
+ * an earlier form of the slices, f16 digits on the tensor cores.)  No
+ * reference counterpart. */
 dg_status dg_set_tensor_contractions(dg_solver *s, int on);
-/* the digit tables of that path for order p = 1..4, built on the host from
+/* the basis tables of order p = 1..4 as f16 digit slices, built on the host from
  * the library's basis tables (for checks; no GPU needed): 2240 pairs of
  * 32-bit words, each two f16 digits, then 3 x 16 int column exponents and 16
  * ints of padding -- bytes >= 18176.  dense (optional, 1280 doubles): the
@@ -266,9 +267,9 @@ dg_status dg_bathymetry_project(dg_solver *s, int kind, const double *prm);
  * restored afterwards.  *block receives the choice. */
 dg_status dg_autotune(dg_solver *s, int *block);
 /* dg_autotune that also chooses the element stage, where a solver has two:
- * the FP64-FMA kernel, one thread per element, or the tensor-core kernel,
- * whose quad of lanes holds two elements (two threads per element; Euler,
- * p = 1..4).  *threads_per_element receives 1 or 2.  The two agree to FP64
+ * the FP64-FMA kernel, one thread per element (1), or the fixed-point kernel
+ * with one thread per element and variable (2; Euler, p = 1..4).
+ * *threads_per_element receives 1 or 2.  The two agree to FP64
  * rounding, not bit for bit, so a run's last bits follow the choice. */
 dg_status dg_autotune_stage(dg_solver *s, int *block, int *threads_per_element);
 
