@@ -5,7 +5,7 @@
 namespace dg {
 namespace fx {
 template void element<Advection>(const Ctx &, const ElemArgs &, int);
-template void trace<Advection>(const Ctx &, double *);
+template void trace<Advection>(const Ctx &, double *, int);
 template void batch_element<Advection>(const BatchLaunch &, cudaStream_t, int, int, int, int, int,
                                   int);
 }  // namespace fx

@@ -5,6 +5,6 @@
 namespace dg {
 namespace fx {
 template void element<Euler>(const Ctx &, const ElemArgs &, int);
-template void trace<Euler>(const Ctx &, double *);
+template void trace<Euler>(const Ctx &, double *, int);
 }  // namespace fx
 }  // namespace dg

@@ -22,10 +22,21 @@ void run_element(const Ctx &c, const ElemArgs &a, int mode) {
   }
 }
 
+// what: 0 the traces, 1 limited and traced, 2 limited only
 template <class Eq, int P>
-void run_trace(const Ctx &c, double *u) {
-  k_trace_fx<Eq, P><<<nblk(c.m.K, kTile), Shape<Eq, P>::kThreads, 0, c.st>>>(
-      *static_cast<const FxTab<P> *>(c.fx), *c.q, u, c.T, c.m.K, c.m.Kp);
+void run_trace(const Ctx &c, double *u, int what) {
+  const FxTab<P> &tab = *static_cast<const FxTab<P> *>(c.fx);
+  const unsigned blocks = nblk(c.m.K, kTile);
+  constexpr int T = Shape<Eq, P>::kThreads;
+  if (what == 0)
+    k_trace_fx<Eq, P, false, true><<<blocks, T, 0, c.st>>>(tab, *c.q, u, c.T, c.m.nbr, c.m.K,
+                                                           c.m.Kp);
+  else if (what == 1)
+    k_trace_fx<Eq, P, true, true><<<blocks, T, 0, c.st>>>(tab, *c.q, u, c.T, c.m.nbr, c.m.K,
+                                                          c.m.Kp);
+  else
+    k_trace_fx<Eq, P, true, false><<<blocks, T, 0, c.st>>>(tab, *c.q, u, c.T, c.m.nbr, c.m.K,
+                                                           c.m.Kp);
 }
 
 template <class Eq>
@@ -39,12 +50,12 @@ void element(const Ctx &c, const ElemArgs &a, int mode) {
 }
 
 template <class Eq>
-void trace(const Ctx &c, double *u) {
+void trace(const Ctx &c, double *u, int what) {
   switch (c.p) {
-    case 1: run_trace<Eq, 1>(c, u); break;
-    case 2: run_trace<Eq, 2>(c, u); break;
-    case 3: run_trace<Eq, 3>(c, u); break;
-    case 4: run_trace<Eq, 4>(c, u); break;
+    case 1: run_trace<Eq, 1>(c, u, what); break;
+    case 2: run_trace<Eq, 2>(c, u, what); break;
+    case 3: run_trace<Eq, 3>(c, u, what); break;
+    case 4: run_trace<Eq, 4>(c, u, what); break;
   }
 }
 

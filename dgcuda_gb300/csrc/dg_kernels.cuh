@@ -1056,8 +1056,9 @@ namespace fx {
 // holds the tables
 template <class Eq>
 void element(const Ctx &c, const ElemArgs &a, int mode);
+// (what: 0 the traces, 1 limited and traced, 2 limited only)
 template <class Eq>
-void trace(const Ctx &c, double *u);
+void trace(const Ctx &c, double *u, int what);
 // of a batch's blocks of one order: the element stage, or with stage < 0 the
 // start-of-run traces
 template <class Eq>
@@ -1117,7 +1118,7 @@ struct Launch {
 
   static void trace(const Ctx &c, double *u) {
     if (!c.m.K) return;
-    if (c.fx) return fx::trace<Eq>(c, u);
+    if (c.fx) return fx::trace<Eq>(c, u, 0);
     DG_DISPATCH_P(if constexpr (fp64(P)) (
         k_trace<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, u, c.T, c.m.K,
                                                                c.m.Kp)));
@@ -1196,8 +1197,16 @@ struct Launch {
   }
   static void limit(const Ctx &c, double *u) {
     if (!c.m.K || c.p < 1) return;
-    DG_DISPATCH_P((k_limit<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), u, c.m.nbr,
-                                                                          c.m.K, c.m.Kp)));
+    if (c.fx) return fx::trace<Eq>(c, u, 2);
+    DG_DISPATCH_P(if constexpr (fp64(P)) (
+        k_limit<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), u, c.m.nbr, c.m.K,
+                                                               c.m.Kp)));
+  }
+  // limit() and trace(): the start of an SSP-RK3 run with the limiter on
+  static void limit_trace(const Ctx &c, double *u) {
+    if (c.m.K && c.fx) return fx::trace<Eq>(c, u, 1);
+    limit(c, u);
+    trace(c, u);
   }
   static void lambda(const Ctx &c, const double *u) {
     const unsigned g = std::min(nblk(c.m.K), (unsigned)kLambdaBlocks);
@@ -1221,7 +1230,7 @@ struct Launch {
 #undef DG_DISPATCH_P
 
   static const Ops &ops() {
-    static const Ops o = {trace,  face,       element,  limit,  lambda,  init,    l2err,
+    static const Ops o = {trace,  face,       element,  limit,  limit_trace, lambda, init, l2err,
                           element_tr, limit_tr, vertex, nullptr, nullptr, nullptr, nullptr};
     return o;
   }

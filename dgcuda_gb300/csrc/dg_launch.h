@@ -148,6 +148,8 @@ struct Ops {
                   double cc, const double *dtp);
   // Barth-Jespersen limiter in place
   void (*limit)(const Ctx &, double *u);
+  // limit, then trace
+  void (*limit_trace)(const Ctx &, double *u);
   // max cell-mean wave speed into ds->lam_bits (atomic max)
   void (*lambda)(const Ctx &, const double *u);
   // L2 projection of the problem's initial condition

@@ -369,9 +369,14 @@ dg_status run_steps(dg_solver *s, int nsteps, int scheme, double fixed_dt, doubl
   s->tr_valid = false;
   if (!resume) {
     // the reference limits once before its step loop (time_integrator.cu:178-184)
-    limit(s, s->U);
-    // SSP-RK3 stages find their input traces in T (fused_stage)
-    if (scheme == DG_SSP_RK3) run(s, K_TRACE, [&] { s->ops->trace(s->ctx, s->U); });
+    // and SSP-RK3 stages find their input traces in T (fused_stage)
+    const bool lim = s->prm.limiter && s->np >= 3;
+    if (lim && scheme == DG_SSP_RK3)
+      run(s, K_LIMIT, [&] { s->ops->limit_trace(s->ctx, s->U); });
+    else if (lim)
+      limit(s, s->U);
+    else if (scheme == DG_SSP_RK3)
+      run(s, K_TRACE, [&] { s->ops->trace(s->ctx, s->U); });
   }
   cudaGraphExec_t g = nullptr;
   if (!s->profiling) {
@@ -1256,6 +1261,7 @@ dg_status batch_run(dg_batch *b, int nsteps, double *t) {
     if (b->limiter && s->np >= 3) {
       dg::Ctx c = s->ctx;
       c.st = b->st;
+      if (b->eq == DG_EULER) c.fx = nullptr;  // FP64, as the rest of an Euler batch
       s->ops->limit(c, s->U);
       b->launches++;
     }
