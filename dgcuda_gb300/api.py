@@ -499,8 +499,9 @@ class Solver:
     @property
     def tensor_contractions(self):
         """True when the Euler element stage computes its contractions as exact
-        integer slices (p = 1..4; on by default from p = 2; the other
-        equations always do at these orders)."""
+        integer slices (p = 2..4, on by default; at p = 1, where it is off by
+        default, the switch has no effect: the stage always does, as the other
+        equations' at p = 1..4)."""
         v = np.zeros(1, dtype=np.int32)
         _check(self._L.dg_get_tensor_contractions(self._h, _iptr(v)))
         return bool(v[0])

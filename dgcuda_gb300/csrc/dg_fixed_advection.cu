@@ -7,6 +7,6 @@ namespace fx {
 template void element<Advection>(const Ctx &, const ElemArgs &, int);
 template void trace<Advection>(const Ctx &, double *, int);
 template void batch_element<Advection>(const BatchLaunch &, cudaStream_t, int, int, int, int, int,
-                                  int);
+                                  int, bool);
 }  // namespace fx
 }  // namespace dg

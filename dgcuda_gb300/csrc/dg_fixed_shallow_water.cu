@@ -7,6 +7,6 @@ namespace fx {
 template void element<ShallowWater>(const Ctx &, const ElemArgs &, int);
 template void trace<ShallowWater>(const Ctx &, double *, int);
 template void batch_element<ShallowWater>(const BatchLaunch &, cudaStream_t, int, int, int, int, int,
-                                  int);
+                                  int, bool);
 }  // namespace fx
 }  // namespace dg

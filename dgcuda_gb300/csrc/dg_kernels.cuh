@@ -1019,6 +1019,7 @@ __global__ void __launch_bounds__(kMaxBlock)
   }
 }
 
+// (the orders that contract in FP64: Euler's p = 2 and 3)
 template <class Eq>
 __global__ void __launch_bounds__(kMaxBlock)
     k_trace_batch(const __grid_constant__ BatchTabs tb, const BatchProb *__restrict__ probs,
@@ -1028,7 +1029,6 @@ __global__ void __launch_bounds__(kMaxBlock)
   const int e = (blockIdx.x - blk0[pi]) * blockDim.x + threadIdx.x;
   if (e >= pr.K) return;
   switch (pr.p) {
-    case 1: trace_body<Eq, 1>(tb.t1, pr.q, pr.U, pr.T, pr.Kp, e); break;
     case 2: trace_body<Eq, 2>(tb.t2, pr.q, pr.U, pr.T, pr.Kp, e); break;
     case 3: trace_body<Eq, 3>(tb.t3, pr.q, pr.U, pr.T, pr.Kp, e); break;
   }
@@ -1063,7 +1063,7 @@ void trace(const Ctx &c, double *u, int what);
 // start-of-run traces
 template <class Eq>
 void batch_element(const BatchLaunch &b, cudaStream_t st, int p, int lo, int n, int blk,
-                   int stage, int check);
+                   int stage, int check, bool lim);
 }  // namespace fx
 inline unsigned nblk(int n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
 
@@ -1084,10 +1084,10 @@ struct Launch {
     case 5: { constexpr int P = 5; expr; } break; \
   }
 
-  // orders whose FP64 traces and element stage are reachable: all of Euler's
-  // (its fixed-point stage can be switched off, and its batch contracts in
-  // FP64), elsewhere only those without a fixed-point stage
-  static constexpr bool fp64(int P) { return Eq::kFusedLimiter || P < 1 || P > 4; }
+  // orders whose FP64 traces and element stage are reachable: Euler's p = 2..4
+  // (its fixed-point stage can be switched off there, and its batch contracts
+  // in FP64), elsewhere only those without a fixed-point stage
+  static constexpr bool fp64(int P) { return (Eq::kFusedLimiter && P != 1) || P < 1 || P > 4; }
 
   static ElemArgs eargs(const Ctx &c, double *us, const double *un, double *out, double ca,
                         double cb, double cc, const double *dtp, double *T, int check) {
@@ -1174,8 +1174,8 @@ struct Launch {
     if (!c.m.K) return;
     const ElemArgs a = eargs(c, us, un, out, ca, cb, cc, dtp, c.T, 0);
     if (c.fx) return fx::element<Eq>(c, a, 2);
-    DG_DISPATCH_P((k_element<Eq, P, true, true><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(
-        tab<P>(c), *c.q, a)));
+    DG_DISPATCH_P(if constexpr (fp64(P)) (
+        k_element<Eq, P, true, true><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, a)));
   }
   static void element_tr(const Ctx &c, double *us, const double *un, double *out, double ca,
                          double cb, double cc, const double *dtp, int check) {
@@ -1240,14 +1240,12 @@ struct Launch {
     return *reinterpret_cast<const BatchTabs *>(b.tabs);
   }
   static void b_trace(const BatchLaunch &b) {
-    if constexpr (Eq::kFusedLimiter) {
-      k_trace_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0);
-    } else {
-      for (int g = 0; g < BatchLaunch::kGroups; g++) {
-        const int lo = b.eblk_g[g], n = b.eblk_g[g + 1] - lo;
-        if (n > 0) fx::batch_element<Eq>(b, b.st, 1 + g / 2, lo, n, b.blk_g[g], -1, 1);
-      }
+    for (int g = 0; g < BatchLaunch::kGroups; g++) {
+      const int lo = b.eblk_g[g], n = b.eblk_g[g + 1] - lo, p = 1 + g / 2;
+      if (n > 0 && b.fx[p]) fx::batch_element<Eq>(b, b.st, p, lo, n, b.blk_g[g], -1, 1, false);
     }
+    if constexpr (Eq::kFusedLimiter)  // the orders that contract in FP64
+      k_trace_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0);
   }
   static void b_face(const BatchLaunch &b, double tcoef) {
     k_face_batch<Eq><<<b.nsblk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.sblk2prob, b.sblk0,
@@ -1268,17 +1266,15 @@ struct Launch {
       const cudaStream_t st = side ? b.gst[g] : b.st;
       first = false;
       if (side) cudaStreamWaitEvent(st, b.fork, 0);
-      if constexpr (!Eq::kFusedLimiter) {
-        fx::batch_element<Eq>(b, st, p, lo, n, blk, stage, check);
-      } else if (p == 1) {
-        k_element_batch_p<Eq, 1, LIM><<<n, blk, 0, st>>>(tb.t1, b.probs, b.eblk2prob, b.eblk0,
-                                                           lo, stage, check);
-      } else if (p == 2) {
-        k_element_batch_p<Eq, 2, LIM><<<n, blk, 0, st>>>(tb.t2, b.probs, b.eblk2prob, b.eblk0,
-                                                           lo, stage, check);
-      } else {
-        k_element_batch_p<Eq, 3, LIM><<<n, blk, 0, st>>>(tb.t3, b.probs, b.eblk2prob, b.eblk0,
-                                                           lo, stage, check);
+      if (b.fx[p]) {
+        fx::batch_element<Eq>(b, st, p, lo, n, blk, stage, check, LIM);
+      } else if constexpr (Eq::kFusedLimiter) {
+        if (p == 2)
+          k_element_batch_p<Eq, 2, LIM><<<n, blk, 0, st>>>(tb.t2, b.probs, b.eblk2prob, b.eblk0,
+                                                             lo, stage, check);
+        else
+          k_element_batch_p<Eq, 3, LIM><<<n, blk, 0, st>>>(tb.t3, b.probs, b.eblk2prob, b.eblk0,
+                                                             lo, stage, check);
       }
       if (side) {
         cudaEventRecord(b.join[g], st);

@@ -281,10 +281,16 @@ void drop_graphs(dg_solver *s) {
   s->graph_launches.clear();
 }
 
-// the element stage's contractions: fixed point at p = 1..4, for Euler only
-// where it is switched on
+// whether the solver's element stage has two forms, fixed point and FP64, that
+// dg_set_tensor_contractions switches between: Euler at p = 2..4
+bool fx_switched(const dg_solver *s) {
+  return s->eq == DG_EULER && s->p >= 2 && !s->fximg.empty();
+}
+
+// the element stage's contractions: fixed point at p = 1..4, for Euler at p =
+// 2..4 only where it is switched on
 void fx_select(dg_solver *s) {
-  const bool on = !s->fximg.empty() && (s->eq != DG_EULER || s->tensor);
+  const bool on = !s->fximg.empty() && (!fx_switched(s) || s->tensor);
   s->ctx.fx = on ? s->fximg.data() : nullptr;
 }
 
@@ -1090,9 +1096,9 @@ extern "C" dg_status dg_autotune_stage(dg_solver *s, int *block, int *threads_pe
   CK(cudaMalloc(&save, s->ndof_p * sizeof(double)));
   CK(cudaMemcpyAsync(save, s->U, s->ndof_p * sizeof(double), cudaMemcpyDeviceToDevice, s->st));
   std::vector<int> variants;  // 1: the FP64 element stage, 2: the fixed-point one
-  const bool two = s->eq == DG_EULER && !s->fximg.empty();
+  const bool two = fx_switched(s);
   if (threads_per_element && two) variants = {1, 2};
-  else variants = {two && s->tensor ? 2 : 1};
+  else variants = {s->ctx.fx ? 2 : 1};
   int best_blk = s->ctx.blk, best_v = variants[0];
   float best_ms = 1e30f;
   for (int v : variants) {
@@ -1261,7 +1267,7 @@ dg_status batch_run(dg_batch *b, int nsteps, double *t) {
     if (b->limiter && s->np >= 3) {
       dg::Ctx c = s->ctx;
       c.st = b->st;
-      if (b->eq == DG_EULER) c.fx = nullptr;  // FP64, as the rest of an Euler batch
+      if (b->eq == DG_EULER && s->p > 1) c.fx = nullptr;  // FP64, as its batch at these orders
       s->ops->limit(c, s->U);
       b->launches++;
     }
@@ -1330,21 +1336,20 @@ extern "C" dg_status dg_batch_create(int n, dg_solver *const *members, dg_batch 
   b->ops = batch_ops_for(b->eq);
   b->tabs.resize(dg::batch_tabs_bytes());
   dg::build_batch_tabs(timg[1], timg[2], timg[3], b->tabs.data());
-  // members that contract in fixed point (every equation but Euler, whose
+  // orders that contract in fixed point (all but Euler's p = 2 and 3, whose
   // batch contracts in FP64): the default tables or the first member's of
   // each order, as the FP64 tables above
-  if (b->eq != DG_EULER)
-    for (int p = 1; p <= 3; p++) {
-      b->fximg[p].resize(dg::fx_tab_bytes(p));
-      if (!timg[p]) {
-        std::vector<char> t(dg::tab_bytes(p));
-        dg::build_tab(p, DG_TABLES[p], t.data());
-        dg::build_fx_tab(p, t.data(), b->fximg[p].data());
-      } else {
-        dg::build_fx_tab(p, timg[p], b->fximg[p].data());
-      }
-      b->bl.fx[p] = b->fximg[p].data();
+  for (int p = 1; p <= (b->eq == DG_EULER ? 1 : 3); p++) {
+    b->fximg[p].resize(dg::fx_tab_bytes(p));
+    if (!timg[p]) {
+      std::vector<char> t(dg::tab_bytes(p));
+      dg::build_tab(p, DG_TABLES[p], t.data());
+      dg::build_fx_tab(p, t.data(), b->fximg[p].data());
+    } else {
+      dg::build_fx_tab(p, timg[p], b->fximg[p].data());
     }
+    b->bl.fx[p] = b->fximg[p].data();
+  }
   std::vector<dg::BatchProb> hp(n);
   for (int i = 0; i < n; i++) {
     dg_solver *s = b->m[i];
@@ -2142,7 +2147,7 @@ extern "C" dg_status dg_load_checkpoint(dg_solver *s, const char *path, double *
 }
 
 // the Euler element stage's basis contractions in fixed point (dg_fixed.cuh) or
-// in FP64 FMAs, p = 1..4
+// in FP64 FMAs, p = 2..4 (at p = 1 the switch is kept and has no effect)
 extern "C" dg_status dg_set_tensor_contractions(dg_solver *s, int on) {
   if (!s) return fail(DG_BAD_ARG, "null solver");
   s->tr_valid = false;
@@ -2158,7 +2163,7 @@ extern "C" dg_status dg_set_tensor_contractions(dg_solver *s, int on) {
 
 extern "C" dg_status dg_get_tensor_contractions(dg_solver *s, int *on) {
   if (!s || !on) return fail(DG_BAD_ARG, "null argument");
-  *on = s->eq == DG_EULER && s->ctx.fx != nullptr;
+  *on = s->eq == DG_EULER && !s->fximg.empty() && s->tensor;
   return DG_OK;
 }
 

@@ -226,11 +226,12 @@ dg_status dg_set_inflow_series(dg_solver *s, int n, const double *amp, const dou
 /* The element stage computes its basis contractions (area values, volume
  * and surface projections, next-stage traces) at p = 1..4 as exact integer
  * slices off the FP64 pipe (56-bit fixed point, per-output error below an
- * FP64 dot product's rounding).  For Euler this can be switched: off, the
- * contractions are FP64 FMAs; it is on by default at p = 2..4 and off at
- * p = 1; DG_UNSUPPORTED for other equations and orders.  (The name is from
- * an earlier form of the slices, f16 digits on the tensor cores.)  No
- * reference counterpart. */
+ * FP64 dot product's rounding).  For Euler at p = 2..4 this can be
+ * switched: off, the contractions are FP64 FMAs; on by default.  At p = 1 the
+ * switch (off by default) is kept and has no effect: the slices are the
+ * faster stage there too.  DG_UNSUPPORTED for other equations and orders.
+ * (The name is from an earlier form of the slices, f16 digits on the tensor
+ * cores.)  No reference counterpart. */
 dg_status dg_set_tensor_contractions(dg_solver *s, int on);
 /* the basis tables of order p = 1..4 as f16 digit slices, built on the host from
  * the library's basis tables (for checks; no GPU needed): 2240 pairs of
@@ -268,7 +269,8 @@ dg_status dg_bathymetry_project(dg_solver *s, int kind, const double *prm);
 dg_status dg_autotune(dg_solver *s, int *block);
 /* dg_autotune that also chooses the element stage, where a solver has two:
  * the FP64-FMA kernel, one thread per element (1), or the fixed-point kernel
- * with one thread per element and variable (2; Euler, p = 1..4).
+ * with one thread per element and variable (2; Euler, p = 2..4 -- at p = 1, and
+ * for the other equations at p = 1..4, there is only the latter).
  * *threads_per_element receives 1 or 2.  The two agree to FP64
  * rounding, not bit for bit, so a run's last bits follow the choice. */
 dg_status dg_autotune_stage(dg_solver *s, int *block, int *threads_per_element);
