@@ -352,6 +352,7 @@ struct Advection {  // advection/advection.cu
   static constexpr bool kBathymetry = false;
   // the velocity may vary in space (q.field): fluxes then take the position
   static constexpr bool kFusedLimiter = false;  // the limiter in the element epilogue
+  static constexpr bool kStateSpeed = false;  // the CFL wave speed depends on the state
   static constexpr bool kField = true;
   static constexpr bool kFolded = false;
   DG_HD static bool physical(const EqP &, const double *) { return true; }
@@ -402,6 +403,7 @@ struct Euler {  // euler/euler.cu
   static constexpr int N = 4;
   static constexpr bool kBathymetry = false;
   static constexpr bool kFusedLimiter = true;  // the limiter in the element epilogue
+  static constexpr bool kStateSpeed = true;  // the CFL wave speed depends on the state
   static constexpr bool kField = false;
   // rho >= 0 and p >= 0 (is_physical, euler.cu:76-86); with rho > 0,
   // p < 0 <=> 2 rho E < |rho u|^2, which needs no FP64 division.  On the
@@ -520,6 +522,7 @@ struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
   static constexpr int N = 3;
   static constexpr bool kBathymetry = true;  // optional bed b(x, y): source -g h grad b
   static constexpr bool kFusedLimiter = false;  // the limiter in the element epilogue
+  static constexpr bool kStateSpeed = true;  // the CFL wave speed depends on the state
   static constexpr bool kField = false;
   static constexpr bool kFolded = false;
   DG_HD static bool physical(const EqP &, const double *U) { return U[0] >= 0.; }
@@ -567,6 +570,7 @@ struct Maxwell {  // maxwells/maxwells.cu, U = (Hx, Hy, Ez)
   static constexpr int N = 3;
   static constexpr bool kBathymetry = false;
   static constexpr bool kFusedLimiter = false;  // the limiter in the element epilogue
+  static constexpr bool kStateSpeed = false;  // the CFL wave speed depends on the state
   static constexpr bool kField = false;
   static constexpr bool kFolded = false;
   DG_HD static bool physical(const EqP &, const double *) { return true; }
@@ -599,6 +603,37 @@ struct Maxwell {  // maxwells/maxwells.cu, U = (Hx, Hy, Ez)
   }
   static constexpr bool outflow_uses_exact = false;
 };
+
+// dt = cfl * d_min / lambda_max / (2p + 1) (time_integrator.cu:217), the
+// last step shortened to land on endtime (:226-231)
+DG_HD void compute_dt(DevScalars *ds, double lam, int p) {
+  double dt = ds->fixed_dt > 0 ? ds->fixed_dt : ds->cfl * ds->dmin / lam / (2. * p + 1.);
+  if (!(dt > 0 && dt <= 1.7976931348623157e308)) {  // NaN, not positive or infinite
+    ds->status = 4;
+    dt = 0.0;
+  }
+  ds->last = 0;
+  if (ds->endtime > 0) {
+    if (ds->t + dt > ds->endtime) {
+      dt = ds->endtime - ds->t;
+      ds->last = 1;
+    }
+    if (dt < 0) dt = 0;
+  }
+  ds->dt = dt;
+  ds->lam = lam;
+}
+// t to the end of the step whose dt ds holds
+DG_HD void advance_time(DevScalars *ds) {
+  if (ds->dt > 0) ds->steps++;
+  ds->t = ds->last ? ds->endtime : ds->t + ds->dt;
+}
+DG_HD void cfl_step(DevScalars *ds, double lam, int p, int mode) {
+  if (mode == CFL_SSP && ds->pending) advance_time(ds);
+  compute_dt(ds, lam, p);
+  if (mode == CFL_RK) advance_time(ds);
+  ds->pending = mode == CFL_SSP;
+}
 
 // the volume integrands g = F . (ys, -xs), h = F . (-yr, xr) of a state U
 // (eval_volume, conserv_kernels.cu:1066-1074): an equation's own folded

@@ -329,6 +329,7 @@ __device__ __forceinline__ void traces_out(const FxTab<P> &tab, const EqP &q,
       block_sync<N>();
     }
   }
+  pdl_end();
   // ---- T: each warp stores whole elements, NF N contiguous doubles ----
   constexpr int C = NF * N;
 #pragma unroll 2
@@ -608,6 +609,7 @@ __global__ void __launch_bounds__(Shape<Eq, P>::kThreads, min_blocks<Eq, P>())
   __shared__ double st[S::kRows * kPitch];
   __shared__ int mxs[S::N * S::N * kTile];
   __shared__ int flag[2 * kTile];
+  pdl_begin();
   element_tile<Eq, P, MODE>(tab, q, a, blockIdx.x * kTile, st, mxs, flag);
 }
 
@@ -640,6 +642,7 @@ __global__ void __launch_bounds__(Shape<Eq, P>::kThreads)
   using S = Shape<Eq, P>;
   __shared__ double st[STORE ? S::NF * S::N * kPitch : 1];
   __shared__ int flag[kTile];
+  pdl_begin();
   trace_tile<Eq, P, LIM, STORE>(tab, q, u, T, nbr, K, Kp, blockIdx.x * kTile, st, flag);
 }
 

@@ -13,12 +13,12 @@ void run_element(const Ctx &c, const ElemArgs &a, int mode) {
   const FxTab<P> &tab = *static_cast<const FxTab<P> *>(c.fx);
   const unsigned blocks = nblk(c.m.K, kTile);
   if (mode == 0) {
-    k_element_fx<Eq, P, 0><<<blocks, S::kThreads, 0, c.st>>>(tab, *c.q, a);
+    launch(k_element_fx<Eq, P, 0>, blocks, S::kThreads, c.st, tab, *c.q, a);
   } else if (mode == 1) {
-    k_element_fx<Eq, P, 1><<<blocks, S::kThreads, 0, c.st>>>(tab, *c.q, a);
+    launch(k_element_fx<Eq, P, 1>, blocks, S::kThreads, c.st, tab, *c.q, a);
   } else {
     if constexpr (Eq::kFusedLimiter)
-      k_element_fx<Eq, P, 2><<<blocks, S::kThreads, 0, c.st>>>(tab, *c.q, a);
+      launch(k_element_fx<Eq, P, 2>, blocks, S::kThreads, c.st, tab, *c.q, a);
   }
 }
 
@@ -29,14 +29,14 @@ void run_trace(const Ctx &c, double *u, int what) {
   const unsigned blocks = nblk(c.m.K, kTile);
   constexpr int T = Shape<Eq, P>::kThreads;
   if (what == 0)
-    k_trace_fx<Eq, P, false, true><<<blocks, T, 0, c.st>>>(tab, *c.q, u, c.T, c.m.nbr, c.m.K,
-                                                           c.m.Kp);
+    launch(k_trace_fx<Eq, P, false, true>, blocks, T, c.st, tab, *c.q, u, c.T, c.m.nbr, c.m.K,
+           c.m.Kp);
   else if (what == 1)
-    k_trace_fx<Eq, P, true, true><<<blocks, T, 0, c.st>>>(tab, *c.q, u, c.T, c.m.nbr, c.m.K,
-                                                          c.m.Kp);
+    launch(k_trace_fx<Eq, P, true, true>, blocks, T, c.st, tab, *c.q, u, c.T, c.m.nbr, c.m.K,
+           c.m.Kp);
   else
-    k_trace_fx<Eq, P, true, false><<<blocks, T, 0, c.st>>>(tab, *c.q, u, c.T, c.m.nbr, c.m.K,
-                                                           c.m.Kp);
+    launch(k_trace_fx<Eq, P, true, false>, blocks, T, c.st, tab, *c.q, u, c.T, c.m.nbr, c.m.K,
+           c.m.Kp);
 }
 
 template <class Eq>

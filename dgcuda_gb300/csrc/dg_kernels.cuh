@@ -49,9 +49,18 @@ namespace dg {
 constexpr int kBlock = 128;     // fixed block of the auxiliary kernels
 constexpr int kMaxBlock = 256;  // largest autotuned block of the stage kernels
 
-template <int P>
-__device__ __forceinline__ size_t trace_stride() {
-  return 3 * (P + 1);
+// Programmatic dependent launch: a kernel of a step waits here, before it
+// touches memory, for the end of its predecessor on the stream, and lets its
+// successor be scheduled shortly before its own end (pdl_end), which hides
+// the successor's launch.  Not earlier: blocks of a grid that does not fill
+// the GPU would all be placed on the SMs that drain first and wait there (a
+// trigger at the start made steps of 33k triangles 15-50 % slower).  Both are
+// no-ops in a launch without the attribute.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_end() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -99,6 +108,7 @@ template <class Eq, int P>
 __global__ void __launch_bounds__(kMaxBlock) k_trace(const __grid_constant__ Tab<P> tab,
                                                      const __grid_constant__ EqP q, double *u,
                                                      double *__restrict__ T, int K, int Kp) {
+  pdl_begin();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < K) trace_body<Eq, P>(tab, q, u, T, Kp, e);
 }
@@ -219,6 +229,7 @@ __device__ __forceinline__ void face_body(const Tab<P> &tab, const EqP &q, const
       store_vars<N>(F + j * N, Fn);
     }
   }
+  pdl_end();
   if (FS) store_vars<N>(a.Fs + (size_t)s * N, fs);
 }
 
@@ -226,6 +237,7 @@ template <class Eq, int P, bool FS = false>
 __global__ void __launch_bounds__(kMaxBlock) k_face(const __grid_constant__ Tab<P> tab,
                                                     const __grid_constant__ EqP q,
                                                     const __grid_constant__ FaceArgs a) {
+  pdl_begin();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < a.S) face_body<Eq, P, FS>(tab, q, a, s);
 }
@@ -446,6 +458,7 @@ template <class Eq, int P, bool TR, bool LIM = false>
 __global__ void __launch_bounds__(kMaxBlock) k_element(const __grid_constant__ Tab<P> tab,
                                                        const __grid_constant__ EqP q,
                                                        const __grid_constant__ ElemArgs a) {
+  pdl_begin();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < a.K) element_body<Eq, P, TR, LIM>(tab, q, a, e);
 }
@@ -511,6 +524,7 @@ __device__ __forceinline__ void means_body(const Tab<P> &tab, const ElemArgs &a,
   }
   const double sc = a.cc * *a.dtp * a.geo[4 * Kp + e];
   const double e0 = tab.E[0][0][0];
+  pdl_end();
 #pragma unroll
   for (int n = 0; n < N; n++) {
     const size_t o = (size_t)(n * NP) * Kp + e;
@@ -525,6 +539,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_means(const __grid_constant__ Tab
                                                      const __grid_constant__ ElemArgs a,
                                                      const double *__restrict__ Fs,
                                                      double *__restrict__ M) {
+  pdl_begin();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < a.K) means_body<Eq, P>(tab, a, Fs, M, e);
 }
@@ -557,6 +572,7 @@ template <class Eq, int P>
 __global__ void __launch_bounds__(kMaxBlock) k_limit(const __grid_constant__ Tab<P> tab,
                                                   double *u, const int *__restrict__ nbr,
                                                   int K, int Kp) {
+  pdl_begin();
   constexpr int N = Eq::N, NP = Tab<P>::NP, N1 = Tab<P>::N1;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= K) return;
@@ -714,73 +730,67 @@ __global__ void __launch_bounds__(kMaxBlock) k_limit_tr(const __grid_constant__ 
                                                         double *u, double *__restrict__ T,
                                                         const int *__restrict__ nbr, int K,
                                                         int Kp) {
+  pdl_begin();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < K) limit_tr_body<Eq, P>(tab, q, u, T, nbr, Kp, e, u, (size_t)Tab<P>::NP * Kp);
 }
 
 // ---------------------------------------------------------------------------
-// block max of the cell-mean wave speed of elements [e0, e0 + blockDim) into
-// ds->lam_bits (the block's elements belong to one problem)
+// The largest cell-mean wave speed, and the time step from it: each block
+// leaves its maximum in ds->lam_bits, and the block that finishes last takes
+// the step (cfl_step) and clears the word for the next one.  One launch
+// where a reset, a maximum, a time-step and an advance kernel cost four.
 template <class Eq, int P>
-__device__ __forceinline__ void lambda_body(const Tab<P> &tab, const EqP &q,
-                                            const double *__restrict__ u, DevScalars *ds, int K,
-                                            int Kp, int e) {
+__device__ __forceinline__ double cell_speed(const Tab<P> &tab, const EqP &q,
+                                             const double *__restrict__ u, DevScalars *ds, int Kp,
+                                             int e) {
   constexpr int N = Eq::N, NP = Tab<P>::NP;
-  double lam = 0.0;
-  if (e < K) {
-    double U[N];
+  double U[N];
 #pragma unroll
-    for (int n = 0; n < N; n++) U[n] = u[(size_t)(n * NP) * Kp + e] * tab.B[0][0];
-    lam = Eq::mean_speed(q, U);
-    if (!(lam == lam)) {
-      atomicExch(&ds->status, 4);
-      lam = 0.0;
-    }
-  }
+  for (int n = 0; n < N; n++) U[n] = u[(size_t)(n * NP) * Kp + e] * tab.B[0][0];
+  const double l = Eq::mean_speed(q, U);
+  if (l == l) return l;
+  atomicExch(&ds->status, 4);
+  return 0.0;
+}
+// the larger of two speeds (no NaN; a comparison and a select where fmax costs
+// an FP64 operation)
+__device__ __forceinline__ double larger(double a, double b) { return b > a ? b : a; }
+// lam: this thread's maximum; nblocks: the blocks that meet in ds
+__device__ __forceinline__ void cfl_reduce(double lam, DevScalars *ds, unsigned nblocks, int p,
+                                           int mode) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lam = fmax(lam, __shfl_xor_sync(0xffffffffu, lam, o));
+  for (int o = 16; o > 0; o >>= 1) lam = larger(lam, __shfl_xor_sync(0xffffffffu, lam, o));
   __shared__ double sm[kBlock / 32];
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = lam;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = sm[0];
-    for (int w = 1; w < kBlock / 32; w++) m = fmax(m, sm[w]);
+  if (threadIdx.x != 0) return;
+  double m = sm[0];
+  for (int w = 1; w < kBlock / 32; w++) m = larger(m, sm[w]);
+  if (nblocks > 1) {
     atomicMax(&ds->lam_bits, (unsigned long long)__double_as_longlong(m));
+    __threadfence();
+    if (atomicAdd(&ds->ticket, 1u) != nblocks - 1) return;
+    __threadfence();
+    m = __longlong_as_double((long long)atomicExch(&ds->lam_bits, 0ull));
+    ds->ticket = 0;
   }
+  cfl_step(ds, m, p, mode);
 }
 
-// the same maximum over a single problem, grid-stride: a few blocks per SM
-// each take the max over many elements, so one atomic per block stays cheap
-// (one per 128 elements serialises on the one word)
+// of a single problem, grid-stride: a few blocks per SM each take the max over
+// many elements, so their atomics on one word stay cheap
 constexpr int kLambdaBlocks = 1024;
 template <class Eq, int P>
 __global__ void __launch_bounds__(kBlock) k_lambda(const __grid_constant__ Tab<P> tab,
                                                    const __grid_constant__ EqP q,
                                                    const double *__restrict__ u, DevScalars *ds,
-                                                   int K, int Kp) {
-  constexpr int N = Eq::N, NP = Tab<P>::NP;
+                                                   int K, int Kp, int mode) {
+  pdl_begin();
   double lam = 0.0;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < K; e += gridDim.x * blockDim.x) {
-    double U[N];
-#pragma unroll
-    for (int n = 0; n < N; n++) U[n] = u[(size_t)(n * NP) * Kp + e] * tab.B[0][0];
-    double l = Eq::mean_speed(q, U);
-    if (!(l == l)) {
-      atomicExch(&ds->status, 4);
-      l = 0.0;
-    }
-    lam = fmax(lam, l);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lam = fmax(lam, __shfl_xor_sync(0xffffffffu, lam, o));
-  __shared__ double sm[kBlock / 32];
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = lam;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double m = sm[0];
-    for (int w = 1; w < kBlock / 32; w++) m = fmax(m, sm[w]);
-    atomicMax(&ds->lam_bits, (unsigned long long)__double_as_longlong(m));
-  }
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < K; e += gridDim.x * blockDim.x)
+    lam = larger(lam, cell_speed<Eq, P>(tab, q, u, ds, Kp, e));
+  cfl_reduce(lam, ds, gridDim.x, P, mode);
 }
 
 // ---------------------------------------------------------------------------
@@ -1041,11 +1051,15 @@ __global__ void __launch_bounds__(kBlock)
   const int pi = blk2prob[blockIdx.x];
   const BatchProb &pr = probs[pi];
   const int e = (blockIdx.x - blk0[pi]) * blockDim.x + threadIdx.x;
-  switch (pr.p) {
-    case 1: lambda_body<Eq, 1>(tb.t1, pr.q, pr.U, pr.ds, pr.K, pr.Kp, e); break;
-    case 2: lambda_body<Eq, 2>(tb.t2, pr.q, pr.U, pr.ds, pr.K, pr.Kp, e); break;
-    case 3: lambda_body<Eq, 3>(tb.t3, pr.q, pr.U, pr.ds, pr.K, pr.Kp, e); break;
+  double lam = 0.0;
+  if (e < pr.K) {
+    switch (pr.p) {
+      case 1: lam = cell_speed<Eq, 1>(tb.t1, pr.q, pr.U, pr.ds, pr.Kp, e); break;
+      case 2: lam = cell_speed<Eq, 2>(tb.t2, pr.q, pr.U, pr.ds, pr.Kp, e); break;
+      case 3: lam = cell_speed<Eq, 3>(tb.t3, pr.q, pr.U, pr.ds, pr.Kp, e); break;
+    }
   }
+  cfl_reduce(lam, pr.ds, (unsigned)(pr.K + kBlock - 1) / kBlock, pr.p, CFL_SSP);
 }
 
 // ---------------------------------------------------------------------------
@@ -1066,6 +1080,24 @@ void batch_element(const BatchLaunch &b, cudaStream_t st, int p, int lo, int n, 
                    int stage, int check, bool lim);
 }  // namespace fx
 inline unsigned nblk(int n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
+
+// a launch with the programmatic-dependence attribute: only for kernels that
+// begin with pdl_begin(), whose predecessor's end implies the end of
+// everything before it for the same reason
+template <class... P, class... A>
+inline void launch(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t st,
+                   const A &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 
 template <class Eq>
 struct Launch {
@@ -1120,8 +1152,8 @@ struct Launch {
     if (!c.m.K) return;
     if (c.fx) return fx::trace<Eq>(c, u, 0);
     DG_DISPATCH_P(if constexpr (fp64(P)) (
-        k_trace<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, u, c.T, c.m.K,
-                                                               c.m.Kp)));
+        launch(k_trace<Eq, P>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q, u, c.T, c.m.K,
+               c.m.Kp)));
   }
   template <bool FS>
   static void face_args(const Ctx &c, const double *t, double tcoef, double *Fs) {
@@ -1140,8 +1172,8 @@ struct Launch {
     a.S = c.m.S;
     a.Sb = c.m.Sb;
     a.Kp = c.m.Kp;
-    DG_DISPATCH_P((k_face<Eq, P, FS><<<nblk(c.m.S, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q,
-                                                                             a)));
+    DG_DISPATCH_P((launch(k_face<Eq, P, FS>, nblk(c.m.S, c.blk), c.blk, c.st, tab<P>(c), *c.q,
+                          a)));
   }
   static void face(const Ctx &c, const double *t, double tcoef) {
     face_args<false>(c, t, tcoef, nullptr);
@@ -1156,8 +1188,8 @@ struct Launch {
                     const double *dtp) {
     if (!c.m.K) return;
     const ElemArgs a = eargs(c, us, un, nullptr, ca, cb, cc, dtp, nullptr, 0);
-    DG_DISPATCH_P((k_means<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), a, c.Fs,
-                                                                          c.M)));
+    DG_DISPATCH_P((launch(k_means<Eq, P>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), a, c.Fs,
+                          c.M)));
   }
   static void element(const Ctx &c, double *us, const double *un, double *out, double ca,
                       double cb, double cc, const double *dtp) {
@@ -1165,7 +1197,7 @@ struct Launch {
     const ElemArgs a = eargs(c, us, un, out, ca, cb, cc, dtp, nullptr, 0);
     if (c.fx) return fx::element<Eq>(c, a, 0);
     DG_DISPATCH_P(if constexpr (fp64(P)) (
-        k_element<Eq, P, false><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, a)));
+        launch(k_element<Eq, P, false>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q, a)));
   }
   // element_tr() with the limiter in the epilogue (c.M holds the output's
   // means from k_means)
@@ -1175,7 +1207,8 @@ struct Launch {
     const ElemArgs a = eargs(c, us, un, out, ca, cb, cc, dtp, c.T, 0);
     if (c.fx) return fx::element<Eq>(c, a, 2);
     DG_DISPATCH_P(if constexpr (fp64(P)) (
-        k_element<Eq, P, true, true><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, a)));
+        launch(k_element<Eq, P, true, true>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q,
+               a)));
   }
   static void element_tr(const Ctx &c, double *us, const double *un, double *out, double ca,
                          double cb, double cc, const double *dtp, int check) {
@@ -1183,7 +1216,7 @@ struct Launch {
     const ElemArgs a = eargs(c, us, un, out, ca, cb, cc, dtp, c.T, check);
     if (c.fx) return fx::element<Eq>(c, a, 1);
     DG_DISPATCH_P(if constexpr (fp64(P)) (
-        k_element<Eq, P, true><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), *c.q, a)));
+        launch(k_element<Eq, P, true>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q, a)));
   }
   static void bed_slopes(const Ctx &c, double *out) {
     if (!c.m.K) return;
@@ -1192,15 +1225,15 @@ struct Launch {
   }
   static void limit_tr(const Ctx &c, double *u) {
     if (!c.m.K || c.p < 1) return;
-    DG_DISPATCH_P((k_limit_tr<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(
-        tab<P>(c), *c.q, u, c.T, c.m.nbr, c.m.K, c.m.Kp)));
+    DG_DISPATCH_P((launch(k_limit_tr<Eq, P>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q, u,
+                          c.T, c.m.nbr, c.m.K, c.m.Kp)));
   }
   static void limit(const Ctx &c, double *u) {
     if (!c.m.K || c.p < 1) return;
     if (c.fx) return fx::trace<Eq>(c, u, 2);
     DG_DISPATCH_P(if constexpr (fp64(P)) (
-        k_limit<Eq, P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(tab<P>(c), u, c.m.nbr, c.m.K,
-                                                               c.m.Kp)));
+        launch(k_limit<Eq, P>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), u, c.m.nbr, c.m.K,
+               c.m.Kp)));
   }
   // limit() and trace(): the start of an SSP-RK3 run with the limiter on
   static void limit_trace(const Ctx &c, double *u) {
@@ -1208,10 +1241,12 @@ struct Launch {
     limit(c, u);
     trace(c, u);
   }
-  static void lambda(const Ctx &c, const double *u) {
-    const unsigned g = std::min(nblk(c.m.K), (unsigned)kLambdaBlocks);
-    DG_DISPATCH_P((k_lambda<Eq, P><<<g, kBlock, 0, c.st>>>(tab<P>(c), *c.q, u, c.ds, c.m.K,
-                                                            c.m.Kp)));
+  static void lambda(const Ctx &c, const double *u, int mode) {
+    // one element's speed is every element's where it does not depend on the state
+    const int K = Eq::kStateSpeed ? c.m.K : 1;
+    const unsigned g = std::min(nblk(K), (unsigned)kLambdaBlocks);
+    DG_DISPATCH_P((launch(k_lambda<Eq, P>, g, kBlock, c.st, tab<P>(c), *c.q, u, c.ds, K,
+                          c.m.Kp, mode)));
   }
   static void init(const Ctx &c, double *u) {
     DG_DISPATCH_P((k_init<Eq, P><<<nblk(c.m.K), kBlock, 0, c.st>>>(tab<P>(c), *c.q, u,

@@ -130,54 +130,21 @@ void launch_rk4_final(cudaStream_t st, int n, double *c, const double *k1, const
   if (n) k_rk4_final<<<grid_for(n), kB, 0, st>>>(n, c, k1, k2, k3, k4);
 }
 
-// dt = cfl * d_min / lambda_max / (2p + 1) (time_integrator.cu:217), the
-// last step shortened to land on endtime (:226-231)
-__device__ __forceinline__ void compute_dt_body(DevScalars *ds, int p) {
-  double lam = __longlong_as_double((long long)ds->lam_bits);
-  double dt = ds->fixed_dt > 0 ? ds->fixed_dt : ds->cfl * ds->dmin / lam / (2. * p + 1.);
-  if (!(dt == dt) || !(dt > 0) || isinf(dt)) {
-    ds->status = 4;
-    dt = 0.0;
-  }
-  ds->last = 0;
-  if (ds->endtime > 0) {
-    if (ds->t + dt > ds->endtime) {
-      dt = ds->endtime - ds->t;
-      ds->last = 1;
-    }
-    if (dt < 0) dt = 0;
-  }
-  ds->dt = dt;
-}
-__device__ __forceinline__ void advance_t_body(DevScalars *ds) {
-  if (ds->dt > 0) ds->steps++;
-  ds->t = ds->last ? ds->endtime : ds->t + ds->dt;
-}
-__global__ void k_compute_dt(DevScalars *ds, int p) { compute_dt_body(ds, p); }
-__global__ void k_reset_lambda(DevScalars *ds) { ds->lam_bits = 0ull; }
-__global__ void k_advance_t(DevScalars *ds) { advance_t_body(ds); }
+__global__ void k_advance_t(DevScalars *ds) { advance_time(ds); }
 
-// one thread per problem of a batch
-__global__ void k_batch_reset_lambda(BatchProb *pr, int n) {
+__global__ void k_batch_put_scalars(BatchProb *pr, const DevScalars *h, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) pr[i].ds->lam_bits = 0ull;
+  if (i < n) *pr[i].ds = h[i];
 }
-__global__ void k_batch_compute_dt(BatchProb *pr, int n) {
+__global__ void k_batch_get_scalars(BatchProb *pr, DevScalars *h, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) compute_dt_body(pr[i].ds, pr[i].p);
+  if (i < n) h[i] = *pr[i].ds;
 }
-__global__ void k_batch_advance_t(BatchProb *pr, int n) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) advance_t_body(pr[i].ds);
+void launch_batch_put_scalars(cudaStream_t st, BatchProb *probs, const DevScalars *h, int n) {
+  if (n) k_batch_put_scalars<<<grid_for(n), kB, 0, st>>>(probs, h, n);
 }
-void launch_batch_reset_lambda(cudaStream_t st, BatchProb *probs, int n) {
-  if (n) k_batch_reset_lambda<<<grid_for(n), kB, 0, st>>>(probs, n);
-}
-void launch_batch_compute_dt(cudaStream_t st, BatchProb *probs, int n) {
-  if (n) k_batch_compute_dt<<<grid_for(n), kB, 0, st>>>(probs, n);
-}
-void launch_batch_advance_t(cudaStream_t st, BatchProb *probs, int n) {
-  if (n) k_batch_advance_t<<<grid_for(n), kB, 0, st>>>(probs, n);
+void launch_batch_get_scalars(cudaStream_t st, BatchProb *probs, DevScalars *h, int n) {
+  if (n) k_batch_get_scalars<<<grid_for(n), kB, 0, st>>>(probs, h, n);
 }
 
 struct BatchTabsImage {
@@ -193,8 +160,6 @@ void build_batch_tabs(const void *t1, const void *t2, const void *t3, void *dst)
   if (t3) std::memcpy(&b->t3, t3, sizeof(Tab<3>));
 }
 
-void launch_compute_dt(cudaStream_t st, DevScalars *ds, int p) { k_compute_dt<<<1, 1, 0, st>>>(ds, p); }
-void launch_reset_lambda(cudaStream_t st, DevScalars *ds) { k_reset_lambda<<<1, 1, 0, st>>>(ds); }
 void launch_advance_t(cudaStream_t st, DevScalars *ds) { k_advance_t<<<1, 1, 0, st>>>(ds); }
 
 }  // namespace dg

@@ -51,10 +51,20 @@ struct DevScalars {
   double cfl;       // CFL number
   double fixed_dt;  // > 0: use it instead of the CFL step
   double endtime;   // > 0: shorten the last step to land here
-  unsigned long long lam_bits;  // max wave speed (non-negative double as bits)
+  unsigned long long lam_bits;  // max wave speed (non-negative double as bits), 0 between steps
+  double lam;       // max wave speed of the last CFL step
   long long steps;  // steps taken with dt > 0
   int status;       // 0 ok, 4 NaN or non-positive CFL step
   int last;         // 1 when this step was shortened to land on endtime
+  unsigned ticket;  // blocks of the wave-speed kernel that have finished, 0 between steps
+  int pending;      // 1: dt belongs to a step whose end t has not reached yet
+};
+
+// what the last block of the wave-speed kernel does once the maximum is known
+enum CflMode {
+  CFL_ONLY = 0,   // dt
+  CFL_SSP = 1,    // t to the end of the step before, if one is pending, then dt, now pending
+  CFL_RK = 2      // dt, then t to the end of the step (the RK4 / RK2 loops' stage times)
 };
 
 struct Ctx {
@@ -134,9 +144,9 @@ const BatchOps &batch_ops_maxwell();
 size_t batch_tabs_bytes();
 // copies the Tab<1>, Tab<2>, Tab<3> images into a BatchTabs image
 void build_batch_tabs(const void *t1, const void *t2, const void *t3, void *dst);
-void launch_batch_reset_lambda(cudaStream_t st, BatchProb *probs, int n);
-void launch_batch_compute_dt(cudaStream_t st, BatchProb *probs, int n);
-void launch_batch_advance_t(cudaStream_t st, BatchProb *probs, int n);
+// the members' device scalars from, and back into, one array of n
+void launch_batch_put_scalars(cudaStream_t st, BatchProb *probs, const DevScalars *h, int n);
+void launch_batch_get_scalars(cudaStream_t st, BatchProb *probs, DevScalars *h, int n);
 
 struct Ops {
   // edge traces of u; flattens (in u) any element with a non-physical trace
@@ -150,8 +160,8 @@ struct Ops {
   void (*limit)(const Ctx &, double *u);
   // limit, then trace
   void (*limit_trace)(const Ctx &, double *u);
-  // max cell-mean wave speed into ds->lam_bits (atomic max)
-  void (*lambda)(const Ctx &, const double *u);
+  // max cell-mean wave speed and, from it, the time step (CflMode)
+  void (*lambda)(const Ctx &, const double *u, int mode);
   // L2 projection of the problem's initial condition
   void (*init)(const Ctx &, double *u);
   // per-block partial sums of the squared L2 error, [nblocks][N]; returns nblocks
@@ -205,9 +215,6 @@ void launch_axpby(cudaStream_t st, int n, double a, const double *x, double b, d
 void launch_xpay(cudaStream_t st, int n, const double *x, double a, const double *y, double *z);
 void launch_rk4_final(cudaStream_t st, int n, double *c, const double *k1, const double *k2,
                       const double *k3, const double *k4);
-// dt from lam_bits (or fixed_dt), clamped to endtime; order p for the (2p+1)
-void launch_compute_dt(cudaStream_t st, DevScalars *ds, int p);
-void launch_reset_lambda(cudaStream_t st, DevScalars *ds);
 void launch_advance_t(cudaStream_t st, DevScalars *ds);
 
 // ---- shallow-water tangent-linear / adjoint operators (dg_adjoint.cu) ----

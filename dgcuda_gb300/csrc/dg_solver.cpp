@@ -195,27 +195,26 @@ void fused_stage(dg_solver *s, double *us, const double *un, double *out, double
   if (lim) run(s, K_LIMIT, [&] { s->ops->limit_tr(s->ctx, out); });
 }
 
-void cfl(dg_solver *s) {
-  run(s, K_CFL, [&] { dg::launch_reset_lambda(s->st, s->ds); });
-  run(s, K_CFL, [&] { s->ops->lambda(s->ctx, s->U); });
-  run(s, K_CFL, [&] { dg::launch_compute_dt(s->st, s->ds, s->p); });
+// the CFL time step of U, and t where the scheme advances it (dg::CflMode)
+void cfl(dg_solver *s, int mode) {
+  run(s, K_CFL, [&] { s->ops->lambda(s->ctx, s->U, mode); });
 }
 
 // one time step of `scheme` on s->U (launch sequence, capturable)
 void one_step(dg_solver *s, int scheme) {
   const int n = (int)s->ndof_p;
   const double *dt = &s->ds->dt;
-  cfl(s);
+  // SSP-RK3's t stays at the start of the step until the next one begins; the
+  // RK4 / RK2 loops advance it first (time_integrator.cu:230)
+  cfl(s, scheme == DG_SSP_RK3 ? dg::CFL_SSP : dg::CFL_RK);
   if (scheme == DG_SSP_RK3) {
     // u1 = u + dt L(u); u2 = 3/4 u + 1/4 (u1 + dt L(u1)); u = 1/3 u + 2/3 (u2 + dt L(u2));
     // T holds the traces of u on entry (run_steps) and of the new u on exit
     fused_stage(s, s->U, nullptr, s->W, 0.0, 1.0, 1.0, 0.0, dt);
     fused_stage(s, s->W, s->U, s->W, 0.75, 0.25, 0.25, 1.0, dt);
     fused_stage(s, s->W, s->U, s->U, 1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0, 0.5, dt);
-    run(s, K_CFL, [&] { dg::launch_advance_t(s->st, s->ds); });
   } else if (scheme == DG_RK4) {
-    // time_integrator.cu:198-400: t advanced first, limiter on each increment
-    run(s, K_CFL, [&] { dg::launch_advance_t(s->st, s->ds); });
+    // time_integrator.cu:198-400: limiter on each increment
     double **k = s->k;
     stage(s, s->U, nullptr, k[0], 0, 0, 1, 0.0, dt);
     limit(s, k[0]);
@@ -232,7 +231,6 @@ void one_step(dg_solver *s, int scheme) {
     limit(s, s->U);
   } else {
     // midpoint RK2, time_integrator.cu:557-690
-    run(s, K_CFL, [&] { dg::launch_advance_t(s->st, s->ds); });
     double **k = s->k;
     stage(s, s->U, nullptr, k[0], 0, 0, 1, 0.0, dt);
     limit(s, k[0]);
@@ -338,9 +336,12 @@ dg_status set_scalar(dg_solver *s, size_t offset, const void *v, size_t bytes) {
   return DG_OK;
 }
 
+// the device scalars, t at the end of the last step
 dg_status read_scalars(dg_solver *s, dg::DevScalars *h) {
   CK(cudaMemcpyAsync(h, s->ds, sizeof *h, cudaMemcpyDeviceToHost, s->st));
   CK(cudaStreamSynchronize(s->st));
+  if (h->pending) dg::advance_time(h);
+  h->pending = 0;
   return DG_OK;
 }
 
@@ -945,12 +946,12 @@ extern "C" dg_status dg_cfl(dg_solver *s, double *dt, double *lambda_max, double
   h.status = 0;
   st = set_scalar(s, 0, &h, sizeof h);
   if (st != DG_OK) return st;
-  cfl(s);
+  cfl(s, dg::CFL_ONLY);
   collect_profile(s);
   st = read_scalars(s, &h);
   if (st != DG_OK) return st;
   if (dt) *dt = h.dt;
-  if (lambda_max) *lambda_max = __builtin_bit_cast(double, h.lam_bits);
+  if (lambda_max) *lambda_max = h.lam;
   if (d_min) *d_min = s->dmin;
   if (h.status == 4) return fail(DG_NAN, "wave speed is NaN");
   return DG_OK;
@@ -1139,6 +1140,7 @@ struct dg_batch {
   std::vector<char> tabs, fximg[4];
   dg::BatchProb *probs = nullptr;
   int *maps = nullptr;  // device: element/side/lambda block maps
+  dg::DevScalars *scal = nullptr;  // device: the members' scalars, in transit
   dg::BatchLaunch bl;
   cudaGraphExec_t graph = nullptr;
   long long graph_nodes = 0, launches = 0;
@@ -1234,9 +1236,7 @@ dg_status batch_build_maps(dg_batch *b) {
 // one SSP-RK3 step of every member (launch sequence, capturable)
 void batch_step_seq(dg_batch *b) {
   const dg::BatchLaunch &L = b->bl;
-  dg::launch_batch_reset_lambda(L.st, L.probs, L.nprob);
   b->ops->lambda(L);
-  dg::launch_batch_compute_dt(L.st, L.probs, L.nprob);
   const double tc[3] = {0.0, 1.0, 0.5};
   for (int stage = 0; stage < 3; stage++) {
     if (L.fused) {  // the limiter in the element epilogue, as the members' own steps
@@ -1249,20 +1249,26 @@ void batch_step_seq(dg_batch *b) {
     b->ops->element(L, stage);
     if (L.limiter) b->ops->limit_tr(L, stage);
   }
-  dg::launch_batch_advance_t(L.st, L.probs, L.nprob);
 }
 
 dg_status batch_run(dg_batch *b, int nsteps, double *t) {
   CK(cudaSetDevice(b->device));
-  for (size_t i = 0; i < b->m.size(); i++) {
+  const int n = (int)b->m.size();
+  std::vector<dg::DevScalars> hs(n);
+  for (int i = 0; i < n; i++) {
     dg_solver *s = b->m[i];
     CK(cudaStreamSynchronize(s->st));
-    dg::DevScalars h{};
+    dg::DevScalars &h = hs[i];
+    h = dg::DevScalars{};
     h.t = t ? t[i] : 0.0;
     h.one = 1.0;
     h.dmin = s->dmin;
     h.cfl = s->prm.cfl;
-    CK(cudaMemcpyAsync(s->ds, &h, sizeof h, cudaMemcpyHostToDevice, b->st));
+  }
+  // the members' scalars in one copy each way
+  CK(cudaMemcpyAsync(b->scal, hs.data(), n * sizeof hs[0], cudaMemcpyHostToDevice, b->st));
+  dg::launch_batch_put_scalars(b->st, b->probs, b->scal, n);
+  for (dg_solver *s : b->m) {
     // the reference limits once before its step loop (time_integrator.cu:178-184)
     if (b->limiter && s->np >= 3) {
       dg::Ctx c = s->ctx;
@@ -1291,12 +1297,14 @@ dg_status batch_run(dg_batch *b, int nsteps, double *t) {
     CK(cudaGraphLaunch(b->graph, b->st));
     b->launches += b->graph_nodes;
   }
+  dg::launch_batch_get_scalars(b->st, b->probs, b->scal, n);
+  CK(cudaMemcpyAsync(hs.data(), b->scal, n * sizeof hs[0], cudaMemcpyDeviceToHost, b->st));
   cudaError_t e = cudaStreamSynchronize(b->st);
   if (e != cudaSuccess) return cuda_fail(e, "batched step");
   int nan = 0;
-  for (size_t i = 0; i < b->m.size(); i++) {
-    dg::DevScalars h{};
-    CK(cudaMemcpy(&h, b->m[i]->ds, sizeof h, cudaMemcpyDeviceToHost));
+  for (int i = 0; i < n; i++) {
+    dg::DevScalars &h = hs[i];
+    if (h.pending) dg::advance_time(&h);
     if (t) t[i] = h.t;
     if (h.status == 4) nan = 1;
   }
@@ -1378,7 +1386,8 @@ extern "C" dg_status dg_batch_create(int n, dg_solver *const *members, dg_batch 
     q.ds = s->ds;
     q.q = s->q;
   }
-  if (cudaMalloc(&b->probs, sizeof(dg::BatchProb) * n) != cudaSuccess)
+  if (cudaMalloc(&b->probs, sizeof(dg::BatchProb) * n) != cudaSuccess ||
+      cudaMalloc(&b->scal, sizeof(dg::DevScalars) * n) != cudaSuccess)
     return bail(fail(DG_CUDA_ERROR, "cudaMalloc"));
   if (cudaMemcpy(b->probs, hp.data(), sizeof(dg::BatchProb) * n, cudaMemcpyHostToDevice) !=
       cudaSuccess)
@@ -1480,6 +1489,7 @@ extern "C" void dg_batch_destroy(dg_batch *b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   if (b->maps) cudaFree(b->maps);
   if (b->probs) cudaFree(b->probs);
+  if (b->scal) cudaFree(b->scal);
   for (int g = 0; g < dg::BatchLaunch::kGroups; g++) {
     if (b->bl.gst[g]) cudaStreamDestroy(b->bl.gst[g]);
     if (b->bl.join[g]) cudaEventDestroy(b->bl.join[g]);
