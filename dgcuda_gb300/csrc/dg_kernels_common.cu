@@ -57,51 +57,70 @@ void build_tab(int p, const dg_order_tables &src, void *dst) {
 static constexpr int kB = 256;
 static unsigned grid_for(size_t n) { return (unsigned)((n + kB - 1) / kB); }
 
+// Layout permutations: a thread takes one element through kRows rows of the
+// state, so its index is read once, kRows loads are in flight, and no index is
+// divided (state in / out at 2.1M triangles, p = 3, 40 rows: 380 / 303 us with one
+// thread per value and a 64-bit division, 209 / 207 us)
+constexpr int kRows = 8;
+static dim3 row_grid(int n, int rows) {
+  return dim3((unsigned)((n + kB - 1) / kB), (unsigned)((rows + kRows - 1) / kRows));
+}
+
+// CMP: also set *changed when any value differs (bitwise) from the one it
+// overwrites
+template <bool CMP>
 __global__ void k_permute_in(const double *__restrict__ user, double *__restrict__ in,
-                             const int *__restrict__ perm, int rows, int K, int Kp) {
-  size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)rows * Kp) return;
-  int r = (int)(idx / Kp), e = (int)(idx % Kp);
-  in[idx] = e < K ? user[(size_t)r * K + perm[e]] : 0.0;
+                             const int *__restrict__ perm, int rows, int K, int Kp,
+                             int *changed) {
+  const int e = blockIdx.x * kB + threadIdx.x;
+  if (e >= Kp) return;
+  const int r0 = blockIdx.y * kRows, o = e < K ? perm[e] : 0;
+  double v[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; r++)
+    v[r] = e < K && r0 + r < rows ? user[(size_t)(r0 + r) * K + o] : 0.0;
+  bool diff = false;
+#pragma unroll
+  for (int r = 0; r < kRows; r++)
+    if (r0 + r < rows) {
+      double *p = in + (size_t)(r0 + r) * Kp + e;
+      if (CMP) diff |= __double_as_longlong(*p) != __double_as_longlong(v[r]);
+      *p = v[r];
+    }
+  if (CMP && diff) *changed = 1;
 }
 
 __global__ void k_permute_out(const double *__restrict__ in, double *__restrict__ user,
                               const int *__restrict__ perm, int rows, int K, int Kp) {
-  size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)rows * K) return;
-  int r = (int)(idx / K), e = (int)(idx % K);
-  user[(size_t)r * K + perm[e]] = in[(size_t)r * Kp + e];
+  const int e = blockIdx.x * kB + threadIdx.x;
+  if (e >= K) return;
+  const int r0 = blockIdx.y * kRows, o = perm[e];
+  double v[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; r++) v[r] = r0 + r < rows ? in[(size_t)(r0 + r) * Kp + e] : 0.0;
+#pragma unroll
+  for (int r = 0; r < kRows; r++)
+    if (r0 + r < rows) user[(size_t)(r0 + r) * K + o] = v[r];
 }
 
 void launch_permute_in(cudaStream_t st, const double *user, double *internal, const int *perm,
                        int rows, int K, int Kp) {
-  size_t n = (size_t)rows * Kp;
-  if (n) k_permute_in<<<grid_for(n), kB, 0, st>>>(user, internal, perm, rows, K, Kp);
-}
-
-// permute_in that also sets *changed when any value differs (bitwise) from
-// the one it overwrites
-__global__ void k_permute_in_cmp(const double *__restrict__ user, double *__restrict__ in,
-                                 const int *__restrict__ perm, int rows, int K, int Kp,
-                                 int *changed) {
-  size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (size_t)rows * Kp) return;
-  int r = (int)(idx / Kp), e = (int)(idx % Kp);
-  const double v = e < K ? user[(size_t)r * K + perm[e]] : 0.0;
-  if (__double_as_longlong(in[idx]) != __double_as_longlong(v)) *changed = 1;
-  in[idx] = v;
+  if (rows > 0 && Kp > 0)
+    k_permute_in<false><<<row_grid(Kp, rows), kB, 0, st>>>(user, internal, perm, rows, K, Kp,
+                                                           nullptr);
 }
 
 void launch_permute_in_cmp(cudaStream_t st, const double *user, double *internal,
                            const int *perm, int rows, int K, int Kp, int *changed) {
-  size_t n = (size_t)rows * Kp;
-  if (n) k_permute_in_cmp<<<grid_for(n), kB, 0, st>>>(user, internal, perm, rows, K, Kp, changed);
+  if (rows > 0 && Kp > 0)
+    k_permute_in<true><<<row_grid(Kp, rows), kB, 0, st>>>(user, internal, perm, rows, K, Kp,
+                                                          changed);
 }
 
 void launch_permute_out(cudaStream_t st, const double *internal, double *user, const int *perm,
                         int rows, int K, int Kp) {
-  size_t n = (size_t)rows * K;
-  if (n) k_permute_out<<<grid_for(n), kB, 0, st>>>(internal, user, perm, rows, K, Kp);
+  if (rows > 0 && K > 0)
+    k_permute_out<<<row_grid(K, rows), kB, 0, st>>>(internal, user, perm, rows, K, Kp);
 }
 
 __global__ void k_axpby(int n, double a, const double *__restrict__ x, double b, double *y) {
