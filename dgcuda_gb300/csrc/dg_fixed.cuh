@@ -361,7 +361,8 @@ __device__ __forceinline__ void load_F(const double *const (&Fp)[3], const bool 
 // The element stage (element_body's inputs, outputs and rules) of the tile of
 // 32 elements from e0.  MODE 0: no traces; 1: the traces of the output into
 // T, with the positivity rule where a.check is set; 2: the same with the
-// limiter (mode 0 of the output is the stored mean a.M).
+// limiter (mode 0 of the output is the stored mean a.M); 3: as 1, and a.acc =
+// a.acc0 + a.ck dt L(us) beside the output (RK4).
 template <class Eq, int P, int MODE>
 __device__ __forceinline__ void element_tile(const FxTab<P> &tab, const EqP &q, const ElemArgs &a,
                                              int e0, double *st, int *mxs, int *flag) {
@@ -559,6 +560,17 @@ __device__ __forceinline__ void element_tile(const FxTab<P> &tab, const EqP &q, 
       for (int i = i0; i < NP; i++) c[i] = st[(i * N + n) * kPitch + lane];
     }
     const double sc = a.cc * *a.dtp * geo[4 * Kp + ec];
+    if constexpr (MODE == 3) {
+      const double sk = a.ck * *a.dtp * geo[4 * Kp + ec];
+      const double *in = a.acc0 + (size_t)(n * NP) * Kp + ec;
+      double r[NP];
+#pragma unroll
+      for (int i = 0; i < NP; i++)  // a flattened stage input counts as its mean here too
+        r[i] = fma(sk, c[i], badv && i > 0 && a.acc0 == a.us ? 0.0 : in[(size_t)i * Kp]);
+      if (live)
+#pragma unroll
+        for (int i = 0; i < NP; i++) a.acc[(size_t)(n * NP + i) * Kp + e] = r[i];
+    }
     const double *unn = a.un + (size_t)(n * NP) * Kp + ec;
     double *outn = a.out + (size_t)(n * NP) * Kp + ec;
 #pragma unroll

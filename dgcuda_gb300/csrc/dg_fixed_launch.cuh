@@ -16,6 +16,8 @@ void run_element(const Ctx &c, const ElemArgs &a, int mode) {
     launch(k_element_fx<Eq, P, 0>, blocks, S::kThreads, c.st, tab, *c.q, a);
   } else if (mode == 1) {
     launch(k_element_fx<Eq, P, 1>, blocks, S::kThreads, c.st, tab, *c.q, a);
+  } else if (mode == 3) {
+    launch(k_element_fx<Eq, P, 3>, blocks, S::kThreads, c.st, tab, *c.q, a);
   } else {
     if constexpr (Eq::kFusedLimiter)
       launch(k_element_fx<Eq, P, 2>, blocks, S::kThreads, c.st, tab, *c.q, a);

@@ -327,6 +327,9 @@ struct ElemArgs {
   const double *bslope;     // its slopes at the area points (fixed-point stage) or null
   const double *vtx;        // element vertices (rows of Kp): positions for a velocity field
   double *T;                // traces of out (TR)
+  double *acc;              // RK4 (fixed-point stage): acc = acc0 + ck dt L(us) beside out
+  const double *acc0;
+  double ck;
   const double *M;          // fused limiter: the means of out (k_means), rows of Kp
   const int *nbr;           // fused limiter: neighbours across faces 0..2, rows of Kp
   double ca, cb, cc;
@@ -1135,6 +1138,9 @@ struct Launch {
     a.bslope = c.m.bslope;
     a.vtx = c.m.vtx;
     a.T = T;
+    a.acc = nullptr;
+    a.acc0 = nullptr;
+    a.ck = 0.0;
     a.M = c.M;
     a.nbr = c.m.nbr;
     a.ca = ca;
@@ -1218,6 +1224,18 @@ struct Launch {
     DG_DISPATCH_P(if constexpr (fp64(P)) (
         launch(k_element<Eq, P, true>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q, a)));
   }
+  // element_tr() with the positivity rule that also adds ck dt L(us) to acc0
+  // into acc (RK4's weighted sum of the increments); only with c.fx
+  static void element_acc(const Ctx &c, double *us, const double *un, double *out, double ca,
+                          double cb, double cc, const double *dtp, double *acc,
+                          const double *acc0, double ck) {
+    if (!c.m.K) return;
+    ElemArgs a = eargs(c, us, un, out, ca, cb, cc, dtp, c.T, 1);
+    a.acc = acc;
+    a.acc0 = acc0;
+    a.ck = ck;
+    fx::element<Eq>(c, a, 3);
+  }
   static void bed_slopes(const Ctx &c, double *out) {
     if (!c.m.K) return;
     DG_DISPATCH_P((k_bed_slopes<P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(
@@ -1266,7 +1284,7 @@ struct Launch {
 
   static const Ops &ops() {
     static const Ops o = {trace,  face,       element,  limit,  limit_trace, lambda, init, l2err,
-                          element_tr, limit_tr, vertex, nullptr, nullptr, nullptr, nullptr};
+                          element_tr, limit_tr, element_acc, vertex, nullptr, nullptr, nullptr, nullptr};
     return o;
   }
 

@@ -213,6 +213,34 @@ void one_step(dg_solver *s, int scheme) {
     fused_stage(s, s->U, nullptr, s->W, 0.0, 1.0, 1.0, 0.0, dt);
     fused_stage(s, s->W, s->U, s->W, 0.75, 0.25, 0.25, 1.0, dt);
     fused_stage(s, s->W, s->U, s->U, 1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0, 0.5, dt);
+  } else if (s->ctx.fx && !(s->prm.limiter && s->np >= 3)) {
+    // RK4 and midpoint RK2 without the limiter: each stage writes the next
+    // one's input and its traces in its epilogue, and RK4's sum of the
+    // increments beside it, so there are no increments, combinations and
+    // trace passes of their own (Euler p = 2, 60k triangles, RK4: 479 -> 373 us a step)
+    double *in = s->k[0], *acc = s->k[1];
+    run(s, K_TRACE, [&] { s->ops->trace(s->ctx, s->U); });
+    auto rk = [&](double *us, double cb, double cc, double tcoef, const double *acc0, double ck) {
+      run(s, K_FACE, [&] { s->ops->face(s->ctx, &s->ds->t, tcoef); });
+      run(s, K_ELEMENT, [&] {
+        s->ops->element_acc(s->ctx, us, s->U, in, 1.0 - cb, cb, cc, dt, acc, acc0, ck);
+      });
+    };
+    if (scheme == DG_RK4) {  // inputs U + k1 / 2, U + k2 / 2, U + k3
+      rk(s->U, 1.0, 0.5, 0.0, s->U, 1.0 / 6.0);
+      rk(in, 0.0, 0.5, 0.5, acc, 1.0 / 3.0);
+      rk(in, 0.0, 1.0, 0.5, acc, 1.0 / 3.0);
+      run(s, K_FACE, [&] { s->ops->face(s->ctx, &s->ds->t, 1.0); });
+      run(s, K_ELEMENT, [&] {
+        s->ops->element(s->ctx, in, acc, s->U, 1.0, 0.0, 1.0 / 6.0, dt);
+      });
+    } else {
+      run(s, K_FACE, [&] { s->ops->face(s->ctx, &s->ds->t, 0.0); });
+      run(s, K_ELEMENT,
+          [&] { s->ops->element_tr(s->ctx, s->U, nullptr, in, 0.0, 1.0, 0.5, dt, 1); });
+      run(s, K_FACE, [&] { s->ops->face(s->ctx, &s->ds->t, 0.5); });
+      run(s, K_ELEMENT, [&] { s->ops->element(s->ctx, in, s->U, s->U, 1.0, 0.0, 1.0, dt); });
+    }
   } else if (scheme == DG_RK4) {
     // time_integrator.cu:198-400: limiter on each increment
     double **k = s->k;
