@@ -18,7 +18,7 @@
 // adjoint: (dL/du)^T Lbar and (dL/db)^T Lbar (with A^T).  The dot-product
 // test <Lbar, dL> = <ubar, du> + <bbar, db> holds to rounding.
 #pragma once
-#include "dg_kernels.cuh"
+#include "dg_fixed.cuh"
 
 namespace dg {
 
@@ -218,23 +218,19 @@ __global__ void __launch_bounds__(kBlock)
 // ---------------------------------------------------------------------------
 // TL element: dout = ca du^n + cb du_s + cc dt (1/J) [dV + dS], dS gathered
 // from dFh like the forward surface term.
-// ADJ element: with Rbar = cc dt (1/J) obar, writes
-//   ubar_s = cb obar + (dV/du)^T Rbar + (surface, gathered from UbL/UbR)
-// and adds (dV/db)^T Rbar to bbar.  The ca u^n term is applied by the caller.
-template <int P, bool ADJ>
+template <int P>
 __global__ void __launch_bounds__(kBlock)
-    k_sw_element_lin(const __grid_constant__ Tab<P> tab, const __grid_constant__ EqP q,
+    k_sw_element_tl(const __grid_constant__ Tab<P> tab, const __grid_constant__ EqP q,
                      const double *__restrict__ us, const double *__restrict__ bz_all,
                      const double *__restrict__ vin, const double *__restrict__ dbz_all,
                      const double *__restrict__ vn, double *__restrict__ vout,
-                     double *__restrict__ bbar, const double *__restrict__ F0,
-                     const double *__restrict__ F1, const int *__restrict__ esd,
+                     const double *__restrict__ F0, const int *__restrict__ esd,
                      const double *__restrict__ geo, double ca, double cb, double ccdt, int K,
                      int Kp) {
   constexpr int N = 3, NP = Tab<P>::NP, NQ = Tab<P>::NQ, N1 = Tab<P>::N1;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= K) return;
-  double c[N][NP], v[N][NP], acc[N][NP], bz[NP], dbz[NP], bb[NP];
+  double c[N][NP], v[N][NP], acc[N][NP], bz[NP], dbz[NP];
 #pragma unroll
   for (int n = 0; n < N; n++)
 #pragma unroll
@@ -246,19 +242,11 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
   for (int i = 0; i < NP; i++) {
     bz[i] = bz_all ? bz_all[(size_t)i * Kp + e] : 0.0;
-    dbz[i] = (!ADJ && dbz_all) ? dbz_all[(size_t)i * Kp + e] : 0.0;
-    bb[i] = 0.0;
+    dbz[i] = dbz_all ? dbz_all[(size_t)i * Kp + e] : 0.0;
   }
   const double xr = geo[e], yr = geo[(size_t)Kp + e], xs = geo[2 * (size_t)Kp + e],
                ys = geo[3 * (size_t)Kp + e], iJ = geo[4 * (size_t)Kp + e];
   const double g = q.g;
-  if (ADJ) {  // Rbar = cc dt (1/J) obar
-    const double f = ccdt * iJ;
-#pragma unroll
-    for (int n = 0; n < N; n++)
-#pragma unroll
-      for (int i = 0; i < NP; i++) v[n][i] *= f;
-  }
 #pragma unroll
   for (int k = 0; k < NQ; k++) {
     double U[N];
@@ -279,81 +267,38 @@ __global__ void __launch_bounds__(kBlock)
       bs = fma(bz[i], tab.GS[k][i], bs);
     }
     const double bx = fma(ys, br, -yr * bs), by = fma(xr, bs, -xs * br);
-    if (!ADJ) {
-      double dU[N];
+    double dU[N];
 #pragma unroll
-      for (int n = 0; n < N; n++) {
-        double a = v[n][0] * tab.B[k][0];
+    for (int n = 0; n < N; n++) {
+      double a = v[n][0] * tab.B[k][0];
 #pragma unroll
-        for (int i = 1; i < NP; i++) a = fma(v[n][i], tab.B[k][i], a);
-        dU[n] = a;
+      for (int i = 1; i < NP; i++) a = fma(v[n][i], tab.B[k][i], a);
+      dU[n] = a;
+    }
+    double dfx[N], dfy[N];
+    sw_jac_mul(uu, vv, uu, gh, 1.0, 0.0, dU, dfx);
+    sw_jac_mul(uu, vv, vv, gh, 0.0, 1.0, dU, dfy);
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      const double gr = fma(dfx[n], ys, -dfy[n] * xs), gs = fma(dfy[n], xr, -dfx[n] * yr);
+#pragma unroll
+      for (int i = 1; i < NP; i++)
+        acc[n][i] = fma(tab.GR[k][i], gr, fma(tab.GS[k][i], gs, acc[n][i]));
+    }
+    if (bz_all || dbz_all) {
+      double dbr = 0.0, dbs = 0.0;
+#pragma unroll
+      for (int i = 1; i < NP; i++) {
+        dbr = fma(dbz[i], tab.GR[k][i], dbr);
+        dbs = fma(dbz[i], tab.GS[k][i], dbs);
       }
-      double dfx[N], dfy[N];
-      sw_jac_mul(uu, vv, uu, gh, 1.0, 0.0, dU, dfx);
-      sw_jac_mul(uu, vv, vv, gh, 0.0, 1.0, dU, dfy);
+      const double dbx = fma(ys, dbr, -yr * dbs), dby = fma(xr, dbs, -xs * dbr);
+      const double sx = -g * fma(dU[0], bx, U[0] * dbx), sy = -g * fma(dU[0], by, U[0] * dby);
 #pragma unroll
-      for (int n = 0; n < N; n++) {
-        const double gr = fma(dfx[n], ys, -dfy[n] * xs), gs = fma(dfy[n], xr, -dfx[n] * yr);
-#pragma unroll
-        for (int i = 1; i < NP; i++)
-          acc[n][i] = fma(tab.GR[k][i], gr, fma(tab.GS[k][i], gs, acc[n][i]));
+      for (int i = 0; i < NP; i++) {
+        acc[1][i] = fma(sx, tab.B[k][i], acc[1][i]);
+        acc[2][i] = fma(sy, tab.B[k][i], acc[2][i]);
       }
-      if (bz_all || dbz_all) {
-        double dbr = 0.0, dbs = 0.0;
-#pragma unroll
-        for (int i = 1; i < NP; i++) {
-          dbr = fma(dbz[i], tab.GR[k][i], dbr);
-          dbs = fma(dbz[i], tab.GS[k][i], dbs);
-        }
-        const double dbx = fma(ys, dbr, -yr * dbs), dby = fma(xr, dbs, -xs * dbr);
-        const double sx = -g * fma(dU[0], bx, U[0] * dbx), sy = -g * fma(dU[0], by, U[0] * dby);
-#pragma unroll
-        for (int i = 0; i < NP; i++) {
-          acc[1][i] = fma(sx, tab.B[k][i], acc[1][i]);
-          acc[2][i] = fma(sy, tab.B[k][i], acc[2][i]);
-        }
-      }
-    } else {
-      double Ub[N], Gr[N], Gs[N];
-#pragma unroll
-      for (int n = 0; n < N; n++) {
-        double a = 0.0, b = 0.0;
-#pragma unroll
-        for (int i = 1; i < NP; i++) {
-          a = fma(tab.GR[k][i], v[n][i], a);
-          b = fma(tab.GS[k][i], v[n][i], b);
-        }
-        Gr[n] = a;
-        Gs[n] = b;
-      }
-      double fxb[N], fyb[N], zx[N], zy[N];
-#pragma unroll
-      for (int n = 0; n < N; n++) {
-        fxb[n] = fma(ys, Gr[n], -yr * Gs[n]);
-        fyb[n] = fma(xr, Gs[n], -xs * Gr[n]);
-      }
-      sw_jac_tmul(uu, vv, uu, gh, 1.0, 0.0, fxb, zx);
-      sw_jac_tmul(uu, vv, vv, gh, 0.0, 1.0, fyb, zy);
-#pragma unroll
-      for (int m = 0; m < N; m++) Ub[m] = zx[m] + zy[m];
-      if (bbar) {
-        double Sx = 0.0, Sy = 0.0;
-#pragma unroll
-        for (int i = 0; i < NP; i++) {
-          Sx = fma(tab.B[k][i], v[1][i], Sx);
-          Sy = fma(tab.B[k][i], v[2][i], Sy);
-        }
-        Ub[0] = fma(-g, fma(bx, Sx, by * Sy), Ub[0]);
-        const double hb = -g * U[0];
-        const double bxb = hb * Sx, byb = hb * Sy;  // adjoints of bx, by
-        const double brb = fma(ys, bxb, -xs * byb), bsb = fma(xr, byb, -yr * bxb);
-#pragma unroll
-        for (int i = 1; i < NP; i++) bb[i] = fma(tab.GR[k][i], brb, fma(tab.GS[k][i], bsb, bb[i]));
-      }
-#pragma unroll
-      for (int n = 0; n < N; n++)
-#pragma unroll
-        for (int i = 0; i < NP; i++) acc[n][i] = fma(tab.B[k][i], Ub[n], acc[n][i]);
     }
   }
   // surface
@@ -367,36 +312,294 @@ __global__ void __launch_bounds__(kBlock)
       const int jj = right ? (N1 - 1 - j) : j;
 #pragma unroll
       for (int n = 0; n < N; n++) {
-        double fv;
-        if (!ADJ) fv = (right ? 1.0 : -1.0) * F0[so + jj * N + n];
-        else fv = right ? F1[so + jj * N + n] : F0[so + jj * N + n];
+        const double fv = (right ? 1.0 : -1.0) * F0[so + jj * N + n];
 #pragma unroll
         for (int i = 0; i < NP; i++) acc[n][i] = fma(fv, tab.E[f][j][i], acc[n][i]);
       }
     }
   }
-  if (!ADJ) {
-    const double s = ccdt * iJ;
+  const double s = ccdt * iJ;
 #pragma unroll
-    for (int n = 0; n < N; n++)
+  for (int n = 0; n < N; n++)
 #pragma unroll
-      for (int i = 0; i < NP; i++) {
-        const size_t o = (size_t)(n * NP + i) * Kp + e;
-        double r = fma(s, acc[n][i], cb * v[n][i]);
-        if (ca != 0.0) r = fma(ca, vn[o], r);
-        vout[o] = r;
+    for (int i = 0; i < NP; i++) {
+      const size_t o = (size_t)(n * NP + i) * Kp + e;
+      double r = fma(s, acc[n][i], cb * v[n][i]);
+      if (ca != 0.0) r = fma(ca, vn[o], r);
+      vout[o] = r;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The adjoint element stage with its contractions in fixed point (dg_fixed.cuh:
+// one warp per variable, one lane per element).  With v = ccdt (1/J) obar,
+//   ubar = cb obar + (dV/du)^T v + (surface, gathered from UbL / UbR)
+//          [+ a0 x0 + a1 x1]
+// and bbar += (dV/db)^T v.  The contractions: U(q) = B us, the projections of
+// v on the gradients and (momenta) on the basis at the area points, and back
+// from the points' adjoints and the side terms to the modes.  With Tv, the
+// traces of tc (1/J) ubar, the next stage's k_lin_trace, follow.
+// Before, p = 2, 45k triangles, us a stage: FP64 element 129, k_lin_trace 24,
+// combination 6 (face 59, forward traces 9); a gradient over 10 steps 9.42 ->
+// 5.77 ms.
+struct AdjArgs {
+  const double *us, *obar, *x0, *x1;  // x0, x1 null: no extra terms
+  double *ubar, *bbar, *Tv;           // Tv null: no traces
+  const double *F0, *F1, *bslope, *geo;
+  const int *esd;
+  double cb, ccdt, a0, a1, tc;
+  int K, Kp;
+};
+
+template <int P>
+__global__ void __launch_bounds__(96, P <= 2 ? 8 : 5)
+    k_adj_element_fx(const __grid_constant__ fx::FxTab<P> tab, const __grid_constant__ EqP q,
+                     const __grid_constant__ AdjArgs a) {
+  using namespace fx;
+  constexpr int N = 3, NP = Tab<P>::NP, NQ = Tab<P>::NQ, N1 = P + 1, NF = 3 * N1;
+  // rows of kPitch doubles: block b of N NQ rows, variable n at point k in row
+  // (b NQ + k) N + n: b = 0 U, then its adjoint; 1, 2 the projections on the
+  // gradients; the momenta's on the basis, then the slopes' adjoints, in
+  // rows 3 NQ N + 2 k + (n - 1)
+  __shared__ double st[(3 * NQ * N + 2 * NQ) * kPitch];
+  __shared__ int mxs[(N + 1) * N * kTile];
+  const int lane = threadIdx.x & 31, n = threadIdx.x >> 5, e0 = blockIdx.x * kTile;
+  const int e = e0 + lane, ec = e < a.K ? e : a.K - 1;
+  const bool live = e < a.K;
+  const size_t Kp = a.Kp;
+  const double *geo = a.geo;
+  const double iJ = geo[4 * Kp + ec];
+  auto at = [&](int b, int k, int v) -> double & { return st[((b * NQ + k) * N + v) * kPitch + lane]; };
+  auto src = [&](int k, int v) -> double & { return st[(3 * NQ * N + 2 * k + (v - 1)) * kPitch + lane]; };
+  {  // U(q)
+    double c[NP];
+    int mx = 0;
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+      c[i] = a.us[(size_t)(n * NP + i) * Kp + ec];
+      mx = max(mx, abs_hi(c[i]));
+    }
+    const Row row = make_row(mx);
+    int h[NP], l[NP];
+#pragma unroll
+    for (int i = 0; i < NP; i++) to_limbs(c[i], row, h[i], l[i]);
+    const int base = base_exp(row, tab.eB);
+#pragma unroll
+    for (int k = 0; k < NQ; k++) {
+      Sum s;
+      zero(s);
+#pragma unroll
+      for (int i = 0; i < NP; i++) mac(s, h[i], l[i], tab.B[k][i]);
+      at(0, k, n) = finish(s, base);
+    }
+    if (row.odd()) fix(&at(0, 0, n), N * kPitch, NQ, row);
+  }
+  {  // v's projections
+    const double f = a.ccdt * iJ;
+    double c[NP];
+    int mx = 0;
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+      c[i] = f * a.obar[(size_t)(n * NP + i) * Kp + ec];
+      mx = max(mx, abs_hi(c[i]));
+    }
+    const Row row = make_row(mx);
+    int h[NP], l[NP];
+#pragma unroll
+    for (int i = 0; i < NP; i++) to_limbs(c[i], row, h[i], l[i]);
+    const int base = base_exp(row, tab.eP), baseB = base_exp(row, tab.eB);
+#pragma unroll
+    for (int k = 0; k < NQ; k++) {
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        Sum s;
+        zero(s);
+#pragma unroll
+        for (int i = 1; i < NP; i++) mac(s, h[i], l[i], tab.G[k][b][i]);
+        at(1 + b, k, n) = finish(s, base);
       }
-  } else {
+      if (n > 0) {
+        Sum s;
+        zero(s);
 #pragma unroll
-    for (int n = 0; n < N; n++)
-#pragma unroll
-      for (int i = 0; i < NP; i++) {
-        const size_t o = (size_t)(n * NP + i) * Kp + e;
-        vout[o] = fma(cb, vn[o], acc[n][i]);
+        for (int i = 0; i < NP; i++) mac(s, h[i], l[i], tab.B[k][i]);
+        src(k, n) = finish(s, baseB);
       }
-    if (bbar)
+    }
+    if (row.odd()) {
+      fix(&at(1, 0, n), N * kPitch, 2 * NQ, row);
+      if (n > 0) fix(&src(0, n), 2 * kPitch, NQ, row);
+    }
+  }
+  // the side terms, read after the points
+  const double *Fp[3];
+  bool right[3];
 #pragma unroll
-      for (int i = 0; i < NP; i++) bbar[(size_t)i * Kp + e] += bb[i];
+  for (int f = 0; f < 3; f++) {
+    const int sd = a.esd[(size_t)f * Kp + ec];
+    right[f] = sd & 1;
+    Fp[f] = (right[f] ? a.F1 : a.F0) + (size_t)(sd >> 1) * (N1 * N) + n;
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(Fp[f]));
+  }
+  __syncthreads();
+  {  // the points' adjoints; the warps share the points out
+    const double xr = geo[ec], yr = geo[Kp + ec], xs = geo[2 * Kp + ec], ys = geo[3 * Kp + ec];
+    int mx[N + 1] = {0, 0, 0, 0};
+#pragma unroll 1
+    for (int k = n; k < NQ; k += N) {
+      const double U0 = at(0, k, 0), ih = rcp(U0);
+      const double uu = at(0, k, 1) * ih, vv = at(0, k, 2) * ih, gh = q.g * U0;
+      double fxb[N], fyb[N], zx[N], zy[N];
+#pragma unroll
+      for (int v = 0; v < N; v++) {
+        const double Gr = at(1, k, v), Gs = at(2, k, v);
+        fxb[v] = fma(ys, Gr, -yr * Gs);
+        fyb[v] = fma(xr, Gs, -xs * Gr);
+      }
+      sw_jac_tmul(uu, vv, uu, gh, 1.0, 0.0, fxb, zx);
+      sw_jac_tmul(uu, vv, vv, gh, 0.0, 1.0, fyb, zy);
+      double Ub[N];
+#pragma unroll
+      for (int v = 0; v < N; v++) Ub[v] = zx[v] + zy[v];
+      if (a.bbar) {
+        const double bx = a.bslope ? a.bslope[(size_t)k * Kp + ec] : 0.0;
+        const double by = a.bslope ? a.bslope[(size_t)(NQ + k) * Kp + ec] : 0.0;
+        const double Sx = src(k, 1), Sy = src(k, 2);
+        Ub[0] = fma(-q.g, fma(bx, Sx, by * Sy), Ub[0]);
+        const double hb = -q.g * U0;
+        const double bxb = hb * Sx, byb = hb * Sy;  // adjoints of bx, by
+        const double brb = fma(ys, bxb, -xs * byb), bsb = fma(xr, byb, -yr * bxb);
+        src(k, 1) = brb;
+        src(k, 2) = bsb;
+        mx[N] = max(mx[N], max(abs_hi(brb), abs_hi(bsb)));
+      }
+#pragma unroll
+      for (int v = 0; v < N; v++) {
+        at(0, k, v) = Ub[v];
+        mx[v] = max(mx[v], abs_hi(Ub[v]));
+      }
+    }
+#pragma unroll
+    for (int v = 0; v <= N; v++) mxs[(v * N + n) * kTile + lane] = mx[v];
+  }
+  __syncthreads();
+  if (n == 0 && a.bbar) {  // the bed's adjoint: the variable without projections on the basis
+    int mx = 0;
+#pragma unroll
+    for (int w = 0; w < N; w++) mx = max(mx, mxs[(N * N + w) * kTile + lane]);
+    const Row row = make_row(mx);
+    Sum s[NP];
+#pragma unroll
+    for (int i = 1; i < NP; i++) zero(s[i]);
+#pragma unroll
+    for (int k = 0; k < NQ; k++)
+#pragma unroll
+      for (int b = 0; b < 2; b++) {
+        int h, l;
+        to_limbs(src(k, 1 + b), row, h, l);
+#pragma unroll
+        for (int i = 1; i < NP; i++) mac(s[i], h, l, tab.G[k][b][i]);
+      }
+    const int base = base_exp(row, tab.eP);
+    double r[NP];
+    r[0] = 0.0;
+#pragma unroll
+    for (int i = 1; i < NP; i++) r[i] = finish(s[i], base);
+    if (row.odd()) {  // through the slopes' rows, which are free now
+#pragma unroll
+      for (int i = 1; i < NP; i++) st[(3 * NQ * N + i) * kPitch + lane] = r[i];
+      fix(&st[(3 * NQ * N + 1) * kPitch + lane], kPitch, NP - 1, row);
+#pragma unroll
+      for (int i = 1; i < NP; i++) r[i] = st[(3 * NQ * N + i) * kPitch + lane];
+    }
+    if (live)
+#pragma unroll
+      for (int i = 1; i < NP; i++) a.bbar[(size_t)i * Kp + e] += r[i];
+  }
+  double c[NP];
+  {
+    double F[NF];
+#pragma unroll
+    for (int f = 0; f < 3; f++)
+#pragma unroll
+      for (int j = 0; j < N1; j++) F[f * N1 + j] = Fp[f][(right[f] ? N1 - 1 - j : j) * N];
+    int mx = 0;
+#pragma unroll
+    for (int w = 0; w < N; w++) mx = max(mx, mxs[(n * N + w) * kTile + lane]);
+#pragma unroll
+    for (int k = 0; k < NF; k++) mx = max(mx, abs_hi(F[k]));
+    const Row row = make_row(mx);
+    Sum s[NP];
+#pragma unroll
+    for (int i = 0; i < NP; i++) zero(s[i]);
+#pragma unroll
+    for (int k = 0; k < NF; k++) {
+      int h, l;
+      to_limbs(F[k], row, h, l);
+#pragma unroll
+      for (int i = 0; i < NP; i++) mac(s[i], h, l, tab.S[k][i]);
+    }
+#pragma unroll
+    for (int k = 0; k < NQ; k++) {
+      int h, l;
+      to_limbs(at(0, k, n), row, h, l);
+#pragma unroll
+      for (int i = 0; i < NP; i++) mac(s[i], h, l, tab.Q[k][i]);
+    }
+    const int base = base_exp(row, tab.eP);
+#pragma unroll
+    for (int i = 0; i < NP; i++) c[i] = finish(s[i], base);
+    if (row.odd()) {  // through the thread's own projection rows, which are free now
+#pragma unroll
+      for (int i = 0; i < NP; i++) at(1, i, n) = c[i];
+      fix(&at(1, 0, n), N * kPitch, NP, row);
+#pragma unroll
+      for (int i = 0; i < NP; i++) c[i] = at(1, i, n);
+    }
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+      const size_t o = (size_t)(n * NP + i) * Kp + ec;
+      double v = fma(a.cb, a.obar[o], c[i]);
+      if (a.x0) v += fma(a.a0, a.x0[o], a.a1 * a.x1[o]);
+      c[i] = v;
+    }
+    if (live)
+#pragma unroll
+      for (int i = 0; i < NP; i++) a.ubar[(size_t)(n * NP + i) * Kp + e] = c[i];
+  }
+  if (!a.Tv) return;
+  {  // traces of tc (1/J) ubar
+    const double f = a.tc * iJ;
+    int mx = 0;
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+      c[i] *= f;
+      mx = max(mx, abs_hi(c[i]));
+    }
+    const Row row = make_row(mx);
+    int h[NP], l[NP];
+#pragma unroll
+    for (int i = 0; i < NP; i++) to_limbs(c[i], row, h[i], l[i]);
+    const int base = base_exp(row, tab.eE);
+#pragma unroll
+    for (int k = 0; k < NF; k++) {
+      Sum s;
+      zero(s);
+#pragma unroll
+      for (int i = 0; i < NP; i++) mac(s, h[i], l[i], tab.E[k][i]);
+      st[(k * N + n) * kPitch + lane] = finish(s, base);
+    }
+    if (row.odd()) fix(&st[n * kPitch + lane], N * kPitch, NF, row);
+    __syncthreads();
+    constexpr int C = NF * N;
+#pragma unroll 2
+    for (int el = n; el < kTile; el += N) {
+      if (e0 + el >= a.K) break;
+      double *Te = a.Tv + (size_t)(e0 + el) * C;
+#pragma unroll
+      for (int r = 0; r < C; r += 32)
+        if (r + lane < C) Te[r + lane] = st[(r + lane) * kPitch + el];
+    }
   }
 }
 

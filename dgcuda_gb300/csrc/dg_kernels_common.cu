@@ -123,10 +123,6 @@ void launch_permute_out(cudaStream_t st, const double *internal, double *user, c
     k_permute_out<<<row_grid(K, rows), kB, 0, st>>>(internal, user, perm, rows, K, Kp);
 }
 
-__global__ void k_axpby(int n, double a, const double *__restrict__ x, double b, double *y) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) y[i] = a * x[i] + b * y[i];
-}
 __global__ void k_xpay(int n, const double *x, double a, const double *y, double *z) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) z[i] = x[i] + a * y[i];  // rk_tempstorage, time_integrator.cu:107-113
@@ -138,9 +134,6 @@ __global__ void k_rk4_final(int n, double *c, const double *__restrict__ k1,
   if (i < n) c[i] += k1[i] / 6. + k2[i] / 3. + k3[i] / 3. + k4[i] / 6.;
 }
 
-void launch_axpby(cudaStream_t st, int n, double a, const double *x, double b, double *y) {
-  if (n) k_axpby<<<grid_for(n), kB, 0, st>>>(n, a, x, b, y);
-}
 void launch_xpay(cudaStream_t st, int n, const double *x, double a, const double *y, double *z) {
   if (n) k_xpay<<<grid_for(n), kB, 0, st>>>(n, x, a, y, z);
 }

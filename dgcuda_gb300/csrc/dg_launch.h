@@ -214,8 +214,6 @@ void launch_permute_in_cmp(cudaStream_t st, const double *user, double *internal
                            const int *perm, int rows, int K, int Kp, int *changed);
 void launch_permute_out(cudaStream_t st, const double *internal, double *user, const int *perm,
                         int rows, int K, int Kp);
-// y = a * x + b * y over n entries (RK4 / RK2 combinations), dt-scaled when dts != 0
-void launch_axpby(cudaStream_t st, int n, double a, const double *x, double b, double *y);
 // z = x + a * y
 void launch_xpay(cudaStream_t st, int n, const double *x, double a, const double *y, double *z);
 void launch_rk4_final(cudaStream_t st, int n, double *c, const double *k1, const double *k2,
@@ -231,12 +229,23 @@ bool tl_face(const Ctx &c, const double *Tv, double *dFh);
 bool adj_face(const Ctx &c, const double *Tbar, double *UbL, double *UbR);
 bool tl_element(const Ctx &c, const double *us, const double *dus, const double *db,
                 const double *dun, double *dout, double ca, double cb, double ccdt);
-bool adj_element(const Ctx &c, const double *us, const double *obar, double *ubar_s,
-                 double *bbar, const double *UbL, const double *UbR, double cb, double ccdt);
+// one stage of the reverse sweep: ubar = cb obar + ccdt (dL/du)^T obar at the
+// stage input us [+ a0 x0 + a1 x1; x0 may be ubar], bbar += ccdt (dL/db)^T obar.
+// Tv: the traces of ccdt (1/J) obar for adj_face; with next_ccdt != 0 the stage
+// leaves those of the next one there, whose obar is this ubar
+struct AdjStage {
+  double *us = nullptr;
+  const double *obar = nullptr, *x0 = nullptr, *x1 = nullptr;
+  double *ubar = nullptr, *bbar = nullptr, *Tv = nullptr;
+  double cb = 0, ccdt = 0, a0 = 0, a1 = 0, next_ccdt = 0;
+};
+bool adj_element(const Ctx &c, const AdjStage &g, const double *UbL, const double *UbR);
 void launch_sample(cudaStream_t st, const double *u, const int *el, const double *phi, int nrec,
                    int np, int Kp, double *out);
-void launch_sample_adj(cudaStream_t st, double *ubar, const int *el, const double *phi, int nrec,
-                       int np, int Kp, const double *sbar);
+// next: nrec links to the following receiver in the same element (-1: none),
+// then nrec flags, 1 where a receiver before it shares the element
+void launch_sample_adj(cudaStream_t st, double *ubar, const int *el, const int *next,
+                       const double *phi, int nrec, int np, int Kp, const double *sbar);
 
 // what other files need to launch a solver's kernels
 struct SolverView {

@@ -1565,14 +1565,17 @@ void tl_stage(dg_solver *s, double *us, const double *dus, const double *db, con
   run(s, K_ELEMENT, [&] { dg::tl_element(c, us, dus, db, dun, dout, ca, cb, ccdt); });
 }
 
-// ubar_s = cb obar + ccdt (dL/du)^T obar ; bbar += ccdt (dL/db)^T obar
-void adj_stage(dg_solver *s, double *us, const double *obar, double *ubar_s, double *bbar,
-               double cb, double ccdt, const LinBufs &lb) {
-  fwd_traces(s, us);
+// one stage of the reverse sweep; traced: lb.Tv holds the traces of g.obar that
+// the stage before left (AdjStage::next_ccdt)
+void adj_stage(dg_solver *s, dg::AdjStage g, bool traced, const LinBufs &lb) {
+  fwd_traces(s, g.us);
   const dg::Ctx &c = s->ctx;
-  run(s, K_TRACE, [&] { dg::lin_trace(c, obar, s->m.geo + 4 * (size_t)s->m.Kp, ccdt, lb.Tv); });
+  g.Tv = lb.Tv;
+  if (!traced)
+    run(s, K_TRACE,
+        [&] { dg::lin_trace(c, g.obar, s->m.geo + 4 * (size_t)s->m.Kp, g.ccdt, lb.Tv); });
   run(s, K_FACE, [&] { dg::adj_face(c, lb.Tv, lb.F0, lb.F1); });
-  run(s, K_ELEMENT, [&] { dg::adj_element(c, us, obar, ubar_s, bbar, lb.F0, lb.F1, cb, ccdt); });
+  run(s, K_ELEMENT, [&] { dg::adj_element(c, g, lb.F0, lb.F1); });
 }
 
 dg_status lin_check(dg_solver *s) {
@@ -1638,7 +1641,13 @@ extern "C" dg_status dg_rhs_adjoint(dg_solver *s, double t, const double *C, con
   dg::launch_permute_in(s->st, s->ubuf, lb_in, s->m.perm, rows, s->K, s->m.Kp);
   CK(cudaMemsetAsync(bb, 0, (size_t)s->np * s->m.Kp * sizeof(double), s->st));
   (void)t;
-  adj_stage(s, u, lb_in, out, bb, 0.0, 1.0, lb);
+  dg::AdjStage g;
+  g.us = u;
+  g.obar = lb_in;
+  g.ubar = out;
+  g.bbar = bb;
+  g.ccdt = 1.0;
+  adj_stage(s, g, false, lb);
   dg::launch_permute_out(s->st, out, s->ubuf, s->m.perm, rows, s->K, s->m.Kp);
   CK(cudaMemcpyAsync(Cbar, s->ubuf, n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
   if (bbar) {
@@ -1656,7 +1665,7 @@ struct dg_adjoint {
   dg_solver *s = nullptr;
   int nrec = 0, nsteps = 0, every = 1, ckpt = 50;
   double dt = 0, t0 = 0;
-  int *rec_el = nullptr;
+  int *rec_el = nullptr, *rec_next = nullptr;  // elements; links as launch_sample_adj takes them
   double *rec_phi = nullptr, *samples = nullptr, *sbar = nullptr;
   std::vector<double *> cks;                  // checkpoints u^{k ckpt}
   std::vector<double *> seg;                  // 3 ckpt states of a segment: u^n, u1, u2
@@ -1668,7 +1677,7 @@ struct dg_adjoint {
   size_t store_n = 0;
   double *ufinal = nullptr;                   // the forward run's final state
   double t_end = 0;                           // and its time
-  double *ub = nullptr, *ub1 = nullptr, *ub2 = nullptr, *acc = nullptr, *bbar = nullptr;
+  double *ub = nullptr, *ub1 = nullptr, *ub2 = nullptr, *bbar = nullptr;
   double *du = nullptr, *dw = nullptr, *dbi = nullptr;
   std::vector<void *> mem;
 };
@@ -1686,18 +1695,17 @@ dg_status amalloc(dg_adjoint *a, T **p, size_t n) {
 
 // one SSP-RK3 step of fixed dt through the fused stages (the adjoint
 // excludes the limiter, and without it a fused stage gives the bits of the
-// unfused one: its element epilogue writes the traces k_trace would compute);
-// keeps the stage inputs u1, u2 when given.  T must hold the traces of U, or
-// need_trace asks for them (the first step of a run or of a segment).
-void plain_step(dg_solver *s, double *u1keep, double *u2keep, bool need_trace) {
-  const size_t bytes = s->ndof_p * sizeof(double);
+// unfused one: its element epilogue writes the traces k_trace would compute),
+// from u to next, which may be u, by the stage states u1 and u2, which may
+// be one buffer: where the states are kept, the stages write them where they
+// stay.  T must hold the traces of u, or need_trace asks for them (the first
+// step of a run or of a segment).
+void plain_step(dg_solver *s, double *u, double *u1, double *u2, double *next, bool need_trace) {
   const double *dt = &s->ds->dt;
-  if (need_trace) run(s, K_TRACE, [&] { s->ops->trace(s->ctx, s->U); });
-  fused_stage(s, s->U, nullptr, s->W, 0.0, 1.0, 1.0, 0.0, dt);
-  if (u1keep) cudaMemcpyAsync(u1keep, s->W, bytes, cudaMemcpyDeviceToDevice, s->st);
-  fused_stage(s, s->W, s->U, s->W, 0.75, 0.25, 0.25, 1.0, dt);
-  if (u2keep) cudaMemcpyAsync(u2keep, s->W, bytes, cudaMemcpyDeviceToDevice, s->st);
-  fused_stage(s, s->W, s->U, s->U, 1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0, 0.5, dt);
+  if (need_trace) run(s, K_TRACE, [&] { s->ops->trace(s->ctx, u); });
+  fused_stage(s, u, nullptr, u1, 0.0, 1.0, 1.0, 0.0, dt);
+  fused_stage(s, u1, u, u2, 0.75, 0.25, 0.25, 1.0, dt);
+  fused_stage(s, u2, u, next, 1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0, 0.5, dt);
   run(s, K_CFL, [&] { dg::launch_advance_t(s->st, s->ds); });
 }
 
@@ -1761,10 +1769,23 @@ extern "C" dg_status dg_adjoint_create(dg_solver *s, int nrec, const double *rx,
       phi[(size_t)r * s->np + i] = (double)v;
     }
   }
+  // receivers of one element, chained in their order
+  std::vector<int> next((size_t)2 * nrec, 0), last(s->K, -1);
+  for (int r = 0; r < nrec; r++) {
+    next[r] = -1;
+    int &l = last[el[r]];
+    if (l >= 0) {
+      next[l] = r;
+      next[nrec + r] = 1;
+    }
+    l = r;
+  }
   if ((st = amalloc(a, &a->rec_el, (size_t)nrec)) != DG_OK) return st;
+  if ((st = amalloc(a, &a->rec_next, next.size())) != DG_OK) return st;
   if ((st = amalloc(a, &a->rec_phi, (size_t)nrec * s->np)) != DG_OK) return st;
   if (nrec) {
     CK(cudaMemcpy(a->rec_el, el.data(), sizeof(int) * nrec, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(a->rec_next, next.data(), sizeof(int) * next.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(a->rec_phi, phi.data(), sizeof(double) * phi.size(), cudaMemcpyHostToDevice));
   }
   *out = a;
@@ -1875,18 +1896,17 @@ extern "C" dg_status dg_adjoint_forward(dg_adjoint *a, int nsteps, double dt, in
   }
   if ((st = set_fixed_dt(s, t0, dt)) != DG_OK) return st;
   const size_t bytes = s->ndof_p * sizeof(double);
+  const size_t nd = s->ndof_p;
+  if (a->stored) CK(cudaMemcpyAsync(a->store, s->U, bytes, cudaMemcpyDeviceToDevice, s->st));
   for (int n = 0; n < nsteps; n++) {
+    double *u = a->stored ? a->store + (size_t)3 * n * nd : s->U;
+    double *next = a->stored && n + 1 < nsteps ? u + 3 * nd : s->U;
     if (n % ckpt == 0)
-      CK(cudaMemcpyAsync(a->cks[n / ckpt], s->U, bytes, cudaMemcpyDeviceToDevice, s->st));
-    if (a->stored) {
-      double *u = a->store + (size_t)3 * n * s->ndof_p;
-      CK(cudaMemcpyAsync(u, s->U, bytes, cudaMemcpyDeviceToDevice, s->st));
-      plain_step(s, u + s->ndof_p, u + 2 * s->ndof_p, n == 0);
-    } else {
-      plain_step(s, nullptr, nullptr, n == 0);
-    }
+      CK(cudaMemcpyAsync(a->cks[n / ckpt], u, bytes, cudaMemcpyDeviceToDevice, s->st));
+    if (a->stored) plain_step(s, u, u + nd, u + 2 * nd, next, n == 0);
+    else plain_step(s, u, s->W, s->W, next, n == 0);
     if ((n + 1) % every == 0)
-      dg::launch_sample(s->st, s->U, a->rec_el, a->rec_phi, a->nrec, s->np, s->m.Kp,
+      dg::launch_sample(s->st, next, a->rec_el, a->rec_phi, a->nrec, s->np, s->m.Kp,
                         a->samples + (size_t)((n + 1) / every - 1) * a->nrec);
   }
   CK(cudaMemcpyAsync(a->ufinal, s->U, bytes, cudaMemcpyDeviceToDevice, s->st));
@@ -1915,7 +1935,6 @@ extern "C" dg_status dg_adjoint_backward(dg_adjoint *a, const double *sbar, doub
     if ((st = amalloc(a, &a->ub, s->ndof_p)) != DG_OK) return st;
     if ((st = amalloc(a, &a->ub1, s->ndof_p)) != DG_OK) return st;
     if ((st = amalloc(a, &a->ub2, s->ndof_p)) != DG_OK) return st;
-    if ((st = amalloc(a, &a->acc, s->ndof_p)) != DG_OK) return st;
     if ((st = amalloc(a, &a->bbar, (size_t)s->np * s->m.Kp)) != DG_OK) return st;
   }
   const int nsamp = a->nsteps / a->every;
@@ -1924,41 +1943,65 @@ extern "C" dg_status dg_adjoint_backward(dg_adjoint *a, const double *sbar, doub
                        s->st));
   CK(cudaMemsetAsync(a->ub, 0, bytes, s->st));
   CK(cudaMemsetAsync(a->bbar, 0, (size_t)s->np * s->m.Kp * sizeof(double), s->st));
-  const int n = (int)s->ndof_p;
   const double dt = a->dt;
   const int nck = (int)a->cks.size();
+  bool traced = false;  // lb.Tv holds the traces of a->ub for the step's first stage
   for (int k = nck - 1; k >= 0; k--) {
     const int n0 = k * a->ckpt, n1 = std::min(n0 + a->ckpt, a->nsteps);
     if (!a->stored) {
       // recompute the segment, keeping u^n, u1, u2 of every step
-      CK(cudaMemcpyAsync(s->U, a->cks[k], bytes, cudaMemcpyDeviceToDevice, s->st));
+      CK(cudaMemcpyAsync(a->seg[0], a->cks[k], bytes, cudaMemcpyDeviceToDevice, s->st));
       if ((st = set_fixed_dt(s, a->t0 + n0 * dt, dt)) != DG_OK) return st;
       for (int m = n0; m < n1; m++) {
-        const int j = m - n0;
-        CK(cudaMemcpyAsync(a->seg[3 * j], s->U, bytes, cudaMemcpyDeviceToDevice, s->st));
-        plain_step(s, a->seg[3 * j + 1], a->seg[3 * j + 2], m == n0);
+        const int j = 3 * (m - n0);
+        plain_step(s, a->seg[j], a->seg[j + 1], a->seg[j + 2], m + 1 < n1 ? a->seg[j + 3] : s->U,
+                   m == n0);
       }
     }
     for (int m = n1 - 1; m >= n0; m--) {
       const int j = m - n0;
       if ((m + 1) % a->every == 0)  // adjoint of the sample taken from u^{m+1}
-        dg::launch_sample_adj(s->st, a->ub, a->rec_el, a->rec_phi, a->nrec, s->np, s->m.Kp,
-                              a->sbar + (size_t)((m + 1) / a->every - 1) * a->nrec);
+        dg::launch_sample_adj(s->st, a->ub, a->rec_el, a->rec_next, a->rec_phi, a->nrec,
+                              s->np, s->m.Kp, a->sbar + (size_t)((m + 1) / a->every - 1) * a->nrec);
       double *un = a->seg[3 * j], *u1 = a->seg[3 * j + 1], *u2 = a->seg[3 * j + 2];
       if (a->stored) {
         un = a->store + (size_t)3 * m * s->ndof_p;
         u1 = un + s->ndof_p;
         u2 = un + 2 * s->ndof_p;
       }
+      dg::AdjStage g;
+      g.bbar = a->bbar;
       // u^{n+1} = 1/3 u^n + 2/3 u2 + 2/3 dt L(u2)
-      adj_stage(s, u2, a->ub, a->ub2, a->bbar, 2.0 / 3.0, 2.0 / 3.0 * dt, lb);
-      dg::launch_axpby(s->st, n, 1.0 / 3.0, a->ub, 0.0, a->acc);
+      g.us = u2;
+      g.obar = a->ub;
+      g.ubar = a->ub2;
+      g.cb = 2.0 / 3.0;
+      g.ccdt = 2.0 / 3.0 * dt;
+      g.next_ccdt = 0.25 * dt;
+      adj_stage(s, g, traced, lb);
       // u2 = 3/4 u^n + 1/4 u1 + 1/4 dt L(u1)
-      adj_stage(s, u1, a->ub2, a->ub1, a->bbar, 0.25, 0.25 * dt, lb);
-      dg::launch_axpby(s->st, n, 0.75, a->ub2, 1.0, a->acc);
-      // u1 = u^n + dt L(u^n)
-      adj_stage(s, un, a->ub1, a->ub, a->bbar, 1.0, dt, lb);
-      dg::launch_axpby(s->st, n, 1.0, a->acc, 1.0, a->ub);
+      g.us = u1;
+      g.obar = a->ub2;
+      g.ubar = a->ub1;
+      g.cb = 0.25;
+      g.ccdt = 0.25 * dt;
+      g.next_ccdt = dt;
+      adj_stage(s, g, true, lb);
+      // u1 = u^n + dt L(u^n); and the adjoint of u^n's own terms above
+      g.us = un;
+      g.obar = a->ub1;
+      g.ubar = a->ub;
+      g.cb = 1.0;
+      g.ccdt = dt;
+      g.x0 = a->ub;
+      g.a0 = 1.0 / 3.0;
+      g.x1 = a->ub2;
+      g.a1 = 0.75;
+      // the step before starts from this ubar, unless a sample is added to it
+      // (step m's samples are of u^{m+1}) or its segment is recomputed first
+      traced = m > n0 && m % a->every != 0;
+      g.next_ccdt = traced ? 2.0 / 3.0 * dt : 0.0;
+      adj_stage(s, g, true, lb);
     }
   }
   const int rows = s->N * s->np;
