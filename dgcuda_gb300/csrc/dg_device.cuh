@@ -108,6 +108,21 @@ DG_HD double mul_rn(double a, double b) {
 #endif
 }
 
+// the larger of two wave speeds: a comparison and a select, where fmax is an
+// FP64 operation
+DG_HD double larger(double a, double b) { return b > a ? b : a; }
+// -x / 2 for x >= 0, exact, on the integer pipe (x below 2^-1021 may lose its
+// last bits; an infinite or NaN x becomes a large finite number, and comes
+// from a momentum that is in every flux by itself)
+DG_HD double neg_half(double x) {
+#ifdef __CUDA_ARCH__
+  const int hi = max(__double2hiint(x) - 0x00100000, 0) ^ (int)0x80000000;
+  return __hiloint2double(hi, __double2loint(x));
+#else
+  return -0.5 * x;
+#endif
+}
+
 // 1/x for the flux evaluations, from the approximate reciprocal r of the PTX
 // instruction rcp.approx.ftz.f64 (about 20 correct bits) by one third-order
 // step of the Newton-Raphson family: with e = 1 - x r, 1/x = r / (1 - e) =
@@ -371,20 +386,20 @@ struct Advection {  // advection/advection.cu
     fx[0] = vx * U[0];
     fy[0] = vy * U[0];
   }
-  // upwind flux with the velocity at the point (advection.cu:94-116)
+  // upwind flux with the velocity at the point (advection.cu:94-116), times sc
   DG_HD static void riemann_at(double vx, double vy, const double *UL, const double *UR,
-                               double nx, double ny, double *F) {
-    double an = fma(nx, vx, ny * vy);
+                               double nx, double ny, double sc, double *F) {
+    const double an = sc * fma(nx, vx, ny * vy);
     F[0] = an > 0 ? an * UL[0] : an * UR[0];
   }
+  // The numerical flux times sc > 0 (half an edge's length times a point's
+  // weight) is riemann(.., kScale sc, ..): every equation takes the factor into
+  // the normal and the wave speed, two products instead of one per variable
+  static constexpr double kScale = 1.0;
   // upwind flux (riemann_solver_upwind, advection.cu:94-116)
-  // riemann_raw(..) * kRawScale is the numerical flux; face kernels fold the
-  // (exact, power-of-two) scale into their own edge-length factor
-  static constexpr double kRawScale = 1.0;
-  DG_HD static void riemann_raw(const EqP &q, const double *UL, const double *UR, double nx,
-                                double ny, double *F) {
-    double an = fma(nx, q.ax, ny * q.ay);
-    F[0] = an > 0 ? an * UL[0] : an * UR[0];
+  DG_HD static void riemann(const EqP &q, const double *UL, const double *UR, double nx,
+                            double ny, double sc, double *F) {
+    riemann_at(q.ax, q.ay, UL, UR, nx, ny, sc, F);
   }
   DG_HD static double mean_speed(const EqP &q, const double *) {
     // a field: the largest speed over the elements, each taken at its middle
@@ -461,24 +476,27 @@ struct Euler {  // euler/euler.cu
     h[3] = H * ub;
   }
   // local Lax-Friedrichs (euler.cu:170-237)
-  static constexpr double kRawScale = 0.5;  // LLF: F = 0.5 [ ... ]
-  DG_HD static void riemann_raw(const EqP &q, const double *UL, const double *UR, double nx,
-                                double ny, double *F) {
+  static constexpr double kScale = 0.5;  // LLF: F = 0.5 [ ... ]
+  DG_HD static void riemann(const EqP &q, const double *UL, const double *UR, double nx,
+                            double ny, double sc, double *F) {
     // every multiply-add is an explicit fma so the rounding does not depend
     // on how the compiler contracts the expression in a given kernel; the
-    // normal momenta m . n are the mass fluxes themselves
+    // normal momenta m . n are the mass fluxes themselves.  62 FP64
+    // operations, what k_face is bound by (67 with the scale applied to the
+    // fluxes, products by -1/2 and fmax)
+    const double sx = sc * nx, sy = sc * ny;
     const double irl = rcp(UL[0]), irr = rcp(UR[0]);
-    const double mnl = fma(UL[1], nx, UL[2] * ny), mnr = fma(UR[1], nx, UR[2] * ny);
+    const double mnl = fma(UL[1], sx, UL[2] * sy), mnr = fma(UR[1], sx, UR[2] * sy);
     const double snl = mnl * irl, snr = mnr * irr;
     const double m2l = fma(UL[1], UL[1], UL[2] * UL[2]), m2r = fma(UR[1], UR[1], UR[2] * UR[2]);
-    const double pl = mul_rn(q.gamma - 1., fma(-0.5 * m2l, irl, UL[3]));
-    const double pr = mul_rn(q.gamma - 1., fma(-0.5 * m2r, irr, UR[3]));
+    const double pl = mul_rn(q.gamma - 1., fma(neg_half(m2l), irl, UL[3]));
+    const double pr = mul_rn(q.gamma - 1., fma(neg_half(m2r), irr, UR[3]));
     const double cl = sqrt_pos(q.gamma * pl * irl), cr = sqrt_pos(q.gamma * pr * irr);
-    const double lam = fmax(fabs(snl) + cl, fabs(snr) + cr);
+    const double lam = larger(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
     const double P = pl + pr;
     F[0] = fma(lam, UL[0] - UR[0], mnl + mnr);
-    F[1] = fma(lam, UL[1] - UR[1], fma(UL[1], snl, fma(UR[1], snr, P * nx)));
-    F[2] = fma(lam, UL[2] - UR[2], fma(UL[2], snl, fma(UR[2], snr, P * ny)));
+    F[1] = fma(lam, UL[1] - UR[1], fma(UL[1], snl, fma(UR[1], snr, P * sx)));
+    F[2] = fma(lam, UL[2] - UR[2], fma(UL[2], snl, fma(UR[2], snr, P * sy)));
     F[3] = fma(lam, UL[3] - UR[3], fma(UL[3] + pl, snl, (UR[3] + pr) * snr));
   }
   DG_HD static double mean_speed(const EqP &q, const double *U) {  // euler.cu:248-277
@@ -536,19 +554,20 @@ struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
     fy[1] = U[1] * v;
     fy[2] = fma(U[2], v, hp);
   }
-  static constexpr double kRawScale = 0.5;  // LLF: F = 0.5 [ ... ]
-  DG_HD static void riemann_raw(const EqP &q, const double *UL, const double *UR, double nx,
-                                double ny, double *F) {  // shallowwater.cu:118-185
+  static constexpr double kScale = 0.5;  // LLF: F = 0.5 [ ... ]
+  DG_HD static void riemann(const EqP &q, const double *UL, const double *UR, double nx,
+                            double ny, double sc, double *F) {  // shallowwater.cu:118-185
     // the normal momenta m . n are the mass fluxes themselves
+    const double sx = sc * nx, sy = sc * ny;
     const double ihl = rcp(UL[0]), ihr = rcp(UR[0]);
-    const double mnl = fma(nx, UL[1], ny * UL[2]), mnr = fma(nx, UR[1], ny * UR[2]);
+    const double mnl = fma(sx, UL[1], sy * UL[2]), mnr = fma(sx, UR[1], sy * UR[2]);
     const double snl = mnl * ihl, snr = mnr * ihr;
     const double cl = sqrt_pos(UL[0] * q.g), cr = sqrt_pos(UR[0] * q.g);
-    const double lam = fmax(fabs(snl) + cl, fabs(snr) + cr);
+    const double lam = larger(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
     const double P = 0.5 * q.g * fma(UL[0], UL[0], UR[0] * UR[0]);
     F[0] = fma(lam, UL[0] - UR[0], mnl + mnr);
-    F[1] = fma(lam, UL[1] - UR[1], fma(UL[1], snl, fma(UR[1], snr, P * nx)));
-    F[2] = fma(lam, UL[2] - UR[2], fma(UL[2], snl, fma(UR[2], snr, P * ny)));
+    F[1] = fma(lam, UL[1] - UR[1], fma(UL[1], snl, fma(UR[1], snr, P * sx)));
+    F[2] = fma(lam, UL[2] - UR[2], fma(UL[2], snl, fma(UR[2], snr, P * sy)));
   }
   DG_HD static double mean_speed(const EqP &q, const double *U) {  // shallowwater.cu:196-224
     // as Euler's: rcp and sqrt_pos within 1 ulp of IEEE division and sqrt
@@ -575,24 +594,23 @@ struct Maxwell {  // maxwells/maxwells.cu, U = (Hx, Hy, Ez)
   static constexpr bool kFolded = false;
   DG_HD static bool physical(const EqP &, const double *) { return true; }
   DG_HD static void flux(const EqP &q, const double *U, double *fx, double *fy) {
-    double imu = 1. / q.mu, ieps = 1. / q.eps;
     fx[0] = 0.;
-    fx[1] = imu * U[2];
-    fx[2] = ieps * U[1];
-    fy[0] = -imu * U[2];
+    fx[1] = q.imu * U[2];
+    fx[2] = q.ieps * U[1];
+    fy[0] = -q.imu * U[2];
     fy[1] = 0.;
-    fy[2] = -ieps * U[0];
+    fy[2] = -q.ieps * U[0];
   }
-  static constexpr double kRawScale = 0.5;  // LLF: F = 0.5 [ ... ]
-  DG_HD static void riemann_raw(const EqP &q, const double *UL, const double *UR, double nx,
-                                double ny, double *F) {  // maxwells.cu:93-163, LLF with lambda = 1/sqrt(eps mu)
-    double imu = 1. / q.mu, ieps = 1. / q.eps, lam = fabs(1. / sqrt(q.eps * q.mu));
-    double ez = UL[2] + UR[2], hx = UL[0] + UR[0], hy = UL[1] + UR[1];
-    F[0] = fma(lam, UL[0] - UR[0], -imu * ez * ny);
-    F[1] = fma(lam, UL[1] - UR[1], imu * ez * nx);
-    F[2] = fma(lam, UL[2] - UR[2], ieps * fma(hy, nx, -hx * ny));
+  static constexpr double kScale = 0.5;  // LLF: F = 0.5 [ ... ]
+  DG_HD static void riemann(const EqP &q, const double *UL, const double *UR, double nx,
+                            double ny, double sc, double *F) {  // maxwells.cu:93-163, LLF with lambda = 1/sqrt(eps mu)
+    const double sx = sc * nx, sy = sc * ny, lam = sc * q.speed;
+    const double ez = q.imu * (UL[2] + UR[2]), hx = UL[0] + UR[0], hy = UL[1] + UR[1];
+    F[0] = fma(lam, UL[0] - UR[0], -ez * sy);
+    F[1] = fma(lam, UL[1] - UR[1], ez * sx);
+    F[2] = fma(lam, UL[2] - UR[2], q.ieps * fma(hy, sx, -hx * sy));
   }
-  DG_HD static double mean_speed(const EqP &q, const double *) { return fabs(1. / sqrt(q.eps * q.mu)); }
+  DG_HD static double mean_speed(const EqP &q, const double *) { return q.speed; }
   DG_HD static void reflect(const EqP &, const double *UL, double *UR, double, double, double nx,
                             double ny) {  // maxwells/cmirror/cmirror.cu:63-77
     // E_z kept; H: the normal component kept, the tangential one reversed

@@ -127,7 +127,10 @@ struct FaceArgs {
 };
 
 // N contiguous doubles at p (16-byte aligned when N is even): 128-bit loads
-// and stores where N is even, scalar ones otherwise
+// and stores where N is even, scalar ones otherwise.  The loads are read-only
+// (__ldg), so that a loop's later ones need not wait for its earlier stores:
+// k_face's points are then all in flight (advection with a field, p = 3, 131k
+// triangles 38 -> 31 us, Maxwell p = 1 32 -> 23 us)
 template <int N>
 __device__ __forceinline__ void load_vars(const double *p, double (&v)[N]) {
   if constexpr (N % 2 == 0) {
@@ -139,7 +142,7 @@ __device__ __forceinline__ void load_vars(const double *p, double (&v)[N]) {
     }
   } else {
 #pragma unroll
-    for (int n = 0; n < N; n++) v[n] = p[n];
+    for (int n = 0; n < N; n++) v[n] = __ldg(p + n);
   }
 }
 template <int N>
@@ -154,78 +157,82 @@ __device__ __forceinline__ void store_vars(double *p, const double (&v)[N]) {
   }
 }
 
+// the scaled flux at edge point j of boundary side s
+template <class Eq, int P>
+__device__ __forceinline__ void boundary_flux(const Tab<P> &tab, const EqP &q, const FaceArgs &a,
+                                              int s, const int4 &sd, int j, double (&Fn)[Eq::N]) {
+  constexpr int N = Eq::N, N1 = P + 1;
+  const int S = a.S, Sb = a.Sb;
+  const double nx = a.sgeo[s], ny = a.sgeo[S + s], hl = a.sgeo[2 * (size_t)S + s];
+  const double t = *a.tptr + a.tcoef * *a.dtp;
+  const double *bxy = a.bxy;
+  const double xa = bxy[s], ya = bxy[Sb + s], xb = bxy[2 * Sb + s], yb = bxy[3 * Sb + s];
+  const double sc = hl * tab.w1[j] * Eq::kScale;  // exact: a power of two
+  double UL[N], UR[N];
+  load_vars<N>(a.T + ((size_t)sd.x * 3 + sd.z) * (N1 * N) + j * N, UL);
+  const double r = 0.5 + 0.5 * tab.t1[j];
+  const double px = fma(r, xb - xa, xa), py = fma(r, yb - ya, ya);
+  ghost_state<Eq>(q, sd.y, UL, UR, px, py, t, nx, ny);
+  if constexpr (Eq::kField) {
+    if (q.field) {
+      double vx, vy;
+      Eq::velocity(q, px, py, vx, vy);
+      Eq::riemann_at(vx, vy, UL, UR, nx, ny, sc, Fn);
+      return;
+    }
+  }
+  Eq::riemann(q, UL, UR, nx, ny, sc, Fn);
+}
+
 // FS: also store the per-side sums of the scaled fluxes in a.Fs
 template <class Eq, int P, bool FS = false>
 __device__ __forceinline__ void face_body(const Tab<P> &tab, const EqP &q, const FaceArgs &a,
                                           int s) {
   constexpr int N = Eq::N, N1 = P + 1;
-  const int S = a.S, Sb = a.Sb;
+  const int S = a.S;
   const int4 sd = a.side[s];
-  const double nx = a.sgeo[s], ny = a.sgeo[S + s], hl = a.sgeo[2 * (size_t)S + s];
-  const double *TL = a.T + ((size_t)sd.x * 3 + sd.z) * (N1 * N);
   double *F = a.Fh + (size_t)s * (N1 * N);
   double fs[N];
 #pragma unroll
   for (int n = 0; n < N; n++) fs[n] = 0.0;
   if (sd.y >= 0) {
+    const double nx = a.sgeo[s], ny = a.sgeo[S + s], hl = a.sgeo[2 * (size_t)S + s];
+    const double *TL = a.T + ((size_t)sd.x * 3 + sd.z) * (N1 * N);
     const double *TR = a.T + ((size_t)sd.y * 3 + sd.w) * (N1 * N);
 #pragma unroll
     for (int j = 0; j < N1; j++) {
+      const double sc = hl * tab.w1[j] * Eq::kScale;  // exact: a power of two
       double UL[N], UR[N], Fn[N];
       load_vars<N>(TL + j * N, UL);
       load_vars<N>(TR + (N1 - 1 - j) * N, UR);
+      bool done = false;
       if constexpr (Eq::kField) {
         if (q.field) {  // the velocity at the edge point, on the left face
           const int va = sd.z, vb = sd.z == 2 ? 0 : sd.z + 1;
           const size_t Kp = a.Kp;
-          const double xa = a.vtx[2 * va * Kp + sd.x], ya = a.vtx[(2 * va + 1) * Kp + sd.x];
-          const double xb = a.vtx[2 * vb * Kp + sd.x], yb = a.vtx[(2 * vb + 1) * Kp + sd.x];
+          const double xa = __ldg(a.vtx + 2 * va * Kp + sd.x);
+          const double ya = __ldg(a.vtx + (2 * va + 1) * Kp + sd.x);
+          const double xb = __ldg(a.vtx + 2 * vb * Kp + sd.x);
+          const double yb = __ldg(a.vtx + (2 * vb + 1) * Kp + sd.x);
           const double r = 0.5 + 0.5 * tab.t1[j];
           double vx, vy;
           Eq::velocity(q, fma(r, xb - xa, xa), fma(r, yb - ya, ya), vx, vy);
-          Eq::riemann_at(vx, vy, UL, UR, nx, ny, Fn);
-        } else {
-          Eq::riemann_raw(q, UL, UR, nx, ny, Fn);
+          Eq::riemann_at(vx, vy, UL, UR, nx, ny, sc, Fn);
+          done = true;
         }
-      } else {
-        Eq::riemann_raw(q, UL, UR, nx, ny, Fn);
       }
-      const double sc = hl * tab.w1[j] * Eq::kRawScale;  // exact: a power of two
+      if (!done) Eq::riemann(q, UL, UR, nx, ny, sc, Fn);
 #pragma unroll
-      for (int n = 0; n < N; n++) {
-        Fn[n] *= sc;
-        if (FS) fs[n] = j == 0 ? Fn[n] : fs[n] + Fn[n];
-      }
+      for (int n = 0; FS && n < N; n++) fs[n] = j == 0 ? Fn[n] : fs[n] + Fn[n];
       store_vars<N>(F + j * N, Fn);
     }
   } else {
-    const double t = *a.tptr + a.tcoef * *a.dtp;
-    const double *bxy = a.bxy;
-    const double xa = bxy[s], ya = bxy[Sb + s], xb = bxy[2 * Sb + s], yb = bxy[3 * Sb + s];
 #pragma unroll
     for (int j = 0; j < N1; j++) {
-      double UL[N], UR[N], Fn[N];
-      load_vars<N>(TL + j * N, UL);
-      const double r = 0.5 + 0.5 * tab.t1[j];
-      const double px = fma(r, xb - xa, xa), py = fma(r, yb - ya, ya);
-      ghost_state<Eq>(q, sd.y, UL, UR, px, py, t, nx, ny);
-      if constexpr (Eq::kField) {
-        if (q.field) {
-          double vx, vy;
-          Eq::velocity(q, px, py, vx, vy);
-          Eq::riemann_at(vx, vy, UL, UR, nx, ny, Fn);
-        } else {
-          Eq::riemann_raw(q, UL, UR, nx, ny, Fn);
-        }
-      } else {
-        Eq::riemann_raw(q, UL, UR, nx, ny, Fn);
-      }
-      const double sc = hl * tab.w1[j] * Eq::kRawScale;  // exact: a power of two
+      double Fn[N];
+      boundary_flux<Eq, P>(tab, q, a, s, sd, j, Fn);
 #pragma unroll
-      for (int n = 0; n < N; n++) {
-        Fn[n] *= sc;
-        if (FS) fs[n] = j == 0 ? Fn[n] : fs[n] + Fn[n];
-      }
+      for (int n = 0; FS && n < N; n++) fs[n] = j == 0 ? Fn[n] : fs[n] + Fn[n];
       store_vars<N>(F + j * N, Fn);
     }
   }
@@ -233,12 +240,33 @@ __device__ __forceinline__ void face_body(const Tab<P> &tab, const EqP &q, const
   if (FS) store_vars<N>(a.Fs + (size_t)s * N, fs);
 }
 
+// threads of k_face: a side each, but without FS a boundary side has one per
+// edge point -- a ghost state may take a few hundred dependent FP64 operations
+// (sines and an exponential of an inflow), and the points of one thread, one
+// after the other, were the length of the whole launch on small meshes
+// (advection with a rotating inflow, 34k triangles, p = 3: 27 -> 14 us)
+template <int P, bool FS>
+__host__ __device__ __forceinline__ int face_threads(int S, int Sb) {
+  return FS ? S : S + Sb * P;
+}
+
 template <class Eq, int P, bool FS = false>
 __global__ void __launch_bounds__(kMaxBlock) k_face(const __grid_constant__ Tab<P> tab,
                                                     const __grid_constant__ EqP q,
                                                     const __grid_constant__ FaceArgs a) {
+  constexpr int N = Eq::N, N1 = P + 1;
   pdl_begin();
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (!FS && i < a.Sb * N1) {
+    const int s = i / N1, j = i % N1;
+    const int4 sd = a.side[s];
+    double Fn[N];
+    boundary_flux<Eq, P>(tab, q, a, s, sd, j, Fn);
+    pdl_end();
+    store_vars<N>(a.Fh + ((size_t)s * N1 + j) * N, Fn);
+    return;
+  }
+  const int s = FS ? i : i - a.Sb * P;
   if (s < a.S) face_body<Eq, P, FS>(tab, q, a, s);
 }
 
@@ -756,9 +784,6 @@ __device__ __forceinline__ double cell_speed(const Tab<P> &tab, const EqP &q,
   atomicExch(&ds->status, 4);
   return 0.0;
 }
-// the larger of two speeds (no NaN; a comparison and a select where fmax costs
-// an FP64 operation)
-__device__ __forceinline__ double larger(double a, double b) { return b > a ? b : a; }
 // lam: this thread's maximum; nblocks: the blocks that meet in ds
 __device__ __forceinline__ void cfl_reduce(double lam, DevScalars *ds, unsigned nblocks, int p,
                                            int mode) {
@@ -1178,8 +1203,8 @@ struct Launch {
     a.S = c.m.S;
     a.Sb = c.m.Sb;
     a.Kp = c.m.Kp;
-    DG_DISPATCH_P((launch(k_face<Eq, P, FS>, nblk(c.m.S, c.blk), c.blk, c.st, tab<P>(c), *c.q,
-                          a)));
+    DG_DISPATCH_P((launch(k_face<Eq, P, FS>, nblk(face_threads<P, FS>(c.m.S, c.m.Sb), c.blk), c.blk,
+                          c.st, tab<P>(c), *c.q, a)));
   }
   static void face(const Ctx &c, const double *t, double tcoef) {
     face_args<false>(c, t, tcoef, nullptr);

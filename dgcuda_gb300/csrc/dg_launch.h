@@ -12,6 +12,7 @@ namespace dg {
 constexpr int kMaxSeries = 16;  // terms of an inflow pressure series
 struct EqP {
   double gamma, g, ax, ay, mu, eps;
+  double imu, ieps, speed;  // Maxwell: 1/mu, 1/eps, 1/sqrt(eps mu)
   int problem;
   int field;        // 1: advection velocity a(x, y) = (ax, ay) + agrad (x, y)
   double prm[8];

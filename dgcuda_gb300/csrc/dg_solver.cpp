@@ -504,6 +504,9 @@ extern "C" dg_status dg_solver_create(const dg_mesh *mesh, dg_equation eq, int p
   s->q.ay = P.ay;
   s->q.mu = P.mu;
   s->q.eps = P.eps;
+  s->q.imu = 1. / P.mu;
+  s->q.ieps = 1. / P.eps;
+  s->q.speed = std::fabs(1. / std::sqrt(P.eps * P.mu));
   s->q.problem = P.problem;
   for (int i = 0; i < 8; i++) s->q.prm[i] = P.prm[i];
   if (P.problem == DG_PB_ADV_ROTATINGHILL || P.problem == DG_PB_ADV_SPIN) {
