@@ -157,22 +157,42 @@ __device__ __forceinline__ void store_vars(double *p, const double (&v)[N]) {
   }
 }
 
-// the scaled flux at edge point j of boundary side s
+// the scaled flux at edge point j of side s
 template <class Eq, int P>
-__device__ __forceinline__ void boundary_flux(const Tab<P> &tab, const EqP &q, const FaceArgs &a,
-                                              int s, const int4 &sd, int j, double (&Fn)[Eq::N]) {
+__device__ __forceinline__ void face_point(const Tab<P> &tab, const EqP &q, const FaceArgs &a,
+                                           int s, int j, double (&Fn)[Eq::N]) {
   constexpr int N = Eq::N, N1 = P + 1;
   const int S = a.S, Sb = a.Sb;
+  const int4 sd = a.side[s];
   const double nx = a.sgeo[s], ny = a.sgeo[S + s], hl = a.sgeo[2 * (size_t)S + s];
-  const double t = *a.tptr + a.tcoef * *a.dtp;
-  const double *bxy = a.bxy;
-  const double xa = bxy[s], ya = bxy[Sb + s], xb = bxy[2 * Sb + s], yb = bxy[3 * Sb + s];
   const double sc = hl * tab.w1[j] * Eq::kScale;  // exact: a power of two
   double UL[N], UR[N];
-  load_vars<N>(a.T + ((size_t)sd.x * 3 + sd.z) * (N1 * N) + j * N, UL);
-  const double r = 0.5 + 0.5 * tab.t1[j];
-  const double px = fma(r, xb - xa, xa), py = fma(r, yb - ya, ya);
-  ghost_state<Eq>(q, sd.y, UL, UR, px, py, t, nx, ny);
+  load_vars<N>(a.T + (((size_t)sd.x * 3 + sd.z) * N1 + j) * N, UL);
+  double px = 0.0, py = 0.0;  // the point, where something depends on it
+  if (sd.y >= 0) {
+    load_vars<N>(a.T + (((size_t)sd.y * 3 + sd.w) * N1 + (N1 - 1 - j)) * N, UR);
+    if constexpr (Eq::kField) {
+      if (q.field) {  // on the left face
+        const int va = sd.z, vb = sd.z == 2 ? 0 : sd.z + 1;
+        const size_t Kp = a.Kp;
+        const double xa = __ldg(a.vtx + 2 * va * Kp + sd.x);
+        const double ya = __ldg(a.vtx + (2 * va + 1) * Kp + sd.x);
+        const double xb = __ldg(a.vtx + 2 * vb * Kp + sd.x);
+        const double yb = __ldg(a.vtx + (2 * vb + 1) * Kp + sd.x);
+        const double r = 0.5 + 0.5 * tab.t1[j];
+        px = fma(r, xb - xa, xa);
+        py = fma(r, yb - ya, ya);
+      }
+    }
+  } else {
+    const double t = *a.tptr + a.tcoef * *a.dtp;
+    const double xa = a.bxy[s], ya = a.bxy[Sb + s], xb = a.bxy[2 * Sb + s],
+                 yb = a.bxy[3 * Sb + s];
+    const double r = 0.5 + 0.5 * tab.t1[j];
+    px = fma(r, xb - xa, xa);
+    py = fma(r, yb - ya, ya);
+    ghost_state<Eq>(q, sd.y, UL, UR, px, py, t, nx, ny);
+  }
   if constexpr (Eq::kField) {
     if (q.field) {
       double vx, vy;
@@ -184,90 +204,53 @@ __device__ __forceinline__ void boundary_flux(const Tab<P> &tab, const EqP &q, c
   Eq::riemann(q, UL, UR, nx, ny, sc, Fn);
 }
 
-// FS: also store the per-side sums of the scaled fluxes in a.Fs
-template <class Eq, int P, bool FS = false>
+// The face kernel: a thread per edge point, a block of 32 sides.  The points
+// of a side are neighbours, so a warp's trace reads are whole lines of the
+// sides' chunks and its flux stores one contiguous run; a thread holds one
+// point's states (fewer registers, more warps on the FP64 pipe, which is what
+// bounds the kernel), and a ghost state of a few hundred dependent operations
+// (the sines and the exponential of an inflow) is not repeated in one thread.
+// With a thread per side, us: shallow water p = 2, 131k triangles 62.8 -> 58.7,
+// Maxwell p = 3 41.3 -> 37.4, Euler p = 3 33k 33.2 -> 30.8 (2.1M: 1469 -> 1482).
+constexpr int kFaceSides = 32;
+
+// thread i of a block on the sides s0 .. s_end - 1, SIDES at most.  FS: also the
+// sums of each side's scaled fluxes over its points, in their order, in a.Fs
+// (sm: SIDES N1 N doubles)
+template <class Eq, int P, bool FS, int SIDES>
 __device__ __forceinline__ void face_body(const Tab<P> &tab, const EqP &q, const FaceArgs &a,
-                                          int s) {
+                                          int s0, int s_end, int i, double *sm) {
   constexpr int N = Eq::N, N1 = P + 1;
-  const int S = a.S;
-  const int4 sd = a.side[s];
-  double *F = a.Fh + (size_t)s * (N1 * N);
-  double fs[N];
+  const int s = s0 + i / N1, j = i % N1;
+  if (i < SIDES * N1 && s < s_end) {
+    double Fn[N];
+    face_point<Eq, P>(tab, q, a, s, j, Fn);
+    store_vars<N>(a.Fh + ((size_t)s * N1 + j) * N, Fn);
+    if (FS)
 #pragma unroll
-  for (int n = 0; n < N; n++) fs[n] = 0.0;
-  if (sd.y >= 0) {
-    const double nx = a.sgeo[s], ny = a.sgeo[S + s], hl = a.sgeo[2 * (size_t)S + s];
-    const double *TL = a.T + ((size_t)sd.x * 3 + sd.z) * (N1 * N);
-    const double *TR = a.T + ((size_t)sd.y * 3 + sd.w) * (N1 * N);
+      for (int n = 0; n < N; n++) sm[i * N + n] = Fn[n];
+  }
+  if constexpr (FS) {
+    __syncthreads();
+    for (int k = i; k < SIDES * N; k += blockDim.x) {
+      const int r = k / N, n = k % N;
+      if (s0 + r >= s_end) break;
+      double v = sm[r * N1 * N + n];
 #pragma unroll
-    for (int j = 0; j < N1; j++) {
-      const double sc = hl * tab.w1[j] * Eq::kScale;  // exact: a power of two
-      double UL[N], UR[N], Fn[N];
-      load_vars<N>(TL + j * N, UL);
-      load_vars<N>(TR + (N1 - 1 - j) * N, UR);
-      bool done = false;
-      if constexpr (Eq::kField) {
-        if (q.field) {  // the velocity at the edge point, on the left face
-          const int va = sd.z, vb = sd.z == 2 ? 0 : sd.z + 1;
-          const size_t Kp = a.Kp;
-          const double xa = __ldg(a.vtx + 2 * va * Kp + sd.x);
-          const double ya = __ldg(a.vtx + (2 * va + 1) * Kp + sd.x);
-          const double xb = __ldg(a.vtx + 2 * vb * Kp + sd.x);
-          const double yb = __ldg(a.vtx + (2 * vb + 1) * Kp + sd.x);
-          const double r = 0.5 + 0.5 * tab.t1[j];
-          double vx, vy;
-          Eq::velocity(q, fma(r, xb - xa, xa), fma(r, yb - ya, ya), vx, vy);
-          Eq::riemann_at(vx, vy, UL, UR, nx, ny, sc, Fn);
-          done = true;
-        }
-      }
-      if (!done) Eq::riemann(q, UL, UR, nx, ny, sc, Fn);
-#pragma unroll
-      for (int n = 0; FS && n < N; n++) fs[n] = j == 0 ? Fn[n] : fs[n] + Fn[n];
-      store_vars<N>(F + j * N, Fn);
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < N1; j++) {
-      double Fn[N];
-      boundary_flux<Eq, P>(tab, q, a, s, sd, j, Fn);
-#pragma unroll
-      for (int n = 0; FS && n < N; n++) fs[n] = j == 0 ? Fn[n] : fs[n] + Fn[n];
-      store_vars<N>(F + j * N, Fn);
+      for (int jj = 1; jj < N1; jj++) v += sm[(r * N1 + jj) * N + n];
+      a.Fs[(size_t)(s0 + r) * N + n] = v;
     }
   }
-  pdl_end();
-  if (FS) store_vars<N>(a.Fs + (size_t)s * N, fs);
-}
-
-// threads of k_face: a side each, but without FS a boundary side has one per
-// edge point -- a ghost state may take a few hundred dependent FP64 operations
-// (sines and an exponential of an inflow), and the points of one thread, one
-// after the other, were the length of the whole launch on small meshes
-// (advection with a rotating inflow, 34k triangles, p = 3: 27 -> 14 us)
-template <int P, bool FS>
-__host__ __device__ __forceinline__ int face_threads(int S, int Sb) {
-  return FS ? S : S + Sb * P;
 }
 
 template <class Eq, int P, bool FS = false>
-__global__ void __launch_bounds__(kMaxBlock) k_face(const __grid_constant__ Tab<P> tab,
-                                                    const __grid_constant__ EqP q,
-                                                    const __grid_constant__ FaceArgs a) {
-  constexpr int N = Eq::N, N1 = P + 1;
+__global__ void __launch_bounds__(kFaceSides *(P + 1)) k_face(const __grid_constant__ Tab<P> tab,
+                                                              const __grid_constant__ EqP q,
+                                                              const __grid_constant__ FaceArgs a) {
+  __shared__ double sm[FS ? kFaceSides * (P + 1) * Eq::N : 1];
   pdl_begin();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (!FS && i < a.Sb * N1) {
-    const int s = i / N1, j = i % N1;
-    const int4 sd = a.side[s];
-    double Fn[N];
-    boundary_flux<Eq, P>(tab, q, a, s, sd, j, Fn);
-    pdl_end();
-    store_vars<N>(a.Fh + ((size_t)s * N1 + j) * N, Fn);
-    return;
-  }
-  const int s = FS ? i : i - a.Sb * P;
-  if (s < a.S) face_body<Eq, P, FS>(tab, q, a, s);
+  face_body<Eq, P, FS, kFaceSides>(tab, q, a, blockIdx.x * kFaceSides, a.S, threadIdx.x, sm);
+  pdl_end();
 }
 
 // ---------------------------------------------------------------------------
@@ -1012,14 +995,26 @@ __global__ void __launch_bounds__(kMaxBlock)
   }
 }
 
+// (blocks of 128 threads, as many sides as they have threads for at the
+// problem's order; `sub` of them for each block of `blk` sides of the map)
+template <class Eq, int P, bool FS>
+__device__ __forceinline__ void face_batch_body(const Tab<P> &tab, const EqP &q,
+                                                const FaceArgs &a, int s_map, int blk, int part,
+                                                double *sm) {
+  constexpr int kSides = kBlock / (P + 1);
+  const int s0 = s_map + part * kSides, s_end = min(a.S, s_map + blk);
+  if (s0 < s_end) face_body<Eq, P, FS, kSides>(tab, q, a, s0, s_end, threadIdx.x, sm);
+}
+
 template <class Eq, bool FS = false>
-__global__ void __launch_bounds__(kMaxBlock)
+__global__ void __launch_bounds__(kBlock)
     k_face_batch(const __grid_constant__ BatchTabs tb, const BatchProb *__restrict__ probs,
-                 const int *__restrict__ blk2prob, const int *__restrict__ blk0, double tcoef) {
-  const int pi = blk2prob[blockIdx.x];
+                 const int *__restrict__ blk2prob, const int *__restrict__ blk0, int blk, int sub,
+                 double tcoef) {
+  __shared__ double sm[FS ? kBlock * Eq::N : 1];
+  const int b = (int)blockIdx.x / sub, part = (int)blockIdx.x % sub, pi = blk2prob[b];
   const BatchProb &pr = probs[pi];
-  const int s = (blockIdx.x - blk0[pi]) * blockDim.x + threadIdx.x;
-  if (s >= pr.S) return;
+  const int s_map = (b - blk0[pi]) * blk;
   FaceArgs a;
   a.T = pr.T;
   a.side = pr.side;
@@ -1035,9 +1030,9 @@ __global__ void __launch_bounds__(kMaxBlock)
   a.Sb = pr.Sb;
   a.Kp = pr.Kp;
   switch (pr.p) {
-    case 1: face_body<Eq, 1, FS>(tb.t1, pr.q, a, s); break;
-    case 2: face_body<Eq, 2, FS>(tb.t2, pr.q, a, s); break;
-    case 3: face_body<Eq, 3, FS>(tb.t3, pr.q, a, s); break;
+    case 1: face_batch_body<Eq, 1, FS>(tb.t1, pr.q, a, s_map, blk, part, sm); break;
+    case 2: face_batch_body<Eq, 2, FS>(tb.t2, pr.q, a, s_map, blk, part, sm); break;
+    case 3: face_batch_body<Eq, 3, FS>(tb.t3, pr.q, a, s_map, blk, part, sm); break;
   }
 }
 
@@ -1203,8 +1198,8 @@ struct Launch {
     a.S = c.m.S;
     a.Sb = c.m.Sb;
     a.Kp = c.m.Kp;
-    DG_DISPATCH_P((launch(k_face<Eq, P, FS>, nblk(face_threads<P, FS>(c.m.S, c.m.Sb), c.blk), c.blk,
-                          c.st, tab<P>(c), *c.q, a)));
+    DG_DISPATCH_P((launch(k_face<Eq, P, FS>, nblk(c.m.S, kFaceSides), kFaceSides * (P + 1), c.st,
+                          tab<P>(c), *c.q, a)));
   }
   static void face(const Ctx &c, const double *t, double tcoef) {
     face_args<false>(c, t, tcoef, nullptr);
@@ -1325,9 +1320,11 @@ struct Launch {
     if constexpr (Eq::kFusedLimiter)  // the orders that contract in FP64
       k_trace_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0);
   }
+  // blocks of k_face_batch per block of the map: enough for p = 3's 32 sides
+  static int face_sub(const BatchLaunch &b) { return (b.blk + kBlock / 4 - 1) / (kBlock / 4); }
   static void b_face(const BatchLaunch &b, double tcoef) {
-    k_face_batch<Eq><<<b.nsblk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.sblk2prob, b.sblk0,
-                                                   tcoef);
+    k_face_batch<Eq><<<b.nsblk * face_sub(b), kBlock, 0, b.st>>>(
+        btabs(b), b.probs, b.sblk2prob, b.sblk0, b.blk, face_sub(b), tcoef);
   }
   template <bool LIM>
   static void b_element_v(const BatchLaunch &b, int stage) {
@@ -1364,8 +1361,8 @@ struct Launch {
   // the fused-limiter stage (instantiated only where an equation uses it)
   static void b_element_lim(const BatchLaunch &b, int stage) { b_element_v<true>(b, stage); }
   static void b_face_fs(const BatchLaunch &b, double tcoef) {
-    k_face_batch<Eq, true><<<b.nsblk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.sblk2prob, b.sblk0,
-                                                         tcoef);
+    k_face_batch<Eq, true><<<b.nsblk * face_sub(b), kBlock, 0, b.st>>>(
+        btabs(b), b.probs, b.sblk2prob, b.sblk0, b.blk, face_sub(b), tcoef);
   }
   static void b_means(const BatchLaunch &b, int stage) {
     k_means_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0,
