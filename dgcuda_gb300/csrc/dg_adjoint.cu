@@ -28,13 +28,13 @@ bool lin_trace(const Ctx &c, const double *u, const double *scale, double sc, do
 }
 
 bool tl_face(const Ctx &c, const double *Tv, double *dFh) {
-  DG_LIN_P((k_sw_face_lin<P, false><<<nblk(c.m.S), kBlock, 0, c.st>>>(
+  DG_LIN_P((k_sw_face_lin<P, false><<<nblk(c.m.S * (P + 1)), kBlock, 0, c.st>>>(
       tabp<P>(c), *c.q, c.T, Tv, c.m.side, c.m.sgeo, dFh, nullptr, c.m.S)));
   return true;
 }
 
 bool adj_face(const Ctx &c, const double *Tbar, double *UbL, double *UbR) {
-  DG_LIN_P((k_sw_face_lin<P, true><<<nblk(c.m.S), kBlock, 0, c.st>>>(
+  DG_LIN_P((k_sw_face_lin<P, true><<<nblk(c.m.S * (P + 1)), kBlock, 0, c.st>>>(
       tabp<P>(c), *c.q, c.T, Tbar, c.m.side, c.m.sgeo, UbL, UbR, c.m.S)));
   return true;
 }

@@ -132,7 +132,8 @@ __global__ void __launch_bounds__(kBlock)
                   const int4 *__restrict__ side, const double *__restrict__ sgeo,
                   double *__restrict__ out0, double *__restrict__ out1, int S) {
   constexpr int N = 3, N1 = P + 1;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  // a thread per edge point, as k_face
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, s = i / N1, j = i % N1;
   if (s >= S) return;
   const int4 sd = side[s];
   const double nx = sgeo[s], ny = sgeo[S + s], hl = sgeo[2 * (size_t)S + s];
@@ -141,8 +142,7 @@ __global__ void __launch_bounds__(kBlock)
   const bool inner = sd.y >= 0;
   const double *TR = inner ? T + ((size_t)sd.y * 3 + sd.w) * (N1 * N) : nullptr;
   const double *VR = inner ? Tv + ((size_t)sd.y * 3 + sd.w) * (N1 * N) : nullptr;
-#pragma unroll
-  for (int j = 0; j < N1; j++) {
+  {
     double UL[N], UR[N], M[3][3];
 #pragma unroll
     for (int n = 0; n < N; n++) UL[n] = TL[j * N + n];

@@ -525,8 +525,6 @@ __device__ __forceinline__ void means_body(const Tab<P> &tab, const ElemArgs &a,
   const size_t Kp = a.Kp;
   double sum[N];
 #pragma unroll
-  for (int n = 0; n < N; n++) sum[n] = 0.0;
-#pragma unroll
   for (int f = 0; f < 3; f++) {
     const int sd = a.esd[f * Kp + e];
     double F[N];
@@ -534,16 +532,18 @@ __device__ __forceinline__ void means_body(const Tab<P> &tab, const ElemArgs &a,
     // the sign as a bit flip (exactly -F), off the FP64 pipe
     const long long sg = (sd & 1) ? 0ll : (long long)0x8000000000000000ull;
 #pragma unroll
-    for (int n = 0; n < N; n++) sum[n] += __longlong_as_double(sg ^ __double_as_longlong(F[n]));
+    for (int n = 0; n < N; n++) {
+      const double v = __longlong_as_double(sg ^ __double_as_longlong(F[n]));
+      sum[n] = f == 0 ? v : sum[n] + v;
+    }
   }
-  const double sc = a.cc * *a.dtp * a.geo[4 * Kp + e];
-  const double e0 = tab.E[0][0][0];
+  const double sc = a.cc * *a.dtp * a.geo[4 * Kp + e] * tab.E[0][0][0];
   pdl_end();
 #pragma unroll
   for (int n = 0; n < N; n++) {
     const size_t o = (size_t)(n * NP) * Kp + e;
-    double v = fma(sc, sum[n] * e0, a.cb == 1.0 ? a.us[o] : a.cb * a.us[o]);
-    if (a.ca != 0.0) v = fma(a.ca, a.un[o], v);
+    double v = fma(sc, sum[n], a.unit_cb ? a.us[o] : a.cb * a.us[o]);
+    if (a.has_un) v = fma(a.ca, a.un[o], v);
     M[(size_t)n * Kp + e] = v;
   }
 }
@@ -767,9 +767,11 @@ __device__ __forceinline__ double cell_speed(const Tab<P> &tab, const EqP &q,
   atomicExch(&ds->status, 4);
   return 0.0;
 }
-// lam: this thread's maximum; nblocks: the blocks that meet in ds
-__device__ __forceinline__ void cfl_reduce(double lam, DevScalars *ds, unsigned nblocks, int p,
-                                           int mode) {
+// lam: this thread's maximum; nblocks: the blocks that meet in ds; d: thread
+// 0's copy of *ds from the start of the kernel (no block but the last writes
+// what the step is taken from, so its loads need not wait for the maximum)
+__device__ __forceinline__ void cfl_reduce(double lam, DevScalars *ds, DevScalars &d,
+                                           unsigned nblocks, int p, int mode) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lam = larger(lam, __shfl_xor_sync(0xffffffffu, lam, o));
   __shared__ double sm[kBlock / 32];
@@ -777,6 +779,7 @@ __device__ __forceinline__ void cfl_reduce(double lam, DevScalars *ds, unsigned 
   __syncthreads();
   if (threadIdx.x != 0) return;
   double m = sm[0];
+#pragma unroll
   for (int w = 1; w < kBlock / 32; w++) m = larger(m, sm[w]);
   if (nblocks > 1) {
     atomicMax(&ds->lam_bits, (unsigned long long)__double_as_longlong(m));
@@ -786,22 +789,32 @@ __device__ __forceinline__ void cfl_reduce(double lam, DevScalars *ds, unsigned 
     m = __longlong_as_double((long long)atomicExch(&ds->lam_bits, 0ull));
     ds->ticket = 0;
   }
-  cfl_step(ds, m, p, mode);
+  d.status = 0;
+  cfl_step(&d, m, p, mode);
+  ds->t = d.t;
+  ds->dt = d.dt;
+  ds->lam = d.lam;
+  ds->steps = d.steps;
+  ds->last = d.last;
+  ds->pending = d.pending;
+  if (d.status) ds->status = d.status;  // else what a NaN speed may have set stays
 }
 
-// of a single problem, grid-stride: a few blocks per SM each take the max over
-// many elements, so their atomics on one word stay cheap
-constexpr int kLambdaBlocks = 1024;
+// of a single problem, grid-stride: a few blocks per SM, so that the atomics on
+// the two words stay few
+constexpr int kLambdaBlocks = 608;
 template <class Eq, int P>
 __global__ void __launch_bounds__(kBlock) k_lambda(const __grid_constant__ Tab<P> tab,
                                                    const __grid_constant__ EqP q,
                                                    const double *__restrict__ u, DevScalars *ds,
                                                    int K, int Kp, int mode) {
   pdl_begin();
+  DevScalars d;
+  if (threadIdx.x == 0) d = *ds;
   double lam = 0.0;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < K; e += gridDim.x * blockDim.x)
     lam = larger(lam, cell_speed<Eq, P>(tab, q, u, ds, Kp, e));
-  cfl_reduce(lam, ds, gridDim.x, P, mode);
+  cfl_reduce(lam, ds, d, gridDim.x, P, mode);
 }
 
 // ---------------------------------------------------------------------------
@@ -1074,6 +1087,8 @@ __global__ void __launch_bounds__(kBlock)
   const int pi = blk2prob[blockIdx.x];
   const BatchProb &pr = probs[pi];
   const int e = (blockIdx.x - blk0[pi]) * blockDim.x + threadIdx.x;
+  DevScalars d;
+  if (threadIdx.x == 0) d = *pr.ds;
   double lam = 0.0;
   if (e < pr.K) {
     switch (pr.p) {
@@ -1082,7 +1097,7 @@ __global__ void __launch_bounds__(kBlock)
       case 3: lam = cell_speed<Eq, 3>(tb.t3, pr.q, pr.U, pr.ds, pr.Kp, e); break;
     }
   }
-  cfl_reduce(lam, pr.ds, (unsigned)(pr.K + kBlock - 1) / kBlock, pr.p, CFL_SSP);
+  cfl_reduce(lam, pr.ds, d, (unsigned)(pr.K + kBlock - 1) / kBlock, pr.p, CFL_SSP);
 }
 
 // ---------------------------------------------------------------------------
