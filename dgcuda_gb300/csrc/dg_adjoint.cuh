@@ -54,12 +54,12 @@ struct SwTrace {
 };
 __device__ __forceinline__ SwTrace sw_trace(double g, const double *U, double nx, double ny) {
   SwTrace w;
-  w.ih = rcp(U[0]);
+  w.ih = rcp_fx(U[0]);
   w.u = U[1] * w.ih;
   w.v = U[2] * w.ih;
   w.qh = fma(U[1], nx, U[2] * ny) * w.ih;
   w.gh = g * U[0];
-  w.c = sqrt_pos(w.gh);
+  w.c = sqrt_fx(w.gh);
   w.lam = fabs(w.qh) + w.c;
   return w;
 }

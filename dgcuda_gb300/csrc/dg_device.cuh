@@ -208,6 +208,87 @@ DG_HD double sqrt_pos(double x) {
   return sqrt(x);
 }
 
+// 1/x and sqrt(x) on the integer pipes, for kernels that wait on the FP64 pipe
+// alone (the face kernels run it at 88 % with the integer pipes at 2 %): an FP64
+// operation occupies its pipe for 16 cycles of an SM, as long as 32 integer
+// operations theirs.  Both refine a single-precision seed (rcp.approx.ftz.f32,
+// rsqrt.approx.ftz.f32, 22 bits or more) by the same third-order steps as rcp()
+// and sqrt_pos(), in 64-bit fixed point, and round once: within 0.64 and 0.67
+// ulp of the exact value (30 million arguments over all exponents, with
+// seeds off by up to 1 and 2 ulp more; the algebra alone bounds them by 0.82
+// and 0.75).  Zeros, denormals, infinities, NaN (and 1/x below 2^-1021, negative
+// radicands) go the FP64 way.
+DG_HD double rcp_fx(double x) {
+#ifdef __CUDA_ARCH__
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned ax = hi & 0x7FFFFFFFu;
+  const int ex = (int)(ax >> 20);
+  if ((unsigned)(ex - 1) > 2042u) return rcp(x);
+  // |x| = X 2^(ex - 1075), f = X 2^-52 in [1, 2); R = r 2^24, r = 1/f to 22 bits
+  const unsigned mh = (ax & 0xFFFFFu) | 0x100000u;
+  float seed;
+  asm("rcp.approx.ftz.f32 %0, %1;"
+      : "=f"(seed)
+      : "f"(__uint_as_float(0x3F800000u | ((ax & 0xFFFFFu) << 3) | (lo >> 29))));
+  const unsigned R = __float_as_uint(seed) - 0x3E800000u;
+  // e = 1 - f r, below 2^-21.8: E = e 2^76, the low 64 bits of -X R
+  const long long E = -(long long)((unsigned long long)lo * R + ((unsigned long long)(mh * R) << 32));
+  // r (1 + e + e^2) in units of 2^-56
+  const int Eh = (int)(E >> 24), q = (int)(E >> 39);
+  const unsigned El = (unsigned)E & 0xFFFFFFu;
+  const long long t1 =
+      ((long long)(int)R * Eh + (long long)(((unsigned long long)R * El) >> 24)) >> 20;
+  const unsigned long long t2 = ((unsigned long long)R * (unsigned)(q * q)) >> 42;
+  const unsigned long long m =
+      (((unsigned long long)R << 32) + (unsigned long long)t1 + t2 + 4) >> 3;
+  const unsigned oh = (unsigned)(m >> 32) + ((unsigned)(2044 - ex) << 20);
+  return __hiloint2double((int)(oh | (hi & 0x80000000u)), (int)(unsigned)m);
+#else
+  return 1.0 / x;
+#endif
+}
+DG_HD double sqrt_fx(double x) {
+#ifdef __CUDA_ARCH__
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  if (hi - 0x00100000u >= 0x7FE00000u) return sqrt(x);
+  const int ex = (int)(hi >> 20), odd = 1 - (ex & 1);
+  // x = f 4^k, f = F 2^-52 in [1, 4); R = r 2^24, r = f^(-1/2) to 22 bits
+  const unsigned long long F =
+      (((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo) << odd;
+  float seed;
+  asm("rsqrt.approx.ftz.f32 %0, %1;"
+      : "=f"(seed)
+      : "f"(__uint_as_float((0x3F800000u + ((unsigned)odd << 23)) | ((hi & 0xFFFFFu) << 3) |
+                            (lo >> 29))));
+  const unsigned R = __float_as_uint(seed) - 0x3E800000u;
+  // e = 1 - f r^2, below 2^-20.6: E = e 2^76, the low 64 bits of -(F R^2 >> 24)
+  const unsigned long long G = (unsigned long long)R * R;
+  const unsigned Fh = (unsigned)(F >> 32), Fl = (unsigned)F, Gh = (unsigned)(G >> 32),
+                 Gl = (unsigned)G;
+  const unsigned long long A =
+      (unsigned long long)Fh * Gl + ((unsigned long long)(Fh * Gh) << 32);
+  const long long E = -(long long)((A << 8) + (((unsigned long long)Fl * Gl) >> 24) +
+                                   (((unsigned long long)Fl * Gh) << 8));
+  // t = e / 2 + 3 e^2 / 8 in units of 2^-64; sqrt(f) = s (1 + t), s = f r in units
+  // of 2^-56
+  const int q = (int)(E >> 40);
+  const long long T = (E >> 13) + (long long)((((unsigned)(q * q) >> 3) * 3u) >> 8);
+  const unsigned long long s =
+      (((unsigned long long)Fh * R) << 12) + (((unsigned long long)Fl * R) >> 20);
+  const int sh = (int)(s >> 27), sl = (int)((unsigned)s & 0x7FFFFFFu);
+  const int Th = (int)(T >> 12);
+  const unsigned Tl = (unsigned)T & 0xFFFu;
+  const long long c =
+      (((long long)sh * Th + (long long)(((unsigned long long)(unsigned)sh * Tl) >> 12)) >> 25) +
+      (((long long)sl * (int)(T >> 21)) >> 43);
+  const unsigned long long m = (s + (unsigned long long)c + 8) >> 4;
+  const unsigned oh = (unsigned)(m >> 32) + ((unsigned)(((ex + 1023 - odd) >> 1) - 1) << 20);
+  return __hiloint2double((int)oh, (int)(unsigned)m);
+#else
+  return sqrt(x);
+#endif
+}
+
 // --------------------------------------------------------------------------
 // problem plugins: exact / initial / inflow state (U0, U_exact, U_inflow)
 // --------------------------------------------------------------------------
@@ -481,17 +562,18 @@ struct Euler {  // euler/euler.cu
                             double ny, double sc, double *F) {
     // every multiply-add is an explicit fma so the rounding does not depend
     // on how the compiler contracts the expression in a given kernel; the
-    // normal momenta m . n are the mass fluxes themselves.  62 FP64
+    // normal momenta m . n are the mass fluxes themselves.  46 FP64
     // operations, what k_face is bound by (67 with the scale applied to the
-    // fluxes, products by -1/2 and fmax)
+    // fluxes, products by -1/2, fmax, and the reciprocals and square roots on
+    // the FP64 pipe)
     const double sx = sc * nx, sy = sc * ny;
-    const double irl = rcp(UL[0]), irr = rcp(UR[0]);
+    const double irl = rcp_fx(UL[0]), irr = rcp_fx(UR[0]);
     const double mnl = fma(UL[1], sx, UL[2] * sy), mnr = fma(UR[1], sx, UR[2] * sy);
     const double snl = mnl * irl, snr = mnr * irr;
     const double m2l = fma(UL[1], UL[1], UL[2] * UL[2]), m2r = fma(UR[1], UR[1], UR[2] * UR[2]);
     const double pl = mul_rn(q.gamma - 1., fma(neg_half(m2l), irl, UL[3]));
     const double pr = mul_rn(q.gamma - 1., fma(neg_half(m2r), irr, UR[3]));
-    const double cl = sqrt_pos(q.gamma * pl * irl), cr = sqrt_pos(q.gamma * pr * irr);
+    const double cl = sqrt_fx(q.gamma * pl * irl), cr = sqrt_fx(q.gamma * pr * irr);
     const double lam = larger(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
     const double P = pl + pr;
     F[0] = fma(lam, UL[0] - UR[0], mnl + mnr);
@@ -501,12 +583,12 @@ struct Euler {  // euler/euler.cu
   }
   DG_HD static double mean_speed(const EqP &q, const double *U) {  // euler.cu:248-277
     // 1/rho and the square roots within 1 ulp of IEEE division and sqrt
-    // (rcp, sqrt_pos): the wave speed is the CFL step's to 1e-15
-    const double ir = rcp(U[0]);
+    // (rcp_fx, sqrt_fx): the wave speed is the CFL step's to 1e-15
+    const double ir = rcp_fx(U[0]);
     const double m2 = fma(U[1], U[1], U[2] * U[2]);
     const double p = (q.gamma - 1.) * fma(-0.5 * m2, ir, U[3]);
-    const double c = sqrt_pos(q.gamma * p * ir);
-    const double s = sqrt_pos(m2) * ir;
+    const double c = sqrt_fx(q.gamma * p * ir);
+    const double s = sqrt_fx(m2) * ir;
     return s > 0 ? s + c : -s + c;
   }
   DG_HD static void reflect(const EqP &q, const double *UL, double *UR, double x, double y,
@@ -559,10 +641,10 @@ struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
                             double ny, double sc, double *F) {  // shallowwater.cu:118-185
     // the normal momenta m . n are the mass fluxes themselves
     const double sx = sc * nx, sy = sc * ny;
-    const double ihl = rcp(UL[0]), ihr = rcp(UR[0]);
+    const double ihl = rcp_fx(UL[0]), ihr = rcp_fx(UR[0]);
     const double mnl = fma(sx, UL[1], sy * UL[2]), mnr = fma(sx, UR[1], sy * UR[2]);
     const double snl = mnl * ihl, snr = mnr * ihr;
-    const double cl = sqrt_pos(UL[0] * q.g), cr = sqrt_pos(UR[0] * q.g);
+    const double cl = sqrt_fx(UL[0] * q.g), cr = sqrt_fx(UR[0] * q.g);
     const double lam = larger(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
     const double P = 0.5 * q.g * fma(UL[0], UL[0], UR[0] * UR[0]);
     F[0] = fma(lam, UL[0] - UR[0], mnl + mnr);
@@ -570,9 +652,9 @@ struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
     F[2] = fma(lam, UL[2] - UR[2], fma(UL[2], snl, fma(UR[2], snr, P * sy)));
   }
   DG_HD static double mean_speed(const EqP &q, const double *U) {  // shallowwater.cu:196-224
-    // as Euler's: rcp and sqrt_pos within 1 ulp of IEEE division and sqrt
-    const double c = sqrt_pos(U[0] * q.g);
-    const double s = sqrt_pos(fma(U[1], U[1], U[2] * U[2])) * rcp(U[0]);
+    // as Euler's: rcp_fx and sqrt_fx within 1 ulp of IEEE division and sqrt
+    const double c = sqrt_fx(U[0] * q.g);
+    const double s = sqrt_fx(fma(U[1], U[1], U[2] * U[2])) * rcp_fx(U[0]);
     return s > 0 ? s + c : -s + c;
   }
   DG_HD static void reflect(const EqP &, const double *UL, double *UR, double, double, double nx,

@@ -22,18 +22,23 @@ __global__ void k_fma64(double *out, int iters, double a, double b) {
   for (int k = 0; k < 8; k++) s += x[k];
   out[blockIdx.x * blockDim.x + threadIdx.x] = s;
 }
+// of the two forms' results the one farther from q (a NaN counts as farthest)
+__device__ double farther(double a, double b, double q) {
+  if (a != a || b != b) return a != a ? (b != b || q == q ? a : b) : (q == q ? b : a);
+  return fabs(a - q) >= fabs(b - q) ? a : b;
+}
 __global__ void k_reciprocal(const double *x, double *r, double *q, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    r[i] = dg::rcp(x[i]);
     q[i] = 1.0 / x[i];
+    r[i] = farther(dg::rcp(x[i]), dg::rcp_fx(x[i]), q[i]);
   }
 }
 __global__ void k_sqrt(const double *x, double *r, double *q, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    r[i] = dg::sqrt_pos(x[i]);
     q[i] = __dsqrt_rn(x[i]);
+    r[i] = farther(dg::sqrt_pos(x[i]), dg::sqrt_fx(x[i]), q[i]);
   }
 }
 __global__ void k_physical(const double *U, int *fast, int *exact, int n) {
@@ -75,8 +80,8 @@ extern "C" dg_status dg_probe_physical(int device, int n, const double *U, int *
   return e == cudaSuccess ? DG_OK : dg::fail(DG_CUDA_ERROR, cudaGetErrorString(e));
 }
 
-// the sound speed's square root (dg::sqrt_pos) and IEEE sqrt on the device
-// for n host values: r[i] = sqrt_pos(x[i]), q[i] = sqrt(x[i])
+// the sound speed's square root (dg::sqrt_pos and sqrt_fx, the one farther from
+// q) and IEEE sqrt on the device for n host values: q[i] = sqrt(x[i])
 extern "C" dg_status dg_probe_sqrt(int device, int n, const double *x, double *r, double *q) {
   if (n < 0 || (n && (!x || !r || !q))) return dg::fail(DG_BAD_ARG, "bad arguments");
   if (!n) return DG_OK;
@@ -95,8 +100,8 @@ extern "C" dg_status dg_probe_sqrt(int device, int n, const double *x, double *r
   return e == cudaSuccess ? DG_OK : dg::fail(DG_CUDA_ERROR, cudaGetErrorString(e));
 }
 
-// the flux kernels' reciprocal (dg::rcp) and IEEE division on the device for
-// n host values: r[i] = rcp(x[i]), q[i] = 1 / x[i]
+// the flux kernels' reciprocal (dg::rcp and rcp_fx, the one farther from q) and
+// IEEE division on the device for n host values: q[i] = 1 / x[i]
 extern "C" dg_status dg_probe_reciprocal(int device, int n, const double *x, double *r,
                                          double *q) {
   if (n < 0 || (n && (!x || !r || !q))) return dg::fail(DG_BAD_ARG, "bad arguments");
