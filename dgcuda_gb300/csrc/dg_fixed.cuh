@@ -52,13 +52,8 @@
 namespace dg {
 namespace fx {
 
-constexpr int kLow = 28;                 // bits of the low limb
 constexpr int kTile = 32;                // elements of a block
 constexpr int kPitch = kTile + 1;        // shared row pitch: rows and columns both conflict-free
-
-struct Limb {
-  int h, l;
-};
 
 // tables of order P in limbs, and what the FP64 parts need of Tab<P>
 template <int P>
@@ -74,81 +69,6 @@ struct FxTab {
   double r[NQ], s[NQ], B0[NQ];           // area points, phi_0 there
   double phi0, e0;                       // phi_0 (area point 0), phi_0 on the edges
 };
-
-// ---- rows -----------------------------------------------------------------
-// a row whose largest entry has biased exponent m.  A row of zeros (or
-// denormals only) takes an exponent that shifts every entry out: all its
-// limbs and sums are zero.  Other rows outside [100, 1900], where a result
-// could leave the normal range, and rows with an infinity or a NaN are
-// odd(): finish() forms their sums as if m were 1023 and fix() scales them
-struct Row {
-  int m;
-  __device__ __forceinline__ bool odd() const { return (unsigned)(m - 100) > 1800u; }
-};
-__device__ __forceinline__ Row make_row(int maxhi) {
-  Row r;
-  r.m = maxhi >> 20;
-  if (r.m == 0) r.m = 1023;
-  return r;
-}
-__device__ __forceinline__ int abs_hi(double x) { return __double2hiint(x) & 0x7FFFFFFF; }
-
-// x on row r: the two limbs
-__device__ __forceinline__ void to_limbs(double x, const Row &r, int &h, int &l) {
-  const int hi = __double2hiint(x);
-  const unsigned lo = (unsigned)__double2loint(x);
-  const int e = (hi >> 20) & 0x7FF;
-  const unsigned mh = ((unsigned)hi & 0xFFFFFu) | 0x100000u;
-  unsigned long long X = (((unsigned long long)mh << 32) | lo) << 3;
-  X >>= min(r.m - e, 63);
-  const int sg = (hi >> 31) | 1;
-  h = (int)(X >> kLow) * sg;
-  l = (int)((unsigned)X & ((1u << kLow) - 1)) * sg;
-}
-
-struct Sum {
-  long long H, M;
-};
-__device__ __forceinline__ void zero(Sum &s) {
-  s.H = 0;
-  s.M = 1ll << (kLow - 1);  // the rounding of M >> 28
-}
-__device__ __forceinline__ void mac(Sum &s, int h, int l, const Limb &t) {
-  s.H += (long long)h * t.h;
-  s.M += (long long)h * t.l;
-  s.M += (long long)l * t.h;
-}
-
-// the results of an odd row, `count` doubles `step` apart, formed with exponent
-// 1023 in place of the row's
-static __device__ __noinline__ void fix(double *v, int step, int count, Row r) {
-  for (int k = 0; k < count; k++, v += step)
-    *v = r.m == 0x7FF ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(*v, r.m - 1023);
-}
-
-// the exponent finish() attaches for results of row r and a table of biased
-// exponent M
-__device__ __forceinline__ int base_exp(Row r, int M) {
-  return (r.odd() ? 1023 : r.m) + M - 1015;
-}
-// the sum as a double, S 2^(base - 1085) with S = H + (M >> 28): magnitude
-// (of a negative S as |S| - 1: half an ulp of a result of full scale over 8),
-// normalised so that 63 bits are used, rounded to 53 (half away from zero),
-// exponent and sign attached
-__device__ __forceinline__ double finish(const Sum &s, int base) {
-  const long long S = s.H + (s.M >> kLow);
-  const int sg = (int)(S >> 63);
-  const unsigned ah = (unsigned)((int)(S >> 32) ^ sg), al = (unsigned)((int)S ^ sg);
-  const bool small = ah == 0;  // below 2^32: normalise a 2^31 instead
-  const unsigned top = small ? al >> 1 : ah, low = small ? al << 31 : al;
-  int b;  // index of the leading bit of top < 2^31, -1 for top = 0
-  asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(top));
-  const unsigned nh = __funnelshift_l(low, top, 30 - b), nl = low << ((30 - b) & 31);
-  const unsigned long long f = ((((unsigned long long)nh << 32) | nl) + 0x200ull) >> 10;
-  unsigned hi = (unsigned)(f >> 32) + ((unsigned)((small ? base - 62 : base - 31) + b) << 20);
-  if ((ah | al) == 0) hi = 0;  // f is 0 then
-  return __hiloint2double((int)(hi | ((unsigned)sg & 0x80000000u)), (int)(unsigned)f);
-}
 
 // ---- shared memory of a block ----------------------------------------------
 // rows of kPitch doubles: g of variable n at point q in row q N + n, h in row

@@ -1,0 +1,153 @@
+// dg_limbs.cuh -- doubles as 56-bit fixed point in two limbs, X = h 2^28 + l,
+// and sums of their products in integer multiply-adds: the arithmetic of the
+// fixed-point element stage (dg_fixed.cuh, which says why) and of the face
+// kernels' momentum sums.
+#pragma once
+#include <cuda_runtime.h>
+
+#ifdef __CUDACC__
+namespace dg {
+namespace fx {
+
+constexpr int kLow = 28;                 // bits of the low limb
+
+struct Limb {
+  int h, l;
+};
+
+// ---- rows -----------------------------------------------------------------
+// a row whose largest entry has biased exponent m.  A row of zeros (or
+// denormals only) takes an exponent that shifts every entry out: all its
+// limbs and sums are zero.  Other rows outside [100, 1900], where a result
+// could leave the normal range, and rows with an infinity or a NaN are
+// odd(): finish() forms their sums as if m were 1023 and fix() scales them
+struct Row {
+  int m;
+  __device__ __forceinline__ bool odd() const { return (unsigned)(m - 100) > 1800u; }
+};
+__device__ __forceinline__ Row make_row(int maxhi) {
+  Row r;
+  r.m = maxhi >> 20;
+  if (r.m == 0) r.m = 1023;
+  return r;
+}
+__device__ __forceinline__ int abs_hi(double x) { return __double2hiint(x) & 0x7FFFFFFF; }
+
+// x on row r: the two limbs
+__device__ __forceinline__ void to_limbs(double x, const Row &r, int &h, int &l) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const int e = (hi >> 20) & 0x7FF;
+  const unsigned mh = ((unsigned)hi & 0xFFFFFu) | 0x100000u;
+  unsigned long long X = (((unsigned long long)mh << 32) | lo) << 3;
+  X >>= min(r.m - e, 63);
+  const int sg = (hi >> 31) | 1;
+  h = (int)(X >> kLow) * sg;
+  l = (int)((unsigned)X & ((1u << kLow) - 1)) * sg;
+}
+
+struct Sum {
+  long long H, M;
+};
+__device__ __forceinline__ void zero(Sum &s) {
+  s.H = 0;
+  s.M = 1ll << (kLow - 1);  // the rounding of M >> 28
+}
+__device__ __forceinline__ void mac(Sum &s, int h, int l, const Limb &t) {
+  s.H += (long long)h * t.h;
+  s.M += (long long)h * t.l;
+  s.M += (long long)l * t.h;
+}
+
+// the results of an odd row, `count` doubles `step` apart, formed with exponent
+// 1023 in place of the row's
+static __device__ __noinline__ void fix(double *v, int step, int count, Row r) {
+  for (int k = 0; k < count; k++, v += step)
+    *v = r.m == 0x7FF ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(*v, r.m - 1023);
+}
+
+// the exponent finish() attaches for results of row r and a table of biased
+// exponent M
+__device__ __forceinline__ int base_exp(Row r, int M) {
+  return (r.odd() ? 1023 : r.m) + M - 1015;
+}
+// the sum as a double, S 2^(base - 1085) with S = H + (M >> 28): magnitude
+// (of a negative S as |S| - 1: half an ulp of a result of full scale over 8),
+// normalised so that 63 bits are used, rounded to 53 (half away from zero),
+// exponent and sign attached
+__device__ __forceinline__ double finish(const Sum &s, int base) {
+  const long long S = s.H + (s.M >> kLow);
+  const int sg = (int)(S >> 63);
+  const unsigned ah = (unsigned)((int)(S >> 32) ^ sg), al = (unsigned)((int)S ^ sg);
+  const bool small = ah == 0;  // below 2^32: normalise a 2^31 instead
+  const unsigned top = small ? al >> 1 : ah, low = small ? al << 31 : al;
+  int b;  // index of the leading bit of top < 2^31, -1 for top = 0
+  asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(top));
+  const unsigned nh = __funnelshift_l(low, top, 30 - b), nl = low << ((30 - b) & 31);
+  const unsigned long long f = ((((unsigned long long)nh << 32) | nl) + 0x200ull) >> 10;
+  unsigned hi = (unsigned)(f >> 32) + ((unsigned)((small ? base - 62 : base - 31) + b) << 20);
+  if ((ah | al) == 0) hi = 0;  // f is 0 then
+  return __hiloint2double((int)(hi | ((unsigned)sg & 0x80000000u)), (int)(unsigned)f);
+}
+
+// ---- sums of two products of variables (face kernels) -----------------------
+// two doubles on one row
+struct Pair {
+  Row r;
+  Limb a, b;
+};
+__device__ __forceinline__ Pair make_pair(double a, double b) {
+  Pair p;
+  p.r = make_row(max(abs_hi(a), abs_hi(b)));
+  to_limbs(a, p.r, p.a.h, p.a.l);
+  to_limbs(b, p.r, p.b.h, p.b.l);
+  return p;
+}
+// whether products of rows x and y stay in the normal range (rows of infinities
+// and NaN are odd)
+__device__ __forceinline__ bool in_range(Row x, Row y) {
+  return !x.odd() && !y.odd() && (unsigned)(x.m + y.m - 1200) < 1700u;
+}
+// x.a y.a + x.b y.b
+__device__ __forceinline__ double dot(const Pair &x, const Pair &y) {
+  Sum s;
+  zero(s);
+  mac(s, x.a.h, x.a.l, y.a);
+  mac(s, x.b.h, x.b.l, y.b);
+  return finish(s, base_exp(x.r, y.r.m));
+}
+// -(x.a^2 + x.b^2) / 2
+__device__ __forceinline__ double neg_half_square(const Pair &x) {
+  Sum s;
+  zero(s);
+  s.H += (long long)x.a.h * x.a.h;
+  s.H += (long long)x.b.h * x.b.h;
+  s.M += (long long)x.a.h * (2 * x.a.l);
+  s.M += (long long)x.b.h * (2 * x.b.l);
+  const double v = finish(s, base_exp(x.r, x.r.m) - 1);
+  return __hiloint2double(__double2hiint(v) ^ (int)0x80000000, __double2loint(v));
+}
+// xa ya + xb yb, the two products on rows of their own: the smaller scale is
+// shifted to the larger one (a zero product, whose rows may be stand-ins for
+// rows of zeros, takes the other's)
+__device__ __forceinline__ double sum2(const Limb &xa, int xm, const Limb &ya, int ym,
+                                       const Limb &xb, int um, const Limb &yb, int vm) {
+  Sum p, q;
+  zero(p);
+  zero(q);
+  mac(p, xa.h, xa.l, ya);
+  mac(q, xb.h, xb.l, yb);
+  const long long P = p.H + (p.M >> kLow), Q = q.H + (q.M >> kLow);
+  int ep = xm + ym, eq = um + vm;
+  if (P == 0) ep = eq;
+  if (Q == 0) eq = ep;
+  const int d = ep - eq;
+  Sum s;
+  s.H = d >= 0 ? P + (Q >> min(d, 63)) : Q + (P >> min(-d, 63));
+  s.M = 0;
+  return finish(s, max(ep, eq) - 1015);
+}
+
+}  // namespace fx
+}  // namespace dg
+#endif
