@@ -176,33 +176,13 @@ __device__ __forceinline__ bool physical_f32(const double *U) {
 }
 #endif
 
-// sqrt(x) for the sound speeds, from the approximate reciprocal square root
-// y of the PTX instruction rsqrt.approx.ftz.f64: with s = x y and e = 1 - s y
-// (= 1 - x y^2), sqrt(x) = s (1 - e)^(-1/2) = s (1 + e/2 + 3 e^2 / 8 + ...),
-// and the truncated series leaves a relative error of about e^3.  Five FP64
-// operations; arguments outside the positive normal range (0, denormals,
-// infinities, NaN, negatives) take the IEEE square root.  Checked against
-// IEEE sqrt by dg_probe_sqrt (within 1 ulp).
-DG_HD double sqrt_pos(double x) {
-#ifdef __CUDA_ARCH__
-  const unsigned hi = (unsigned)__double2hiint(x);
-  if (hi - 0x00100000u < 0x7FE00000u) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double s = x * y;
-    const double e = fma(-s, y, 1.0);
-    return fma(s, e * fma(e, 0.375, 0.5), s);
-  }
-#endif
-  return sqrt(x);
-}
-
 // 1/x and sqrt(x) on the integer pipes, for kernels that wait on the FP64 pipe
 // alone (the face kernels run it at 88 % with the integer pipes at 2 %): an FP64
 // operation occupies its pipe for 16 cycles of an SM, as long as 32 integer
 // operations theirs.  Both refine a single-precision seed (rcp.approx.ftz.f32,
-// rsqrt.approx.ftz.f32, 22 bits or more) by the same third-order steps as rcp()
-// and sqrt_pos(), in 64-bit fixed point, and round once: within 0.64 and 0.67
+// rsqrt.approx.ftz.f32, 22 bits or more) by third-order steps (1 + e + e^2 as in
+// rcp(); s = x r, e = 1 - x r^2, s + s (e / 2 + 3 e^2 / 8), the series of
+// (1 - e)^(-1/2)), in 64-bit fixed point, and round once: within 0.64 and 0.67
 // ulp of the exact value (30 million arguments over all exponents, with
 // seeds off by up to 1 and 2 ulp more; the algebra alone bounds them by 0.82
 // and 0.75).  Zeros, denormals, infinities, NaN (and 1/x below 2^-1021, negative
@@ -436,7 +416,8 @@ DG_HD void init_state(const EqP &q, double *U, double x, double y) {
 // Euler's 46 FP64 operations a point, 8 of shallow water's 28 (k_face,
 // us: Euler p = 3, 2.1M triangles 1270 -> 1007, p = 1 627 -> 496; shallow water p =
 // 2, 131k 48.9 -> 41.8).  Errors against rational arithmetic, in units of 2^-53 of
-// the largest product: 1.5 (m . n; FP64 1.8), 1.8 (advected momenta; FP64 2.0).
+// the largest product: 1.5 (m . n; FP64 1.8), 1.2 (|m|^2; 1.9), 1.8 (advected
+// momenta; 2.0).
 // Where an exponent leaves the range (infinities, NaN, extreme states), and on
 // the host, in FP64.
 struct FluxMomentum {

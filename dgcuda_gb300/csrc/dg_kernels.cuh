@@ -2,43 +2,44 @@
 //
 // One RK stage is three kernels plus an optional limiter pass:
 //
-//   k_trace    one thread per element: the solution's values at the
-//              3 x (p+1) Gauss points of its faces ("traces"), written
-//              [elem][face][j][var]; an element with a non-physical trace is
-//              flattened to its mean first (check_physical, euler.cu:92-116).
-//   k_face     one thread per side: the numerical flux F*(u-, u+; n) at each
-//              edge point, the right trace read at the mirrored point p-j
+//   k_trace    the solution's values at the 3 x (p+1) Gauss points of each
+//              element's faces ("traces"), written [elem][face][j][var]; an
+//              element with a non-physical trace is flattened to its mean
+//              first (check_physical, euler.cu:92-116).
+//   k_face     one thread per edge point: the numerical flux F*(u-, u+; n),
+//              the right trace read at the mirrored point p-j
 //              (eval_left_right, conserv_kernels.cu:850-892) or built from
 //              the boundary code (eval_boundary, :820-843), scaled by
 //              len/2 * w_j and stored [side][j][var].  Each flux is computed
 //              once, where the reference's element-side formulation needs it
 //              once per side too (eval_surface, :899-985).
-//   k_element  one thread per element: the volume integral (eval_volume,
-//              :992-1083) -- solution and flux at the area points projected
-//              on the weighted basis gradients through the element metric --
-//              plus a deterministic gather of the three faces' fluxes
-//              projected on the edge basis (eval_rhs, time_integrator.cu:
-//              26-101), times 1/J, and the RK stage update as epilogue:
-//              out = ca*u^n + cb*u_s + cc*dt*du/dt.
+//   element    the volume integral (eval_volume, :992-1083) -- solution and
+//              flux at the area points projected on the weighted basis
+//              gradients through the element metric -- plus a deterministic
+//              gather of the three faces' fluxes projected on the edge basis
+//              (eval_rhs, time_integrator.cu:26-101), times 1/J, and the RK
+//              stage update as epilogue: out = ca*u^n + cb*u_s + cc*dt*du/dt.
 //   k_limit    Barth-Jespersen limiter in place (limit_c, :640-720).
 //
-// SSP-RK3 steps skip k_trace after the first stage: k_element<TR=true>
-// writes the traces of its output as it stores it, so T always holds what
-// k_trace would have computed from the next stage's input.  With the limiter
-// on, the limiter runs on those traces: for Euler in the element kernel's own
-// epilogue (k_element<TR, LIM>, or the fixed-point stage of dg_fixed.cuh),
-// with the neighbours' new cell means found before the element stage by
-// k_means from the per-side flux sums k_face<FS> leaves; for the other
-// equations as the pass k_limit_tr.  Either way a limited element's traces
-// are rebuilt from its limited modes.
-//
 // FP64 is the binding resource on GB300 (the FP64 pipe runs at 1/62 of the
-// FP32 rate), so the design minimises FP64 instructions: every basis value
-// is a constant-bank operand (tables are __grid_constant__ parameters and
-// all loops are unrolled), each Riemann flux is evaluated once per side,
-// metric terms are folded into the flux before the projection (2 FMAs per
-// mode and point instead of 6), and the limiter needs two divisions per
-// variable instead of one per edge point.
+// FP32 rate), so the contractions of the element stage and the traces run on
+// the integer pipes in fixed point: k_element_fx and k_trace_fx (dg_fixed.cuh)
+// carry every equation and order.  k_element and k_trace here, one thread per
+// element in FP64, stay for the Euler equations at p >= 2 with the contraction
+// switch off and for the Euler batch at p >= 2 (Launch::fp64).  What is left on
+// the FP64 pipe uses few instructions: basis values are constant-bank operands
+// (tables are __grid_constant__ parameters, loops are unrolled), each Riemann
+// flux is evaluated once per side, with its reciprocals, square roots and
+// momentum sums on the integer pipes too, and metric terms are folded into
+// the flux before the projection.
+//
+// The element stage writes the traces of its output as it stores it, so T
+// always holds what k_trace would have computed from the next stage's input.
+// With the limiter on, the limiter runs on those traces: for Euler in the
+// element stage's own epilogue, with the neighbours' new cell means found
+// before it by k_means from the per-side flux sums k_face<FS> leaves; for the
+// other equations as the pass k_limit_tr.  Either way a limited element's
+// traces are rebuilt from its limited modes.
 #pragma once
 #include <algorithm>
 #include "dg_device.cuh"

@@ -38,7 +38,7 @@ __global__ void k_sqrt(const double *x, double *r, double *q, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     q[i] = __dsqrt_rn(x[i]);
-    r[i] = farther(dg::sqrt_pos(x[i]), dg::sqrt_fx(x[i]), q[i]);
+    r[i] = dg::sqrt_fx(x[i]);
   }
 }
 __global__ void k_physical(const double *U, int *fast, int *exact, int n) {
@@ -80,8 +80,7 @@ extern "C" dg_status dg_probe_physical(int device, int n, const double *U, int *
   return e == cudaSuccess ? DG_OK : dg::fail(DG_CUDA_ERROR, cudaGetErrorString(e));
 }
 
-// the sound speed's square root (dg::sqrt_pos and sqrt_fx, the one farther from
-// q) and IEEE sqrt on the device for n host values: q[i] = sqrt(x[i])
+// the sound speed's square root (dg::sqrt_fx) and IEEE sqrt on the device for n host values: q[i] = sqrt(x[i])
 extern "C" dg_status dg_probe_sqrt(int device, int n, const double *x, double *r, double *q) {
   if (n < 0 || (n && (!x || !r || !q))) return dg::fail(DG_BAD_ARG, "bad arguments");
   if (!n) return DG_OK;

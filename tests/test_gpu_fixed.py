@@ -56,6 +56,21 @@ def test_rows_at_the_ends_of_the_range(dglib, eq, p, k):
     assert relerr(np.ldexp(s.eval_rhs(np.ldexp(c, k), 0.0), -k), r, s.N) <= RHS_TOL
 
 
+@pytest.mark.parametrize("k", [-450, -260, 260, 450])
+def test_face_momenta_at_the_ends_of_the_range(dglib, k):
+    """The Euler flux is homogeneous of degree one: a state scaled by 2^k has
+    the right-hand side scaled by 2^k, with momenta whose products stay in
+    the range that the face kernel computes in fixed point (|k| = 260) and
+    with such as leave it (450), and states at rest among them."""
+    dg = dglib
+    _, s = problem(dg, dg.EULER, 1, 5, 4)
+    c = random_state(s, 5)
+    c[1:3, :, ::3] = 0
+    c[2, :, 1::3] = 0
+    r = s.eval_rhs(c, 0.0)
+    assert relerr(np.ldexp(s.eval_rhs(np.ldexp(c, k), 0.0), -k), r, s.N) <= RHS_TOL
+
+
 @pytest.mark.parametrize("eq", [0, 3])
 def test_zero_and_non_finite_rows(dglib, eq):
     """A zero state has a zero right-hand side; a NaN or an infinity in one
