@@ -41,12 +41,12 @@
 // Measured, Euler with the limiter, ms per launch (before: the contractions
 // as f16 digit slices on the tensor cores, 34 MMAs per 7 x 7 digit product on
 // 16 x 8 x 16 blocks of which half is padding): p = 3, 2.1M triangles 5.41 ->
-// 2.75.  The other equations (before: FP64 FMAs), microseconds at 131k triangles
+// 2.78.  The other equations (before: FP64 FMAs), microseconds at 131k triangles
 // (p = 4: 80k; advection 131k), p = 1 to 4: shallow water with a bed 92 -> 40,
 // 268 -> 80, 676 -> 182, 891 -> 223; Maxwell 71 -> 37, 205 -> 65, 527 -> 135, 710
 // -> 164; advection with a velocity field 35 -> 23, 86 -> 37, 206 -> 71, 371 ->
 // 113.  At p = 3 (ncu, 524k) the FP64 pipe -- fluxes, RK combination, limiter --
-// is 74 % busy and the heavy FMA pipe 54 %.
+// is 58 % busy, the heavy FMA pipe 65 % and the integer ALU 36 %.
 #pragma once
 #include "dg_kernels.cuh"
 namespace dg {
@@ -89,6 +89,11 @@ __device__ __forceinline__ double ratio(double a, double b) {
   if (__double_as_longlong(a) == 0) return 0.0;
   const unsigned eb = (unsigned)__double2hiint(b) >> 20;
   return eb - 2u < 2040u ? a * rcp(b) : a / b;
+}
+
+// a / b < c / d, for products out of range
+static __device__ __noinline__ bool smaller_quotient(double a, double b, double c, double d) {
+  return a / b < c / d;
 }
 
 // barrier of the block's N warps
@@ -191,8 +196,15 @@ __device__ __forceinline__ void traces_out(const FxTab<P> &tab, const EqP &q,
       if (above || below) {
         // alpha = min(lo / up, hi / dn) over the bounds passed: the smaller
         // quotient by cross products, then one division
-        const bool low = above && (!below || __double_as_longlong(lo * dn) <
-                                                 __double_as_longlong(hi * up));
+        bool low = above;
+        if (above && below) {
+          const double pl = lo * dn, ph = hi * up;
+          low = __double_as_longlong(pl) < __double_as_longlong(ph);
+          // the larger product zero, denormal or infinite: they do not tell
+          if ((unsigned)max(__double2hiint(pl), __double2hiint(ph)) - 0x00100000u >= 0x7FE00000u &&
+              (lob | hib) != 0)
+            low = smaller_quotient(lo, up, hi, dn);
+        }
         const double al = ratio(low ? lo : hi, low ? up : dn);
         const double c1 = c[1] * al, c2 = c[2] * al;
         if (live) {

@@ -91,3 +91,24 @@ def test_zero_and_non_finite_rows(dglib, eq):
         q = s.eval_rhs(d, 0.0)
         assert np.array_equal(q[:, :, far], r[:, :, far])
         assert not np.isfinite(q[:, 1:, e]).all()
+
+
+@pytest.mark.parametrize("p", [1, 3])
+@pytest.mark.parametrize("eq", [1, 3])
+def test_limiter_of_tiny_and_huge_states(dglib, eq, p):
+    """The limiter commutes with a scaling by 2^k, also where the products of
+    the bounds' distances that pick the smaller quotient leave the range."""
+    dg = dglib
+    mesh = dg.Mesh.square(6, 5, jitter=0.1, seed=2, bc=OPEN)
+    s = dg.Solver(mesh, eq, p, limiter=1)
+    c = random_state(s, 6, amp=0.2)
+
+    def limited(k):
+        s.set_state(np.ldexp(c, k))
+        s.limit_c()
+        return np.ldexp(s.get_state(), -k)
+
+    r = limited(0)
+    assert not np.array_equal(r, c)
+    for k in (-560, 600):
+        assert relerr(limited(k), r, s.N) <= RHS_TOL
