@@ -176,6 +176,15 @@ __device__ __forceinline__ bool physical_f32(const double *U) {
 }
 #endif
 
+// x, in a branch that is seldom taken: what is computed from it stays there (the
+// compiler computes both sides of a small branch and selects)
+DG_HD double rare(double x) {
+#ifdef __CUDA_ARCH__
+  asm volatile("" : "+d"(x));
+#endif
+  return x;
+}
+
 // 1/x and sqrt(x) on the integer pipes, for kernels that wait on the FP64 pipe
 // alone (the face kernels run it at 88 % with the integer pipes at 2 %): an FP64
 // operation occupies its pipe for 16 cycles of an SM, as long as 32 integer
@@ -192,7 +201,7 @@ DG_HD double rcp_fx(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const unsigned ax = hi & 0x7FFFFFFFu;
   const int ex = (int)(ax >> 20);
-  if ((unsigned)(ex - 1) > 2042u) return rcp(x);
+  if ((unsigned)(ex - 1) > 2042u) return rcp(rare(x));
   // |x| = X 2^(ex - 1075), f = X 2^-52 in [1, 2); R = r 2^24, r = 1/f to 22 bits
   const unsigned mh = (ax & 0xFFFFFu) | 0x100000u;
   float seed;
@@ -445,11 +454,12 @@ struct FluxMomentum {
       return;
     }
 #endif
-    mnl = fma(UL[1], sx, UL[2] * sy);
-    mnr = fma(UR[1], sx, UR[2] * sy);
+    const double l1 = rare(UL[1]), l2 = rare(UL[2]), r1 = rare(UR[1]), r2 = rare(UR[2]);
+    mnl = fma(l1, sx, l2 * sy);
+    mnr = fma(r1, sx, r2 * sy);
     if (SQ) {
-      hl = -0.5 * fma(UL[1], UL[1], UL[2] * UL[2]);
-      hr = -0.5 * fma(UR[1], UR[1], UR[2] * UR[2]);
+      hl = -0.5 * fma(l1, l1, l2 * l2);
+      hr = -0.5 * fma(r1, r1, r2 * r2);
     }
   }
   // a = UL[1] sl + UR[1] sr, b the same of entries 2
@@ -466,6 +476,8 @@ struct FluxMomentum {
       return;
     }
 #endif
+    sl = rare(sl);
+    sr = rare(sr);
     a = fma(UL[1], sl, UR[1] * sr);
     b = fma(UL[2], sl, UR[2] * sr);
   }
@@ -576,7 +588,7 @@ struct Euler {  // euler/euler.cu
     const double m2 = fma(U[1], U[1], U[2] * U[2]);
     // k = |m|^2/rho - 2E = -2 p / (gamma - 1): with k2 = (1 - gamma)/2, p = k2 k
     // enters through the products k2 ys, k2 xs, ... formed once per element
-    const double k2 = 0.5 * (1. - q.gamma), k = fma(m2, ir, -2.0 * U[3]);
+    const double k2 = q.k2, k = fma(m2, ir, -2.0 * U[3]);
     const double H = fma(k2, k, U[3]);
     g[0] = ma;
     g[1] = fma(U[1], ua, k * (k2 * ys));
@@ -602,9 +614,10 @@ struct Euler {  // euler/euler.cu
     m.begin<true>(UL, UR, sx, sy);
     const double irl = rcp_fx(UL[0]), irr = rcp_fx(UR[0]);
     const double snl = m.mnl * irl, snr = m.mnr * irr;
-    const double pl = mul_rn(q.gamma - 1., fma(m.hl, irl, UL[3]));
-    const double pr = mul_rn(q.gamma - 1., fma(m.hr, irr, UR[3]));
-    const double cl = sqrt_fx(q.gamma * pl * irl), cr = sqrt_fx(q.gamma * pr * irr);
+    const double pl = mul_rn(q.gm1, fma(m.hl, irl, UL[3]));
+    const double pr = mul_rn(q.gm1, fma(m.hr, irr, UR[3]));
+    const double cl = sqrt_fx(q.gamma * pl * irl);
+    const double cr = sqrt_fx(q.gamma * pr * irr);
     double a1, a2;
     m.advect(UL, UR, snl, snr, a1, a2);
     const double lam = larger(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
@@ -619,7 +632,7 @@ struct Euler {  // euler/euler.cu
     // (rcp_fx, sqrt_fx): the wave speed is the CFL step's to 1e-15
     const double ir = rcp_fx(U[0]);
     const double m2 = fma(U[1], U[1], U[2] * U[2]);
-    const double p = (q.gamma - 1.) * fma(-0.5 * m2, ir, U[3]);
+    const double p = q.gm1 * fma(-0.5 * m2, ir, U[3]);
     const double c = sqrt_fx(q.gamma * p * ir);
     const double s = sqrt_fx(m2) * ir;
     return s > 0 ? s + c : -s + c;
@@ -661,7 +674,7 @@ struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
   DG_HD static bool physical(const EqP &, const double *U) { return U[0] >= 0.; }
   DG_HD static void flux(const EqP &q, const double *U, double *fx, double *fy) {
     double ih = rcp(U[0]);
-    double u = U[1] * ih, v = U[2] * ih, hp = 0.5 * q.g * U[0] * U[0];
+    double u = U[1] * ih, v = U[2] * ih, hp = q.hg * U[0] * U[0];
     fx[0] = U[1];
     fx[1] = fma(U[1], u, hp);
     fx[2] = U[2] * u;
@@ -682,7 +695,7 @@ struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
     double a1, a2;
     m.advect(UL, UR, snl, snr, a1, a2);
     const double lam = larger(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
-    const double P = 0.5 * q.g * fma(UL[0], UL[0], UR[0] * UR[0]);
+    const double P = q.hg * fma(UL[0], UL[0], UR[0] * UR[0]);
     F[0] = fma(lam, UL[0] - UR[0], m.mnl + m.mnr);
     F[1] = fma(lam, UL[1] - UR[1], fma(P, sx, a1));
     F[2] = fma(lam, UL[2] - UR[2], fma(P, sy, a2));

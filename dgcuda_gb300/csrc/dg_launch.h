@@ -13,6 +13,7 @@ constexpr int kMaxSeries = 16;  // terms of an inflow pressure series
 struct EqP {
   double gamma, g, ax, ay, mu, eps;
   double imu, ieps, speed;  // Maxwell: 1/mu, 1/eps, 1/sqrt(eps mu)
+  double gm1, k2, hg;       // Euler: gamma - 1, (1 - gamma) / 2; shallow water: g / 2
   int problem;
   int field;        // 1: advection velocity a(x, y) = (ax, ay) + agrad (x, y)
   double prm[8];

@@ -500,6 +500,9 @@ extern "C" dg_status dg_solver_create(const dg_mesh *mesh, dg_equation eq, int p
   s->ops = ops_for(eq);
   s->q.gamma = P.gamma;
   s->q.g = P.gravity;
+  s->q.gm1 = P.gamma - 1.;
+  s->q.k2 = 0.5 * (1. - P.gamma);
+  s->q.hg = 0.5 * P.gravity;
   s->q.ax = P.ax;
   s->q.ay = P.ay;
   s->q.mu = P.mu;
