@@ -423,8 +423,8 @@ DG_HD void init_state(const EqP &q, double *U, double x, double y) {
 // advected momenta m_L s_L + m_R s_R.  On the device in fixed point
 // (dg_limbs.cuh), off the FP64 pipe, which the face kernels are bound by: 12 of
 // Euler's 46 FP64 operations a point, 8 of shallow water's 28 (k_face,
-// us: Euler p = 3, 2.1M triangles 1270 -> 1007, p = 1 627 -> 496; shallow water p =
-// 2, 131k 48.9 -> 41.8).  Errors against rational arithmetic, in units of 2^-53 of
+// us: Euler p = 3, 2.1M triangles 1270 -> 985, p = 1 627 -> 486; shallow water p =
+// 2, 131k 48.9 -> 40.5).  Errors against rational arithmetic, in units of 2^-53 of
 // the largest product: 1.5 (m . n; FP64 1.8), 1.2 (|m|^2; 1.9), 1.8 (advected
 // momenta; 2.0).
 // Where an exponent leaves the range (infinities, NaN, extreme states), and on
@@ -605,7 +605,7 @@ struct Euler {  // euler/euler.cu
                             double ny, double sc, double *F) {
     // every multiply-add is an explicit fma so the rounding does not depend
     // on how the compiler contracts the expression in a given kernel; the
-    // normal momenta m . n are the mass fluxes themselves.  34 FP64
+    // normal momenta m . n are the mass fluxes themselves.  30 FP64
     // operations, what k_face is bound by (67 with the scale applied to the
     // fluxes, products by -1/2, fmax, and with the reciprocals, square roots
     // and momentum sums on the FP64 pipe)

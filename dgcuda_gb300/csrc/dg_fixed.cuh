@@ -41,7 +41,7 @@
 // Measured, Euler with the limiter, ms per launch (before: the contractions
 // as f16 digit slices on the tensor cores, 34 MMAs per 7 x 7 digit product on
 // 16 x 8 x 16 blocks of which half is padding): p = 3, 2.1M triangles 5.41 ->
-// 2.78.  The other equations (before: FP64 FMAs), microseconds at 131k triangles
+// 2.72.  The other equations (before: FP64 FMAs), microseconds at 131k triangles
 // (p = 4: 80k; advection 131k), p = 1 to 4: shallow water with a bed 92 -> 40,
 // 268 -> 80, 676 -> 182, 891 -> 223; Maxwell 71 -> 37, 205 -> 65, 527 -> 135, 710
 // -> 164; advection with a velocity field 35 -> 23, 86 -> 37, 206 -> 71, 371 ->
