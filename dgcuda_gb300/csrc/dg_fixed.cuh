@@ -118,7 +118,7 @@ __device__ __forceinline__ bool block_or(bool b) {
 template <class Eq, int P, bool LIM, bool STORE = true>
 __device__ __forceinline__ void traces_out(const FxTab<P> &tab, const EqP &q,
                                            const double (&c)[Tab<P>::NP], double *out,
-                                           double *__restrict__ T, const int *__restrict__ nbr,
+                                           double *T, const int *__restrict__ nbr,
                                            const double *mean, size_t mstride, bool check, int K,
                                            int Kp, int e0, int lane, int n, double *st, int *flag) {
   using S = Shape<Eq, P>;
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(Shape<Eq, P>::kThreads, min_blocks<Eq, P>())
 // 3, 2.1M triangles, k_limit + k_trace_fx 2.89 + 0.44 ms -> 0.66.
 template <class Eq, int P, bool LIM, bool STORE>
 __device__ __forceinline__ void trace_tile(const FxTab<P> &tab, const EqP &q, double *u,
-                                           double *__restrict__ T, const int *__restrict__ nbr,
+                                           double *T, const int *__restrict__ nbr,
                                            int K, int Kp, int e0, double *st, int *flag) {
   constexpr int N = Eq::N, NP = Tab<P>::NP;
   const int lane = threadIdx.x & 31, n = N == 1 ? 0 : (int)(threadIdx.x >> 5);
@@ -582,7 +582,7 @@ __device__ __forceinline__ void trace_tile(const FxTab<P> &tab, const EqP &q, do
 template <class Eq, int P, bool LIM, bool STORE>
 __global__ void __launch_bounds__(Shape<Eq, P>::kThreads)
     k_trace_fx(const __grid_constant__ FxTab<P> tab, const __grid_constant__ EqP q, double *u,
-               double *__restrict__ T, const int *__restrict__ nbr, int K, int Kp) {
+               double *T, const int *__restrict__ nbr, int K, int Kp) {
   using S = Shape<Eq, P>;
   __shared__ double st[STORE ? S::NF * S::N * kPitch : 1];
   __shared__ int flag[kTile];

@@ -56,7 +56,10 @@ constexpr int kMaxBlock = 256;  // largest autotuned block of the stage kernels
 // the successor's launch.  Not earlier: blocks of a grid that does not fill
 // the GPU would all be placed on the SMs that drain first and wait there (a
 // trigger at the start made steps of 33k triangles 15-50 % slower).  Both are
-// no-ops in a launch without the attribute.
+// no-ops in a launch without the attribute.  A kernel launched this way lives
+// beside its predecessor's last stores, so what a step computes is not
+// read-only for its whole life, nor its own: no __ldg and no __restrict__ on it,
+// which let the compiler take loads across the wait; only on the mesh.
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
@@ -67,7 +70,7 @@ __device__ __forceinline__ void pdl_end() {
 // ---------------------------------------------------------------------------
 template <class Eq, int P>
 __device__ __forceinline__ void trace_body(const Tab<P> &tab, const EqP &q, double *u,
-                                           double *__restrict__ T, int Kp, int e) {
+                                           double *T, int Kp, int e) {
   constexpr int N = Eq::N, NP = Tab<P>::NP, N1 = Tab<P>::N1;
   double c[N][NP];
 #pragma unroll
@@ -108,7 +111,7 @@ __device__ __forceinline__ void trace_body(const Tab<P> &tab, const EqP &q, doub
 template <class Eq, int P>
 __global__ void __launch_bounds__(kMaxBlock) k_trace(const __grid_constant__ Tab<P> tab,
                                                      const __grid_constant__ EqP q, double *u,
-                                                     double *__restrict__ T, int K, int Kp) {
+                                                     double *T, int K, int Kp) {
   pdl_begin();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < K) trace_body<Eq, P>(tab, q, u, T, Kp, e);
@@ -128,22 +131,21 @@ struct FaceArgs {
 };
 
 // N contiguous doubles at p (16-byte aligned when N is even): 128-bit loads
-// and stores where N is even, scalar ones otherwise.  The loads are read-only
-// (__ldg), so that a loop's later ones need not wait for its earlier stores:
-// k_face's points are then all in flight (advection with a field, p = 3, 131k
-// triangles 38 -> 31 us, Maxwell p = 1 32 -> 23 us)
+// and stores where N is even, scalar ones otherwise.  Ordinary loads: what they
+// read (traces, flux sums) is still being written by the predecessor grid
+// when a dependent launch starts, which rules out read-only ones
 template <int N>
 __device__ __forceinline__ void load_vars(const double *p, double (&v)[N]) {
   if constexpr (N % 2 == 0) {
 #pragma unroll
     for (int k = 0; k < N / 2; k++) {
-      const double2 d = __ldg(reinterpret_cast<const double2 *>(p) + k);
+      const double2 d = reinterpret_cast<const double2 *>(p)[k];
       v[2 * k] = d.x;
       v[2 * k + 1] = d.y;
     }
   } else {
 #pragma unroll
-    for (int n = 0; n < N; n++) v[n] = __ldg(p + n);
+    for (int n = 0; n < N; n++) v[n] = p[n];
   }
 }
 template <int N>
@@ -322,7 +324,7 @@ __device__ __forceinline__ bool volume(const Tab<P> &tab, const EqP &q,
 
 template <class Eq, int P>
 __device__ __forceinline__ void limit_tr_body(const Tab<P> &tab, const EqP &q, double *u,
-                                              double *__restrict__ T,
+                                              double *T,
                                               const int *__restrict__ nbr, int Kp, int e,
                                               const double *mean, size_t mstride);
 
@@ -520,8 +522,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_bed_slopes(const __grid_constant_
 // mode 0, so the limiter's neighbour bounds see exactly the stored means.
 template <class Eq, int P>
 __device__ __forceinline__ void means_body(const Tab<P> &tab, const ElemArgs &a,
-                                           const double *__restrict__ Fs, double *__restrict__ M,
-                                           int e) {
+                                           const double *Fs, double *M, int e) {
   constexpr int N = Eq::N, NP = Tab<P>::NP;
   const size_t Kp = a.Kp;
   double sum[N];
@@ -540,11 +541,17 @@ __device__ __forceinline__ void means_body(const Tab<P> &tab, const ElemArgs &a,
   }
   const double sc = a.cc * *a.dtp * a.geo[4 * Kp + e] * tab.E[0][0][0];
   pdl_end();
+  double us[N], un[N];  // all read before the first store
 #pragma unroll
   for (int n = 0; n < N; n++) {
     const size_t o = (size_t)(n * NP) * Kp + e;
-    double v = fma(sc, sum[n], a.unit_cb ? a.us[o] : a.cb * a.us[o]);
-    if (a.has_un) v = fma(a.ca, a.un[o], v);
+    us[n] = a.us[o];
+    un[n] = a.has_un ? a.un[o] : 0.0;
+  }
+#pragma unroll
+  for (int n = 0; n < N; n++) {
+    double v = fma(sc, sum[n], a.unit_cb ? us[n] : a.cb * us[n]);
+    if (a.has_un) v = fma(a.ca, un[n], v);
     M[(size_t)n * Kp + e] = v;
   }
 }
@@ -552,8 +559,7 @@ __device__ __forceinline__ void means_body(const Tab<P> &tab, const ElemArgs &a,
 template <class Eq, int P>
 __global__ void __launch_bounds__(kMaxBlock) k_means(const __grid_constant__ Tab<P> tab,
                                                      const __grid_constant__ ElemArgs a,
-                                                     const double *__restrict__ Fs,
-                                                     double *__restrict__ M) {
+                                                     const double *Fs, double *M) {
   pdl_begin();
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e < a.K) means_body<Eq, P>(tab, a, Fs, M, e);
@@ -651,7 +657,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_limit(const __grid_constant__ Tab
 // mstride = Kp), when the neighbours' rows may not be written yet
 template <class Eq, int P>
 __device__ __forceinline__ void limit_tr_body(const Tab<P> &tab, const EqP &q, double *u,
-                                              double *__restrict__ T,
+                                              double *T,
                                               const int *__restrict__ nbr, int Kp, int e,
                                               const double *mean, size_t mstride) {
   constexpr int N = Eq::N, NP = Tab<P>::NP, N1 = Tab<P>::N1;
@@ -742,7 +748,7 @@ __device__ __forceinline__ void limit_tr_body(const Tab<P> &tab, const EqP &q, d
 template <class Eq, int P>
 __global__ void __launch_bounds__(kMaxBlock) k_limit_tr(const __grid_constant__ Tab<P> tab,
                                                         const __grid_constant__ EqP q,
-                                                        double *u, double *__restrict__ T,
+                                                        double *u, double *T,
                                                         const int *__restrict__ nbr, int K,
                                                         int Kp) {
   pdl_begin();
@@ -757,7 +763,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_limit_tr(const __grid_constant__ 
 // where a reset, a maximum, a time-step and an advance kernel cost four.
 template <class Eq, int P>
 __device__ __forceinline__ double cell_speed(const Tab<P> &tab, const EqP &q,
-                                             const double *__restrict__ u, DevScalars *ds, int Kp,
+                                             const double *u, DevScalars *ds, int Kp,
                                              int e) {
   constexpr int N = Eq::N, NP = Tab<P>::NP;
   double U[N];
@@ -807,8 +813,8 @@ constexpr int kLambdaBlocks = 608;
 template <class Eq, int P>
 __global__ void __launch_bounds__(kBlock) k_lambda(const __grid_constant__ Tab<P> tab,
                                                    const __grid_constant__ EqP q,
-                                                   const double *__restrict__ u, DevScalars *ds,
-                                                   int K, int Kp, int mode) {
+                                                   const double *u, DevScalars *ds, int K,
+                                                   int Kp, int mode) {
   pdl_begin();
   DevScalars d;
   if (threadIdx.x == 0) d = *ds;
