@@ -109,9 +109,10 @@ DG_HD double mul_rn(double a, double b) {
 #endif
 }
 
-// the larger of two wave speeds: a comparison and a select, where fmax is an
-// FP64 operation
-DG_HD double larger(double a, double b) { return b > a ? b : a; }
+// the larger of two wave speeds, a NaN on one side ignored as fmax ignores it (the
+// sound speed of an element whose mean is not physical): comparisons and a
+// select, where fmax is an FP64 operation
+DG_HD double larger(double a, double b) { return b > a || a != a ? b : a; }
 // 1/x for the flux evaluations, from the approximate reciprocal r of the PTX
 // instruction rcp.approx.ftz.f64 (about 20 correct bits) by one third-order
 // step of the Newton-Raphson family: with e = 1 - x r, 1/x = r / (1 - e) =
