@@ -424,56 +424,57 @@ DG_HD void init_state(const EqP &q, double *U, double x, double y) {
 // advected momenta m_L s_L + m_R s_R.  On the device in fixed point
 // (dg_limbs.cuh), off the FP64 pipe, which the face kernels are bound by: 12 of
 // Euler's 46 FP64 operations a point, 8 of shallow water's 28 (k_face,
-// us: Euler p = 3, 2.1M triangles 1270 -> 985, p = 1 627 -> 486; shallow water p =
-// 2, 131k 48.9 -> 40.5).  Errors against rational arithmetic, in units of 2^-53 of
-// the largest product: 1.5 (m . n; FP64 1.8), 1.2 (|m|^2; 1.9), 1.8 (advected
-// momenta; 2.0).
+// us: Euler p = 3, 2.1M triangles 1270 -> 1011, p = 1 627 -> 498; shallow water p =
+// 2, 131k 48.9 -> 41.8).  Every component has a row of its own: a small momentum
+// beside a large one keeps its bits.  Errors against 113-bit arithmetic, in units
+// of 2^-53 of the larger product (|m|^2: of the result), largest and RMS, at ratios
+// of the components from 1 to 0: m . n and the advected momenta 2.0, 0.47 (FP64 2.9,
+// 0.58; one component zero 1.0, 0.30, as FP64), |m|^2 1.0, 0.42 (1.9, 0.59; as FP64).
 // Where an exponent leaves the range (infinities, NaN, extreme states), and on
 // the host, in FP64.
 struct FluxMomentum {
   double mnl, mnr, hl, hr;  // m . (sx, sy) and -|m|^2 / 2, left and right
 #ifdef __CUDA_ARCH__
-  fx::Pair L, R;
+  fx::Num l1, l2, r1, r2;
   bool ok;
 #endif
   // SQ: |m|^2 is wanted
   template <bool SQ>
   DG_HD void begin(const double *UL, const double *UR, double sx, double sy) {
 #ifdef __CUDA_ARCH__
-    L = fx::make_pair(UL[1], UL[2]);
-    R = fx::make_pair(UR[1], UR[2]);
-    const fx::Pair n = fx::make_pair(sx, sy);
-    ok = fx::in_range(L.r, n.r) && fx::in_range(R.r, n.r) &&
-         (!SQ || (fx::in_range(L.r, L.r) && fx::in_range(R.r, R.r)));
+    l1 = fx::make_num(UL[1]);
+    l2 = fx::make_num(UL[2]);
+    r1 = fx::make_num(UR[1]);
+    r2 = fx::make_num(UR[2]);
+    const fx::Num nx = fx::make_num(sx), ny = fx::make_num(sy);
+    ok = fx::in_range(min(min(min(l1.m, l2.m), min(r1.m, r2.m)), min(nx.m, ny.m)),
+                      max(max(max(l1.m, l2.m), max(r1.m, r2.m)), max(nx.m, ny.m)));
     if (ok) {
-      mnl = fx::dot(L, n);
-      mnr = fx::dot(R, n);
+      mnl = fx::dot(l1, nx, l2, ny);
+      mnr = fx::dot(r1, nx, r2, ny);
       if (SQ) {
-        hl = fx::neg_half_square(L);
-        hr = fx::neg_half_square(R);
+        hl = fx::neg_half_square(l1, l2);
+        hr = fx::neg_half_square(r1, r2);
       }
       return;
     }
 #endif
-    const double l1 = rare(UL[1]), l2 = rare(UL[2]), r1 = rare(UR[1]), r2 = rare(UR[2]);
-    mnl = fma(l1, sx, l2 * sy);
-    mnr = fma(r1, sx, r2 * sy);
+    const double a1 = rare(UL[1]), a2 = rare(UL[2]), b1 = rare(UR[1]), b2 = rare(UR[2]);
+    mnl = fma(a1, sx, a2 * sy);
+    mnr = fma(b1, sx, b2 * sy);
     if (SQ) {
-      hl = -0.5 * fma(l1, l1, l2 * l2);
-      hr = -0.5 * fma(r1, r1, r2 * r2);
+      hl = -0.5 * fma(a1, a1, a2 * a2);
+      hr = -0.5 * fma(b1, b1, b2 * b2);
     }
   }
   // a = UL[1] sl + UR[1] sr, b the same of entries 2
   DG_HD void advect(const double *UL, const double *UR, double sl, double sr, double &a,
                     double &b) const {
 #ifdef __CUDA_ARCH__
-    const fx::Row rl = fx::make_row(fx::abs_hi(sl)), rr = fx::make_row(fx::abs_hi(sr));
-    if (ok && fx::in_range(L.r, rl) && fx::in_range(R.r, rr)) {
-      fx::Limb l, r;
-      fx::to_limbs(sl, rl, l.h, l.l);
-      fx::to_limbs(sr, rr, r.h, r.l);
-      a = fx::sum2(L.a, L.r.m, l, rl.m, R.a, R.r.m, r, rr.m);
-      b = fx::sum2(L.b, L.r.m, l, rl.m, R.b, R.r.m, r, rr.m);
+    const fx::Num l = fx::make_num(sl), r = fx::make_num(sr);
+    if (ok && fx::in_range(min(l.m, r.m), max(l.m, r.m))) {
+      a = fx::dot(l1, l, r1, r);
+      b = fx::dot(l2, l, r2, r);
       return;
     }
 #endif

@@ -91,66 +91,65 @@ __device__ __forceinline__ double finish(const Sum &s, int base) {
 }
 
 // ---- sums of two products of variables (face kernels) -----------------------
-// two doubles on one row
-struct Pair {
-  Row r;
-  Limb a, b;
+// a double on a row of its own, so that it keeps all its bits beside a much
+// larger one: x = (h 2^28 + l) 2^(m - 1078), t the upper half of l.  m: 1023 for a
+// zero, 0 for a denormal, which in_range() then leaves to FP64
+struct Num {
+  int m, h, l, t;
 };
-__device__ __forceinline__ Pair make_pair(double a, double b) {
-  Pair p;
-  p.r = make_row(max(abs_hi(a), abs_hi(b)));
-  to_limbs(a, p.r, p.a.h, p.a.l);
-  to_limbs(b, p.r, p.b.h, p.b.l);
-  return p;
+__device__ __forceinline__ Num make_num(double x) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const unsigned mh = ((unsigned)hi & 0xFFFFFu) | 0x100000u;
+  const int sg = (hi >> 31) | 1;
+  Num n;
+  n.m = (hi >> 20) & 0x7FF;
+  n.h = (int)((mh << 7) | (lo >> 25)) * sg;
+  n.l = (int)((lo << 3) & ((1u << kLow) - 1)) * sg;
+  if (n.m == 0) {
+    n.h = n.l = 0;
+    if (((hi & 0x7FFFFFFF) | (int)lo) == 0) n.m = 1023;
+  }
+  n.t = n.l >> (kLow / 2);
+  return n;
 }
-// whether products of rows x and y stay in the normal range (rows of infinities
-// and NaN are odd)
-__device__ __forceinline__ bool in_range(Row x, Row y) {
-  return !x.odd() && !y.odd() && (unsigned)(x.m + y.m - 1200) < 1700u;
+// whether the products of numbers with exponents in [lo, hi] stay in the normal
+// range, and the sums of two of them (an infinity or a NaN has 2047)
+__device__ __forceinline__ bool in_range(int lo, int hi) { return lo >= 620 && hi < 1400; }
+// x y in units of 2^(x.m + y.m - 2156 + 51), below 2^61
+__device__ __forceinline__ long long prod(const Num &x, const Num &y) {
+  long long M = 1ll << 22;
+  M += (long long)x.h * y.l;
+  M += (long long)x.l * y.h;
+  M += (long long)x.t * y.t;  // l l' >> 28
+  return ((long long)x.h * y.h << 5) + (M >> (kLow - 5));
 }
-// x.a y.a + x.b y.b
-__device__ __forceinline__ double dot(const Pair &x, const Pair &y) {
-  Sum s;
-  zero(s);
-  mac(s, x.a.h, x.a.l, y.a);
-  mac(s, x.b.h, x.b.l, y.b);
-  return finish(s, base_exp(x.r, y.r.m));
+__device__ __forceinline__ long long square(const Num &x) {
+  long long M = 1ll << 22;
+  M += (long long)x.h * (2 * x.l);
+  M += (long long)x.t * x.t;
+  return ((long long)x.h * x.h << 5) + (M >> (kLow - 5));
 }
-// -(x.a^2 + x.b^2) / 2.  The low limbs' squares, which mac() leaves out, all have
-// one sign: without them the error reached 2.0 units of 2^-53 of the result,
-// with them 1.2 (FP64 1.9)
-__device__ __forceinline__ double neg_half_square(const Pair &x) {
-  Sum s;
-  zero(s);
-  long long low = (long long)x.a.l * x.a.l;
-  low += (long long)x.b.l * x.b.l;
-  s.H += (long long)x.a.h * x.a.h;
-  s.H += (long long)x.b.h * x.b.h;
-  s.M += (long long)x.a.h * (2 * x.a.l);
-  s.M += (long long)x.b.h * (2 * x.b.l);
-  s.M += low >> kLow;
-  const double v = finish(s, base_exp(x.r, x.r.m) - 1);
-  return __hiloint2double(__double2hiint(v) ^ (int)0x80000000, __double2loint(v));
-}
-// xa ya + xb yb, the two products on rows of their own: the smaller scale is
-// shifted to the larger one (a zero product, whose rows may be stand-ins for
-// rows of zeros, takes the other's)
-__device__ __forceinline__ double sum2(const Limb &xa, int xm, const Limb &ya, int ym,
-                                       const Limb &xb, int um, const Limb &yb, int vm) {
-  Sum p, q;
-  zero(p);
-  zero(q);
-  mac(p, xa.h, xa.l, ya);
-  mac(q, xb.h, xb.l, yb);
-  const long long P = p.H + (p.M >> kLow), Q = q.H + (q.M >> kLow);
-  int ep = xm + ym, eq = um + vm;
-  if (P == 0) ep = eq;
-  if (Q == 0) eq = ep;
+// the sum of the products p and q, whose numbers' exponents add up to ep and eq,
+// times 2^k: the smaller scale is shifted to the larger one (a zero product,
+// whose exponents may be stand-ins, takes the other's)
+__device__ __forceinline__ double sum2(long long p, int ep, long long q, int eq, int k = 0) {
+  if (p == 0) ep = eq;
+  if (q == 0) eq = ep;
   const int d = ep - eq;
   Sum s;
-  s.H = d >= 0 ? P + (Q >> min(d, 63)) : Q + (P >> min(-d, 63));
+  s.H = d >= 0 ? p + (q >> min(d, 63)) : q + (p >> min(-d, 63));
   s.M = 0;
-  return finish(s, max(ep, eq) - 1015);
+  return finish(s, max(ep, eq) - 1020 + k);
+}
+// xa ya + xb yb
+__device__ __forceinline__ double dot(const Num &xa, const Num &ya, const Num &xb, const Num &yb) {
+  return sum2(prod(xa, ya), xa.m + ya.m, prod(xb, yb), xb.m + yb.m);
+}
+// -(a^2 + b^2) / 2
+__device__ __forceinline__ double neg_half_square(const Num &a, const Num &b) {
+  const double v = sum2(square(a), 2 * a.m, square(b), 2 * b.m, -1);
+  return __hiloint2double(__double2hiint(v) ^ (int)0x80000000, __double2loint(v));
 }
 
 }  // namespace fx

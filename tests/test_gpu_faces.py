@@ -1,5 +1,6 @@
 """The numerical fluxes of the face kernels where one state is far from the
-other: a wave speed that is not a number on one side only."""
+other: a wave speed that is not a number on one side only, and small
+components beside large ones."""
 import numpy as np
 import pytest
 
@@ -44,3 +45,21 @@ def test_a_sound_speed_that_is_not_a_number_gives_way_to_the_other_sides(dglib, 
                 lefts += 1
                 assert relerr(r[:, :, k], ref, s.N) <= RHS_TOL
     assert lefts > 0
+
+
+@pytest.mark.parametrize("var", [1, 2])
+@pytest.mark.parametrize("r", [1e-3, 1e-9, 1e-15])
+def test_a_small_momentum_beside_a_large_one_keeps_its_bits(dglib, oracle_mod, var, r):
+    """Flow along one axis (shallow water with next to no gravity): the
+    small component's right-hand side, all of whose terms are as small, to
+    the parity bound of its own norm."""
+    dg = dglib
+    mesh = dg.Mesh.square(6, 5, jitter=0.1, seed=4, bc=OPEN)
+    s = dg.Solver(mesh, dg.SHALLOW_WATER, 2, gravity=1e-40)
+    rng = np.random.default_rng(3)
+    c = uniform(s, (1.0, 1.0, 1.0))
+    c[:, 0, :] *= 1 + 0.2 * rng.standard_normal((3, s.K))
+    c[:, 1:, :] = 0.02 * rng.standard_normal((3, s.n_p - 1, s.K))
+    c[var] *= r
+    o = oracle_mod.Oracle.from_mesh(mesh, dg.SHALLOW_WATER, 2, oracle_mod.prm_vec(g=1e-40), 0)
+    assert relerr(s.eval_rhs(c, 0.0), o.rhs(c, 0.0), 3) <= RHS_TOL
