@@ -109,10 +109,11 @@ DG_HD double mul_rn(double a, double b) {
 #endif
 }
 
-// the larger of two wave speeds, a NaN on one side ignored as fmax ignores it (the
-// sound speed of an element whose mean is not physical): comparisons and a
-// select, where fmax is an FP64 operation
-DG_HD double larger(double a, double b) { return b > a || a != a ? b : a; }
+// the larger of two wave speeds, by comparisons and a select, where fmax is an FP64
+// operation: of two numbers, and with a NaN on one side ignored as fmax ignores
+// it (the sound speed of an element whose mean is not physical)
+DG_HD double larger(double a, double b) { return b > a ? b : a; }
+DG_HD double larger_number(double a, double b) { return b > a || a != a ? b : a; }
 // 1/x for the flux evaluations, from the approximate reciprocal r of the PTX
 // instruction rcp.approx.ftz.f64 (about 20 correct bits) by one third-order
 // step of the Newton-Raphson family: with e = 1 - x r, 1/x = r / (1 - e) =
@@ -622,7 +623,7 @@ struct Euler {  // euler/euler.cu
     const double cr = sqrt_fx(q.gamma * pr * irr);
     double a1, a2;
     m.advect(UL, UR, snl, snr, a1, a2);
-    const double lam = larger(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
+    const double lam = larger_number(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
     const double P = pl + pr;
     F[0] = fma(lam, UL[0] - UR[0], m.mnl + m.mnr);
     F[1] = fma(lam, UL[1] - UR[1], fma(P, sx, a1));
@@ -696,7 +697,7 @@ struct ShallowWater {  // shallowwater/shallowwater.cu (g is a parameter here)
     const double cl = sqrt_fx(UL[0] * q.g), cr = sqrt_fx(UR[0] * q.g);
     double a1, a2;
     m.advect(UL, UR, snl, snr, a1, a2);
-    const double lam = larger(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
+    const double lam = larger_number(fma(cl, sc, fabs(snl)), fma(cr, sc, fabs(snr)));
     const double P = q.hg * fma(UL[0], UL[0], UR[0] * UR[0]);
     F[0] = fma(lam, UL[0] - UR[0], m.mnl + m.mnr);
     F[1] = fma(lam, UL[1] - UR[1], fma(P, sx, a1));
