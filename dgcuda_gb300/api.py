@@ -116,6 +116,7 @@ def _declare(L):
         "dg_eval_vertices_view": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_double, _dp]),
         "dg_save_checkpoint": (C.c_int, [C.c_void_p, C.c_char_p, C.c_double]),
         "dg_set_tensor_contractions": (C.c_int, [C.c_void_p, C.c_int]),
+        "dg_fx_table_image": (C.c_int, [C.c_int, C.c_void_p, C.c_size_t]),
         "dg_oz_table_image": (C.c_int, [C.c_int, C.c_void_p, C.c_size_t, _dp]),
         "dg_get_tensor_contractions": (C.c_int, [C.c_void_p, _ip]),
         "dg_load_checkpoint": (C.c_int, [C.c_void_p, C.c_char_p, _dp]),
@@ -305,6 +306,26 @@ def oz_table_image(p):
     _check(L.dg_oz_table_image(p, buf.ctypes.data_as(C.c_void_p), buf.nbytes, _dptr(dense)))
     return (buf[:4480].reshape(2240, 2).copy(),
             buf[4480:4528].view(np.int32).reshape(3, 16).copy(), dense)
+
+
+def fx_table_image(p):
+    """The element stage's limb tables of order p (host-built; no GPU needed):
+    int arrays T = h 2^28 + l named B[nq, np], G[nq, 2, np], S[nf, np],
+    Q[nq, np], E[nf, np], and the biased exponents eB (B), eP (G, S, Q) and
+    eE (E) of their units 2^(M - 1078)."""
+    L = load_library()
+    buf = np.zeros(4096, dtype=np.int32)
+    _check(L.dg_fx_table_image(p, buf.ctypes.data_as(C.c_void_p), buf.nbytes))
+    nm, nq, nf = (p + 1) * (p + 2) // 2, (0, 3, 6, 12, 16)[p], 3 * (p + 1)
+    out, o = {}, 0
+    for name, shape in (("B", (nq, nm)), ("G", (nq, 2, nm)), ("S", (nf, nm)), ("Q", (nq, nm)),
+                        ("E", (nf, nm))):
+        n = 2 * int(np.prod(shape))
+        limbs = buf[o:o + n].astype(np.int64).reshape(shape + (2,))
+        out[name] = (limbs[..., 0] << 28) + limbs[..., 1]
+        o += n
+    out["eB"], out["eP"], out["eE"] = (int(v) for v in buf[o:o + 3])
+    return out
 
 
 def measure_fp64_peak(device=0):

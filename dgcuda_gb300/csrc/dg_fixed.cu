@@ -1,9 +1,12 @@
 // dg_fixed.cu -- host side of the fixed-point contractions: the limb tables
 // of the element stage's basis tables.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <vector>
 
 #include "dg_fixed.cuh"
+#include "dg_internal.h"
 
 namespace dg {
 namespace fx {
@@ -15,8 +18,8 @@ int host_bexp(double x) {
   return (int)((b >> 52) & 0x7FF);
 }
 
-// t in units of 2^(M - 1078), M the table's largest biased exponent: a
-// signed integer below 2^56, as h 2^28 + l with l in [-2^27, 2^27)
+// t in units of 2^(M - 1078): a signed integer, |T| <= 2^58, as h 2^28 + l with l
+// in [-2^27, 2^27)
 Limb limb(double t, int M) {
   const long long T = std::llrint(std::ldexp(t, 1078 - M));
   Limb r;
@@ -25,19 +28,53 @@ Limb limb(double t, int M) {
   return r;
 }
 
+// The unit of the projection's tables, 2^(M - 1078): the smallest with every |T|
+// <= 2^58 and the |T| that meet in one sum adding up to 2^61 at most, so that sums of
+// at most 63 products with inputs below 2^56 stay in 64 bits.  For the library's
+// tables two bits below the largest entry's exponent, the unit of the other
+// tables: the product that the sums leave out, l tl, is what their error was made
+// of (the header of dg_fixed.cuh has the figures).
+struct Unit {
+  double top = 0, sum = 0;  // the largest |t|, the largest sum of |t|
+  template <class... D>
+  void add(D... t) {
+    ((top = std::max(top, std::fabs(t)), part += std::fabs(t)), ...);
+  }
+  void end() {
+    sum = std::max(sum, part);
+    part = 0;
+  }
+  int exponent() const {
+    int k = 0;
+    if (sum > 0) std::frexp(sum, &k);  // sum <= 2^k
+    return std::max(1, std::max(host_bexp(top) - 2, k + 1017));
+  }
+
+ private:
+  double part = 0;
+};
+
 template <int P>
 void build(const Tab<P> &t, FxTab<P> *o) {
   constexpr int NP = Tab<P>::NP, NQ = Tab<P>::NQ, N1 = Tab<P>::N1, NF = 3 * N1;
-  int mB = 1, mG = 1, mE = 1;
+  int mB = 1, mE = 1;
   for (int q = 0; q < NQ; q++)
-    for (int i = 0; i < NP; i++) {
-      mB = std::max(mB, host_bexp(t.B[q][i]));
-      mG = std::max(mG, std::max(host_bexp(t.GR[q][i]), host_bexp(t.GS[q][i])));
-    }
+    for (int i = 0; i < NP; i++) mB = std::max(mB, host_bexp(t.B[q][i]));
   for (int k = 0; k < NF; k++)
     for (int i = 0; i < NP; i++) mE = std::max(mE, host_bexp(t.E[k / N1][k % N1][i]));
+  Unit u;
+  for (int i = 0; i < NP; i++, u.end()) {  // to the modes: edge points, slopes, a bed
+    for (int k = 0; k < NF; k++) u.add(t.E[k / N1][k % N1][i]);
+    for (int q = 0; q < NQ; q++) u.add(t.GR[q][i], t.GS[q][i], t.B[q][i]);
+  }
+  for (int q = 0; q < NQ; q++) {  // the adjoint's projections on the slopes
+    for (int i = 0; i < NP; i++) u.add(t.GR[q][i]);
+    u.end();
+    for (int i = 0; i < NP; i++) u.add(t.GS[q][i]);
+    u.end();
+  }
   o->eB = mB;
-  o->eP = std::max(mB, std::max(mG, mE));
+  o->eP = u.exponent();
   o->eE = mE;
   o->c0 = 1;
   for (int q = 1; q < NQ; q++)
@@ -87,3 +124,14 @@ void build_fx_tab(int p, const void *tabimg, void *out) {
 }
 
 }  // namespace dg
+
+// the limb tables of order p (1..4) built from the library's basis tables, as
+// fx::FxTab<p> holds them
+extern "C" dg_status dg_fx_table_image(int p, void *out, size_t bytes) {
+  if (p < 1 || p > 4 || !out) return dg::fail(DG_BAD_ARG, "order must be 1..4");
+  if (bytes < dg::fx_tab_bytes(p)) return dg::fail(DG_BAD_ARG, "buffer too small");
+  std::vector<char> tab(dg::tab_bytes(p));
+  dg::build_tab(p, DG_TABLES[p], tab.data());
+  dg::build_fx_tab(p, tab.data(), out);
+  return DG_OK;
+}

@@ -240,6 +240,13 @@ dg_status dg_set_tensor_contractions(dg_solver *s, int on);
  * tables that were split, as [K block][K slot][N slot] matrices (EVAL,
  * PROJ x 3, TRACE) */
 dg_status dg_oz_table_image(int p, void *out, size_t bytes, double *dense);
+/* the basis tables of order p = 1..4 as the element stage's two-limb integers
+ * T = h 2^28 + l (int h, l), built on the host from the library's basis tables
+ * (for checks; no GPU needed): with np modes, nq area points and nf = 3 (p + 1)
+ * edge points B[nq][np], G[nq][2][np], S[nf][np], Q[nq][np], E[nf][np], then the
+ * biased exponents M of the units 2^(M - 1078): int eB (B), eP (G, S, Q), eE (E).
+ * bytes >= 16384 */
+dg_status dg_fx_table_image(int p, void *out, size_t bytes);
 dg_status dg_get_tensor_contractions(dg_solver *s, int *on);
 
 /* binary checkpoint / restart (no reference counterpart: the reference's
