@@ -182,6 +182,19 @@ __device__ __forceinline__ void traces_out(const FxTab<P> &tab, const EqP &q,
           kmin = min(kmin, kk);
         }
       }
+      if (LIM && row.m == 0x7FF) {
+        // as FP64 traces have it: a NaN limits nothing and stays, infinities beside
+        // a finite mean are overshoots like any other
+        bool inf = live;
+#pragma unroll 1
+        for (int i = 0; i < NP && live; i++) {
+          const double v = outn[(size_t)i * Kp];
+          inf &= i == 0 ? abs_hi(v) < 0x7FF00000 : v == v;
+        }
+        const double top = __hiloint2double(inf ? 0x7FF00000 : (int)0xFFF00000, 0);
+        kmax = order_key(top);
+        kmin = order_key(-top);
+      }
     }
     if constexpr (LIM) {
       // products reused as addends are rounded explicitly, as in limit_tr_body

@@ -20,7 +20,10 @@ struct Limb {
 // denormals only) takes an exponent that shifts every entry out: all its
 // limbs and sums are zero.  Other rows outside [100, 1900], where a result
 // could leave the normal range, and rows with an infinity or a NaN are
-// odd(): finish() forms their sums as if m were 1023 and fix() scales them
+// odd(): finish() forms their sums as if m were 1023 and fix() scales them, to NaN
+// in the latter.  Below 2^-967 a zero or a denormal counts as 2^-1023: an error
+// under the smallest normal number, which lifting such rows first would take away
+// at 2 to 9 % of the element stage's time
 struct Row {
   int m;
   __device__ __forceinline__ bool odd() const { return (unsigned)(m - 100) > 1800u; }
