@@ -84,15 +84,7 @@ struct Shape {
   static constexpr int kThreads = 32 * N;
 };
 
-// a / b for 0 <= a < b (the limiter's quotients) within 2 ulp of IEEE
-// division; a = 0 without dividing, and b outside rcp()'s range divided
-__device__ __forceinline__ double ratio(double a, double b) {
-  if (__double_as_longlong(a) == 0) return 0.0;
-  const unsigned eb = (unsigned)__double2hiint(b) >> 20;
-  return eb - 2u < 2040u ? a * rcp(b) : a / b;
-}
-
-// a / b < c / d, for products out of range
+// a / b < c / d, where the cross products do not tell
 static __device__ __noinline__ bool smaller_quotient(double a, double b, double c, double d) {
   return a / b < c / d;
 }
@@ -208,18 +200,23 @@ __device__ __forceinline__ void traces_out(const FxTab<P> &tab, const EqP &q,
       const long long lob = __double_as_longlong(lo), hib = __double_as_longlong(hi);
       const bool above = __double_as_longlong(up) > lob, below = __double_as_longlong(dn) > hib;
       if (above || below) {
-        // alpha = min(lo / up, hi / dn) over the bounds passed: the smaller
-        // quotient by cross products, then one division
+        // alpha = min(lo / up, hi / dn) over the bounds passed, as IEEE division
+        // rounds it: the smaller quotient by cross products, then one division
         bool low = above;
         if (above && below) {
           const double pl = lo * dn, ph = hi * up;
-          low = __double_as_longlong(pl) < __double_as_longlong(ph);
-          // the larger product zero, denormal or infinite: they do not tell
-          if ((unsigned)max(__double2hiint(pl), __double2hiint(ph)) - 0x00100000u >= 0x7FE00000u &&
+          const long long d = __double_as_longlong(pl) - __double_as_longlong(ph);
+          low = d < 0;
+          // within a few units of rounding of each other, or the larger one zero,
+          // denormal or infinite: they do not tell
+          if (((unsigned long long)(d + 8) <= 16ull ||
+               (unsigned)max(__double2hiint(pl), __double2hiint(ph)) - 0x00100000u >= 0x7FE00000u) &&
               (lob | hib) != 0)
             low = smaller_quotient(lo, up, hi, dn);
         }
-        const double al = ratio(low ? lo : hi, low ? up : dn);
+        // (a collapsed bound, +0 on its bits, without dividing)
+        const double num = low ? lo : hi;
+        const double al = __double_as_longlong(num) == 0 ? 0.0 : num / (low ? up : dn);
         const double c1 = c[1] * al, c2 = c[2] * al;
         if (live) {
           outn[(size_t)Kp] = c1;

@@ -1,6 +1,8 @@
-"""The limiter on states with infinities and NaN."""
+"""The limiter: its quotients, and states with infinities and NaN."""
 import numpy as np
 import pytest
+
+from conftest import ref_tables, split_tables
 
 pytestmark = pytest.mark.gpu
 OPEN = (-4, -4, -4, -4)
@@ -52,3 +54,42 @@ def test_an_infinity_is_an_overshoot_like_any_other(dglib, eq, p):
     s.set_state(d)
     s.limit_c()
     assert np.array_equal(s.get_state(), c)
+
+
+@pytest.mark.parametrize("eq", [0, 1, 2, 3])
+def test_alpha_is_the_smaller_ieee_quotient(dglib, eq):
+    """Tables and states of a few bits, so that traces, bounds and overshoots
+    are exact: the limited slopes are those of IEEE division and
+    multiplication, bit for bit."""
+    dg = dglib
+    mesh = dg.Mesh.square(12, 11, jitter=0.1, seed=2)
+    s = dg.Solver(mesh, eq, 1, limiter=1)
+    tab = [t.copy() for t in split_tables(ref_tables(1), 1)]
+    tab[0][:3] = 1.0  # phi_0 = 1 at the area points
+    E = np.array([[[1.0, 0.5, -0.25], [1.0, 0.25, 1.0]], [[1.0, -0.5, 0.25], [1.0, -1.0, 0.5]],
+                  [[1.0, 0.125, -1.0], [1.0, -0.25, -0.5]]])  # [face][point][mode]
+    tab[3][:] = E.transpose(0, 2, 1).ravel()
+    s.set_tables(*tab)
+    if eq == dg.EULER:
+        s.tensor_contractions = True
+    rng = np.random.default_rng(eq)
+    c = np.round(rng.uniform(-1, 1, s.shape) * 2.0 ** 20) / 2.0 ** 20
+    c[:, 0] *= 0.25
+    s.set_state(c)
+    s.limit_c()
+    _, es, _, se = mesh.arrays()
+    nb = np.array([[se[1, sd] if se[0, sd] == e else se[0, sd] for sd in es[:, e]]
+                   for e in range(s.K)])
+    ref, limited = c.copy(), 0
+    for n in range(s.N):
+        for e in range(s.K):
+            m = c[n, 0, [e] + list(nb[e])]
+            T = np.einsum("fji,i->fj", E, c[n, :, e])
+            up, dn = T.max() - m[0], m[0] - T.min()
+            lo, hi = m[0] - m.min(), m.max() - m[0]
+            al = min(lo / up if up > lo else 1.0, hi / dn if dn > hi else 1.0)
+            if al < 1:
+                limited += 1
+                ref[n, 1:, e] *= al
+    assert limited > s.N * s.K // 2
+    assert np.array_equal(s.get_state(), ref)
