@@ -98,7 +98,6 @@ void build(const Tab<P> &t, FxTab<P> *o) {
     }
   }
   o->phi0 = t.B[0][0];
-  o->e0 = t.E[0][0][0];
 }
 
 }  // namespace

@@ -68,7 +68,7 @@ struct FxTab {
   int eB, eP, eE;                        // biased exponents of eval, projection, traces
   int c0;                                // phi_0 has one value at all area points (on the edges it has)
   double r[NQ], s[NQ], B0[NQ];           // area points, phi_0 there
-  double phi0, e0;                       // phi_0 (area point 0), phi_0 on the edges
+  double phi0;                           // phi_0 (area point 0)
 };
 
 // ---- shared memory of a block ----------------------------------------------
@@ -87,6 +87,19 @@ struct Shape {
 // a / b < c / d, where the cross products do not tell
 static __device__ __noinline__ bool smaller_quotient(double a, double b, double c, double d) {
   return a / b < c / d;
+}
+
+// the trace of an element that has its mean alone, as the contraction rounds it
+static __device__ __noinline__ double mean_trace(double c0, Limb E0, int eE) {
+  const Row row = make_row(abs_hi(c0));
+  int h, l;
+  to_limbs(c0, row, h, l);
+  Sum s;
+  zero(s);
+  mac(s, h, l, E0);
+  double v = finish(s, base_exp(row, eE));
+  if (row.odd()) fix(&v, 1, 1, row);
+  return v;
 }
 
 // barrier of the block's N warps
@@ -262,7 +275,7 @@ __device__ __forceinline__ void traces_out(const FxTab<P> &tab, const EqP &q,
       if (bad) flag[lane] = 1;
       block_sync<N>();
       if (flag[lane]) {  // flatten: higher modes to zero, traces to the mean
-        const double a0 = c[0] * tab.e0;
+        const double a0 = mean_trace(c[0], tab.E[0][0], tab.eE);
 #pragma unroll 1
         for (int k = 0; k < NF; k++) st[(k * N + n) * kPitch + lane] = a0;
         if (live)
