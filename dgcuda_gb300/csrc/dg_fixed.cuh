@@ -641,11 +641,12 @@ __global__ void __launch_bounds__(Shape<Eq, P>::kThreads, min_blocks<Eq, P>())
   element_tile<Eq, P, MODE>(tab, pr.q, a, e0, st, mxs, flag);
 }
 
-template <class Eq, int P>
+// the traces of the states U, and with LIM the limiter of a stage's output first
+template <class Eq, int P, bool LIM>
 __global__ void __launch_bounds__(Shape<Eq, P>::kThreads)
     k_trace_batch_fx(const __grid_constant__ FxTab<P> tab, const BatchProb *__restrict__ probs,
                      const int *__restrict__ blk2prob, const int *__restrict__ blk0, int b_lo,
-                     int sub) {
+                     int sub, int stage) {
   using S = Shape<Eq, P>;
   __shared__ double st[S::NF * S::N * kPitch];
   __shared__ int flag[kTile];
@@ -653,7 +654,8 @@ __global__ void __launch_bounds__(Shape<Eq, P>::kThreads)
   const int e0 = batch_tile(blk2prob, blk0, b_lo, sub, pi);
   const BatchProb &pr = probs[pi];
   if (e0 >= pr.K) return;
-  trace_tile<Eq, P, false, true>(tab, pr.q, pr.U, pr.T, nullptr, pr.K, pr.Kp, e0, st, flag);
+  trace_tile<Eq, P, LIM, true>(tab, pr.q, LIM && stage < 2 ? pr.W : pr.U, pr.T, pr.nbr, pr.K,
+                               pr.Kp, e0, st, flag);
 }
 
 }  // namespace fx

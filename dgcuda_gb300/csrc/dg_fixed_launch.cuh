@@ -71,8 +71,8 @@ void run_batch(const BatchLaunch &b, cudaStream_t st, int lo, int n, int blk, in
   const FxTab<P> &tab = *static_cast<const FxTab<P> *>(b.fx[P]);
   const int sub = blk / kTile;
   if (stage < 0) {
-    k_trace_batch_fx<Eq, P><<<n * sub, S::kThreads, 0, st>>>(tab, b.probs, b.eblk2prob, b.eblk0,
-                                                             lo, sub);
+    k_trace_batch_fx<Eq, P, false><<<n * sub, S::kThreads, 0, st>>>(
+        tab, b.probs, b.eblk2prob, b.eblk0, lo, sub, 0);
   } else if (!lim) {
     k_element_batch_fx<Eq, P, 1><<<n * sub, S::kThreads, 0, st>>>(
         tab, b.probs, b.eblk2prob, b.eblk0, lo, sub, stage, check);
@@ -91,6 +91,22 @@ void batch_element(const BatchLaunch &b, cudaStream_t st, int p, int lo, int n, 
     if (p == 2) run_batch<Eq, 2>(b, st, lo, n, blk, stage, check, lim);
     if (p == 3) run_batch<Eq, 3>(b, st, lo, n, blk, stage, check, lim);
   }
+}
+
+// the limiter of a stage's output and its traces, of the same blocks (equations
+// without the limiter in the element stage)
+template <class Eq, int P>
+void run_batch_limit(const BatchLaunch &b, int lo, int n, int blk, int stage) {
+  const int sub = blk / kTile;
+  k_trace_batch_fx<Eq, P, true><<<n * sub, Shape<Eq, P>::kThreads, 0, b.st>>>(
+      *static_cast<const FxTab<P> *>(b.fx[P]), b.probs, b.eblk2prob, b.eblk0, lo, sub, stage);
+}
+
+template <class Eq>
+void batch_limit(const BatchLaunch &b, int p, int lo, int n, int blk, int stage) {
+  if (p == 1) run_batch_limit<Eq, 1>(b, lo, n, blk, stage);
+  if (p == 2) run_batch_limit<Eq, 2>(b, lo, n, blk, stage);
+  if (p == 3) run_batch_limit<Eq, 3>(b, lo, n, blk, stage);
 }
 
 }  // namespace fx

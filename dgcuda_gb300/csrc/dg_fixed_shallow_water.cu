@@ -8,5 +8,6 @@ template void element<ShallowWater>(const Ctx &, const ElemArgs &, int);
 template void trace<ShallowWater>(const Ctx &, double *, int);
 template void batch_element<ShallowWater>(const BatchLaunch &, cudaStream_t, int, int, int, int, int,
                                   int, bool);
+template void batch_limit<ShallowWater>(const BatchLaunch &, int, int, int, int, int);
 }  // namespace fx
 }  // namespace dg

@@ -38,8 +38,9 @@
 // With the limiter on, the limiter runs on those traces: for Euler in the
 // element stage's own epilogue, with the neighbours' new cell means found
 // before it by k_means from the per-side flux sums k_face<FS> leaves; for the
-// other equations as the pass k_limit_tr.  Either way a limited element's
-// traces are rebuilt from its limited modes.
+// other equations in the pass that limits and traces a state (k_trace_fx; p = 5
+// k_limit_tr).  Either way a limited element's traces are rebuilt from its limited
+// modes, by the contraction of the other traces.
 #pragma once
 #include <algorithm>
 #include "dg_device.cuh"
@@ -1056,22 +1057,6 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-template <class Eq>
-__global__ void __launch_bounds__(kMaxBlock)
-    k_limit_tr_batch(const __grid_constant__ BatchTabs tb, const BatchProb *__restrict__ probs,
-                     const int *__restrict__ blk2prob, const int *__restrict__ blk0, int stage) {
-  const int pi = blk2prob[blockIdx.x];
-  const BatchProb &pr = probs[pi];
-  const int e = (blockIdx.x - blk0[pi]) * blockDim.x + threadIdx.x;
-  if (e >= pr.K) return;
-  double *u = stage == 2 ? pr.U : pr.W;
-  switch (pr.p) {
-    case 1: limit_tr_body<Eq, 1>(tb.t1, pr.q, u, pr.T, pr.nbr, pr.Kp, e, u, (size_t)Tab<1>::NP * pr.Kp); break;
-    case 2: limit_tr_body<Eq, 2>(tb.t2, pr.q, u, pr.T, pr.nbr, pr.Kp, e, u, (size_t)Tab<2>::NP * pr.Kp); break;
-    case 3: limit_tr_body<Eq, 3>(tb.t3, pr.q, u, pr.T, pr.nbr, pr.Kp, e, u, (size_t)Tab<3>::NP * pr.Kp); break;
-  }
-}
-
 // (the orders that contract in FP64: Euler's p = 2 and 3)
 template <class Eq>
 __global__ void __launch_bounds__(kMaxBlock)
@@ -1123,6 +1108,9 @@ void trace(const Ctx &c, double *u, int what);
 template <class Eq>
 void batch_element(const BatchLaunch &b, cudaStream_t st, int p, int lo, int n, int blk,
                    int stage, int check, bool lim);
+// the limiter of a stage's output and its traces, of the same blocks
+template <class Eq>
+void batch_limit(const BatchLaunch &b, int p, int lo, int n, int blk, int stage);
 }  // namespace fx
 inline unsigned nblk(int n, int b = kBlock) { return (unsigned)((n + b - 1) / b); }
 
@@ -1283,10 +1271,13 @@ struct Launch {
     DG_DISPATCH_P((k_bed_slopes<P><<<nblk(c.m.K, c.blk), c.blk, 0, c.st>>>(
         tab<P>(c), c.m.bathy, c.m.geo, out, c.m.K, c.m.Kp)));
   }
+  // (p = 5 of the equations without the limiter in the element stage: at p = 1..4
+  // limit_trace() forms the limited traces as the next trace pass would)
   static void limit_tr(const Ctx &c, double *u) {
     if (!c.m.K || c.p < 1) return;
-    DG_DISPATCH_P((launch(k_limit_tr<Eq, P>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q, u,
-                          c.T, c.m.nbr, c.m.K, c.m.Kp)));
+    DG_DISPATCH_P(if constexpr (P == 5 && !Eq::kFusedLimiter) (
+        launch(k_limit_tr<Eq, P>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q, u, c.T,
+               c.m.nbr, c.m.K, c.m.Kp)));
   }
   static void limit(const Ctx &c, double *u) {
     if (!c.m.K || c.p < 1) return;
@@ -1295,7 +1286,8 @@ struct Launch {
         launch(k_limit<Eq, P>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), u, c.m.nbr, c.m.K,
                c.m.Kp)));
   }
-  // limit() and trace(): the start of an SSP-RK3 run with the limiter on
+  // limit() and trace(): the start of an SSP-RK3 run with the limiter on, and the
+  // limiter of a stage where the element stage has none
   static void limit_trace(const Ctx &c, double *u) {
     if (c.m.K && c.fx) return fx::trace<Eq>(c, u, 1);
     limit(c, u);
@@ -1390,9 +1382,13 @@ struct Launch {
     k_means_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0,
                                                     stage);
   }
+  // (Euler's batch limits in its element stage)
   static void b_limit_tr(const BatchLaunch &b, int stage) {
-    k_limit_tr_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0,
-                                                       stage);
+    if constexpr (!Eq::kFusedLimiter)
+      for (int g = 0; g < BatchLaunch::kGroups; g++) {
+        const int lo = b.eblk_g[g], n = b.eblk_g[g + 1] - lo, p = 1 + g / 2;
+        if (n > 0) fx::batch_limit<Eq>(b, p, lo, n, b.blk_g[g], stage);
+      }
   }
   static void b_lambda(const BatchLaunch &b) {
     k_lambda_batch<Eq><<<b.nlblk, kBlock, 0, b.st>>>(btabs(b), b.probs, b.lblk2prob, b.lblk0);

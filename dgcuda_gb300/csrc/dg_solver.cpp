@@ -179,7 +179,10 @@ void limit(dg_solver *s, double *u) {
 // With the limiter on (Euler), the limiter runs in the element stage's
 // epilogue: the face kernel also sums each side's fluxes, and
 // k_means turns the sums into the output's cell means, which the element
-// stage needs for its neighbours' bounds; no separate limiter pass.
+// stage needs for its neighbours' bounds; no separate limiter pass.  The other
+// equations' limiter forms the limited traces in the pass that starts a run, so
+// that a run begun from the limited state finds the bits of the one that went on
+// (k_limit_tr, at p = 5, does so in FP64).
 void fused_stage(dg_solver *s, double *us, const double *un, double *out, double ca, double cb,
                  double cc, double tcoef, const double *dtp) {
   const bool lim = s->prm.limiter && s->np >= 3;
@@ -190,6 +193,11 @@ void fused_stage(dg_solver *s, double *us, const double *un, double *out, double
     return;
   }
   run(s, K_FACE, [&] { s->ops->face(s->ctx, &s->ds->t, tcoef); });
+  if (lim && s->ctx.fx) {
+    run(s, K_ELEMENT, [&] { s->ops->element(s->ctx, us, un, out, ca, cb, cc, dtp); });
+    run(s, K_LIMIT, [&] { s->ops->limit_trace(s->ctx, out); });
+    return;
+  }
   run(s, K_ELEMENT,
       [&] { s->ops->element_tr(s->ctx, us, un, out, ca, cb, cc, dtp, lim ? 0 : 1); });
   if (lim) run(s, K_LIMIT, [&] { s->ops->limit_tr(s->ctx, out); });
