@@ -118,6 +118,7 @@ def _declare(L):
         "dg_set_tensor_contractions": (C.c_int, [C.c_void_p, C.c_int]),
         "dg_fx_table_image": (C.c_int, [C.c_int, C.c_void_p, C.c_size_t]),
         "dg_oz_table_image": (C.c_int, [C.c_int, C.c_void_p, C.c_size_t, _dp]),
+        "dg_get_element_stage": (C.c_int, [C.c_void_p, _ip]),
         "dg_get_tensor_contractions": (C.c_int, [C.c_void_p, _ip]),
         "dg_load_checkpoint": (C.c_int, [C.c_void_p, C.c_char_p, _dp]),
         "dg_set_bathymetry": (C.c_int, [C.c_void_p, _dp]),
@@ -519,10 +520,10 @@ class Solver:
 
     @property
     def tensor_contractions(self):
-        """True when the Euler element stage computes its contractions as exact
-        integer slices (p = 2..4, on by default; at p = 1, where it is off by
-        default, the switch has no effect: the stage always does, as the other
-        equations' at p = 1..4)."""
+        """The switch of the Euler element stage at p = 1..4: True for contractions
+        as exact integer slices, False for FP64 multiply-adds.  Not set, the stage
+        takes the slices and the switch reads True at p = 2..4, False at p = 1;
+        `element_stage` says which stage runs."""
         v = np.zeros(1, dtype=np.int32)
         _check(self._L.dg_get_tensor_contractions(self._h, _iptr(v)))
         return bool(v[0])
@@ -530,6 +531,13 @@ class Solver:
     @tensor_contractions.setter
     def tensor_contractions(self, on):
         _check(self._L.dg_set_tensor_contractions(self._h, int(bool(on))))
+
+    @property
+    def element_stage(self):
+        """The element stage that runs: 1 FP64 multiply-adds, 2 fixed point."""
+        v = np.zeros(1, dtype=np.int32)
+        _check(self._L.dg_get_element_stage(self._h, _iptr(v)))
+        return int(v[0])
 
     def set_velocity_field(self, ax, ay, grad=None):
         """Advection velocity a(x, y) = (ax, ay) + grad (x, y), grad =

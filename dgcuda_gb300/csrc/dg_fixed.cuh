@@ -624,7 +624,7 @@ __device__ __forceinline__ int batch_tile(const int *__restrict__ blk2prob,
   return ((b - blk0[pi]) * sub + (int)blockIdx.x % sub) * kTile;
 }
 
-template <class Eq, int P, int MODE>
+template <class Eq, int P>
 __global__ void __launch_bounds__(Shape<Eq, P>::kThreads, min_blocks<Eq, P>())
     k_element_batch_fx(const __grid_constant__ FxTab<P> tab, const BatchProb *__restrict__ probs,
                        const int *__restrict__ blk2prob, const int *__restrict__ blk0, int b_lo,
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(Shape<Eq, P>::kThreads, min_blocks<Eq, P>())
   const BatchProb &pr = probs[pi];
   if (e0 >= pr.K) return;
   const ElemArgs a = batch_elem_args(pr, stage, check);
-  element_tile<Eq, P, MODE>(tab, pr.q, a, e0, st, mxs, flag);
+  element_tile<Eq, P, 1>(tab, pr.q, a, e0, st, mxs, flag);
 }
 
 // the traces of the states U, and with LIM the limiter of a stage's output first

@@ -7,7 +7,7 @@ namespace fx {
 template void element<Advection>(const Ctx &, const ElemArgs &, int);
 template void trace<Advection>(const Ctx &, double *, int);
 template void batch_element<Advection>(const BatchLaunch &, cudaStream_t, int, int, int, int, int,
-                                  int, bool);
+                                  int);
 template void batch_limit<Advection>(const BatchLaunch &, int, int, int, int, int);
 }  // namespace fx
 }  // namespace dg

@@ -6,7 +6,5 @@ namespace dg {
 namespace fx {
 template void element<Euler>(const Ctx &, const ElemArgs &, int);
 template void trace<Euler>(const Ctx &, double *, int);
-template void batch_element<Euler>(const BatchLaunch &, cudaStream_t, int, int, int, int, int,
-                                  int, bool);
 }  // namespace fx
 }  // namespace dg

@@ -61,40 +61,31 @@ void trace(const Ctx &c, double *u, int what) {
   }
 }
 
-// the element stage (lim: with the limiter), and with stage < 0 the
-// start-of-run traces, of n blocks of blk elements from block lo of a batch's
-// map, all of order p
+// the element stage, and with stage < 0 the start-of-run traces, of n blocks of
+// blk elements from block lo of a batch's map, all of order p
 template <class Eq, int P>
-void run_batch(const BatchLaunch &b, cudaStream_t st, int lo, int n, int blk, int stage, int check,
-               bool lim) {
+void run_batch(const BatchLaunch &b, cudaStream_t st, int lo, int n, int blk, int stage,
+               int check) {
   using S = Shape<Eq, P>;
   const FxTab<P> &tab = *static_cast<const FxTab<P> *>(b.fx[P]);
   const int sub = blk / kTile;
-  if (stage < 0) {
+  if (stage < 0)
     k_trace_batch_fx<Eq, P, false><<<n * sub, S::kThreads, 0, st>>>(
         tab, b.probs, b.eblk2prob, b.eblk0, lo, sub, 0);
-  } else if (!lim) {
-    k_element_batch_fx<Eq, P, 1><<<n * sub, S::kThreads, 0, st>>>(
-        tab, b.probs, b.eblk2prob, b.eblk0, lo, sub, stage, check);
-  } else {
-    if constexpr (Eq::kFusedLimiter)
-      k_element_batch_fx<Eq, P, 2><<<n * sub, S::kThreads, 0, st>>>(
-          tab, b.probs, b.eblk2prob, b.eblk0, lo, sub, stage, check);
-  }
+  else
+    k_element_batch_fx<Eq, P><<<n * sub, S::kThreads, 0, st>>>(tab, b.probs, b.eblk2prob, b.eblk0,
+                                                               lo, sub, stage, check);
 }
 
 template <class Eq>
 void batch_element(const BatchLaunch &b, cudaStream_t st, int p, int lo, int n, int blk,
-                   int stage, int check, bool lim) {
-  if (p == 1) return run_batch<Eq, 1>(b, st, lo, n, blk, stage, check, lim);
-  if constexpr (!Eq::kFusedLimiter) {  // Euler's batch contracts in FP64 at p = 2 and 3
-    if (p == 2) run_batch<Eq, 2>(b, st, lo, n, blk, stage, check, lim);
-    if (p == 3) run_batch<Eq, 3>(b, st, lo, n, blk, stage, check, lim);
-  }
+                   int stage, int check) {
+  if (p == 1) run_batch<Eq, 1>(b, st, lo, n, blk, stage, check);
+  if (p == 2) run_batch<Eq, 2>(b, st, lo, n, blk, stage, check);
+  if (p == 3) run_batch<Eq, 3>(b, st, lo, n, blk, stage, check);
 }
 
-// the limiter of a stage's output and its traces, of the same blocks (equations
-// without the limiter in the element stage)
+// the limiter of a stage's output and its traces, of the same blocks
 template <class Eq, int P>
 void run_batch_limit(const BatchLaunch &b, int lo, int n, int blk, int stage) {
   const int sub = blk / kTile;

@@ -7,7 +7,7 @@ namespace fx {
 template void element<Maxwell>(const Ctx &, const ElemArgs &, int);
 template void trace<Maxwell>(const Ctx &, double *, int);
 template void batch_element<Maxwell>(const BatchLaunch &, cudaStream_t, int, int, int, int, int,
-                                  int, bool);
+                                  int);
 template void batch_limit<Maxwell>(const BatchLaunch &, int, int, int, int, int);
 }  // namespace fx
 }  // namespace dg

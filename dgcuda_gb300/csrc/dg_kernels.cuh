@@ -25,8 +25,8 @@
 // FP32 rate), so the contractions of the element stage and the traces run on
 // the integer pipes in fixed point: k_element_fx and k_trace_fx (dg_fixed.cuh)
 // carry every equation and order.  k_element and k_trace here, one thread per
-// element in FP64, stay for the Euler equations at p >= 2 with the contraction
-// switch off and for the Euler batch at p >= 2 (Launch::fp64).  What is left on
+// element in FP64, stay for the Euler equations with the contraction switch off
+// and for the Euler batch (Launch::fp64).  What is left on
 // the FP64 pipe uses few instructions: basis values are constant-bank operands
 // (tables are __grid_constant__ parameters, loops are unrolled), each Riemann
 // flux is evaluated once per side, with its reciprocals, square roots and
@@ -1057,7 +1057,7 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-// (the orders that contract in FP64: Euler's p = 2 and 3)
+// (Euler's batch, which contracts in FP64)
 template <class Eq>
 __global__ void __launch_bounds__(kMaxBlock)
     k_trace_batch(const __grid_constant__ BatchTabs tb, const BatchProb *__restrict__ probs,
@@ -1067,6 +1067,7 @@ __global__ void __launch_bounds__(kMaxBlock)
   const int e = (blockIdx.x - blk0[pi]) * blockDim.x + threadIdx.x;
   if (e >= pr.K) return;
   switch (pr.p) {
+    case 1: trace_body<Eq, 1>(tb.t1, pr.q, pr.U, pr.T, pr.Kp, e); break;
     case 2: trace_body<Eq, 2>(tb.t2, pr.q, pr.U, pr.T, pr.Kp, e); break;
     case 3: trace_body<Eq, 3>(tb.t3, pr.q, pr.U, pr.T, pr.Kp, e); break;
   }
@@ -1104,10 +1105,10 @@ void element(const Ctx &c, const ElemArgs &a, int mode);
 template <class Eq>
 void trace(const Ctx &c, double *u, int what);
 // of a batch's blocks of one order: the element stage, or with stage < 0 the
-// start-of-run traces
+// start-of-run traces (all equations but Euler, whose batch contracts in FP64)
 template <class Eq>
 void batch_element(const BatchLaunch &b, cudaStream_t st, int p, int lo, int n, int blk,
-                   int stage, int check, bool lim);
+                   int stage, int check);
 // the limiter of a stage's output and its traces, of the same blocks
 template <class Eq>
 void batch_limit(const BatchLaunch &b, int p, int lo, int n, int blk, int stage);
@@ -1149,10 +1150,10 @@ struct Launch {
     case 5: { constexpr int P = 5; expr; } break; \
   }
 
-  // orders whose FP64 traces and element stage are reachable: Euler's p = 2..4
-  // (its fixed-point stage can be switched off there, and its batch contracts
-  // in FP64), elsewhere only those without a fixed-point stage
-  static constexpr bool fp64(int P) { return (Eq::kFusedLimiter && P != 1) || P < 1 || P > 4; }
+  // orders whose FP64 traces and element stage are reachable: Euler's (its
+  // fixed-point stage can be switched off, and its batch contracts in FP64),
+  // elsewhere only those without a fixed-point stage
+  static constexpr bool fp64(int P) { return Eq::kFusedLimiter || P < 1 || P > 4; }
 
   static ElemArgs eargs(const Ctx &c, double *us, const double *un, double *out, double ca,
                         double cb, double cc, const double *dtp, double *T, int check) {
@@ -1327,12 +1328,13 @@ struct Launch {
     return *reinterpret_cast<const BatchTabs *>(b.tabs);
   }
   static void b_trace(const BatchLaunch &b) {
-    for (int g = 0; g < BatchLaunch::kGroups; g++) {
-      const int lo = b.eblk_g[g], n = b.eblk_g[g + 1] - lo, p = 1 + g / 2;
-      if (n > 0 && b.fx[p]) fx::batch_element<Eq>(b, b.st, p, lo, n, b.blk_g[g], -1, 1, false);
-    }
-    if constexpr (Eq::kFusedLimiter)  // the orders that contract in FP64
+    if constexpr (Eq::kFusedLimiter)
       k_trace_batch<Eq><<<b.nublk, b.blk, 0, b.st>>>(btabs(b), b.probs, b.ublk2prob, b.ublk0);
+    else
+      for (int g = 0; g < BatchLaunch::kGroups; g++) {
+        const int lo = b.eblk_g[g], n = b.eblk_g[g + 1] - lo, p = 1 + g / 2;
+        if (n > 0) fx::batch_element<Eq>(b, b.st, p, lo, n, b.blk_g[g], -1, 1);
+      }
   }
   // blocks of k_face_batch per block of the map: enough for p = 3's 32 sides
   static int face_sub(const BatchLaunch &b) { return (b.blk + kBlock / 4 - 1) / (kBlock / 4); }
@@ -1355,10 +1357,13 @@ struct Launch {
       const cudaStream_t st = side ? b.gst[g] : b.st;
       first = false;
       if (side) cudaStreamWaitEvent(st, b.fork, 0);
-      if (b.fx[p]) {
-        fx::batch_element<Eq>(b, st, p, lo, n, blk, stage, check, LIM);
-      } else if constexpr (Eq::kFusedLimiter) {
-        if (p == 2)
+      if constexpr (!Eq::kFusedLimiter) {
+        fx::batch_element<Eq>(b, st, p, lo, n, blk, stage, check);
+      } else {
+        if (p == 1)
+          k_element_batch_p<Eq, 1, LIM><<<n, blk, 0, st>>>(tb.t1, b.probs, b.eblk2prob, b.eblk0,
+                                                             lo, stage, check);
+        else if (p == 2)
           k_element_batch_p<Eq, 2, LIM><<<n, blk, 0, st>>>(tb.t2, b.probs, b.eblk2prob, b.eblk0,
                                                              lo, stage, check);
         else

@@ -102,7 +102,7 @@ struct BatchLaunch {
   cudaStream_t st = nullptr;
   const void *tabs = nullptr;       // BatchTabs image (Tab<1>, Tab<2>, Tab<3>)
   // host FxTab<p> images of p = 1..3 where the batch contracts in fixed point
-  // (null: FP64, Euler at p = 2 and 3)
+  // (null: FP64, Euler)
   const void *fx[4] = {nullptr, nullptr, nullptr, nullptr};
   BatchProb *probs = nullptr;       // device array
   int nprob = 0, blk = 128, limiter = 0;

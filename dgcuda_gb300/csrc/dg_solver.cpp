@@ -56,7 +56,9 @@ struct dg_solver {
   // rows, so that the permutation of one chunk overlaps the copy of the next
   cudaStream_t cst = nullptr;
   std::vector<cudaEvent_t> cev;
-  bool tensor = true;             // Euler: fixed-point contractions (dg_set_tensor_contractions)
+  // Euler: fixed-point contractions (dg_set_tensor_contractions): 1 on, 0 off, -1 as
+  // the order has it (on; reported as off at p = 1)
+  int tensor = -1;
   // T holds the traces of U as the last fused SSP-RK3 stage left them (and U
   // is already limited): the next dg_step continues without recomputing
   // them, so a run split over several calls is the uninterrupted run
@@ -316,15 +318,13 @@ void drop_graphs(dg_solver *s) {
 }
 
 // whether the solver's element stage has two forms, fixed point and FP64, that
-// dg_set_tensor_contractions switches between: Euler at p = 2..4
-bool fx_switched(const dg_solver *s) {
-  return s->eq == DG_EULER && s->p >= 2 && !s->fximg.empty();
-}
+// dg_set_tensor_contractions switches between: Euler at p = 1..4
+bool fx_switched(const dg_solver *s) { return s->eq == DG_EULER && !s->fximg.empty(); }
 
-// the element stage's contractions: fixed point at p = 1..4, for Euler at p =
-// 2..4 only where it is switched on
+// the element stage's contractions: fixed point at p = 1..4, for Euler unless it
+// is switched off
 void fx_select(dg_solver *s) {
-  const bool on = !s->fximg.empty() && (!fx_switched(s) || s->tensor);
+  const bool on = !s->fximg.empty() && (!fx_switched(s) || s->tensor != 0);
   s->ctx.fx = on ? s->fximg.data() : nullptr;
 }
 
@@ -688,7 +688,6 @@ extern "C" dg_status dg_solver_create(const dg_mesh *mesh, dg_equation eq, int p
   c.Fs = s->Fs;
   c.M = s->M;
   c.ds = s->ds;
-  s->tensor = p >= 2;
   fx_refresh(s);
   *out = s;
   return DG_OK;
@@ -1315,7 +1314,7 @@ dg_status batch_run(dg_batch *b, int nsteps, double *t) {
     if (b->limiter && s->np >= 3) {
       dg::Ctx c = s->ctx;
       c.st = b->st;
-      if (b->eq == DG_EULER && s->p > 1) c.fx = nullptr;  // FP64, as its batch at these orders
+      if (b->eq == DG_EULER) c.fx = nullptr;  // FP64, as its batch
       s->ops->limit(c, s->U);
       b->launches++;
     }
@@ -1386,10 +1385,9 @@ extern "C" dg_status dg_batch_create(int n, dg_solver *const *members, dg_batch 
   b->ops = batch_ops_for(b->eq);
   b->tabs.resize(dg::batch_tabs_bytes());
   dg::build_batch_tabs(timg[1], timg[2], timg[3], b->tabs.data());
-  // orders that contract in fixed point (all but Euler's p = 2 and 3, whose
-  // batch contracts in FP64): the default tables or the first member's of
-  // each order, as the FP64 tables above
-  for (int p = 1; p <= (b->eq == DG_EULER ? 1 : 3); p++) {
+  // fixed point (all but Euler, whose batch contracts in FP64): the default
+  // tables or the first member's of each order, as the FP64 tables above
+  for (int p = 1; p <= (b->eq == DG_EULER ? 0 : 3); p++) {
     b->fximg[p].resize(dg::fx_tab_bytes(p));
     if (!timg[p]) {
       std::vector<char> t(dg::tab_bytes(p));
@@ -2242,11 +2240,11 @@ extern "C" dg_status dg_load_checkpoint(dg_solver *s, const char *path, double *
 }
 
 // the Euler element stage's basis contractions in fixed point (dg_fixed.cuh) or
-// in FP64 FMAs, p = 2..4 (at p = 1 the switch is kept and has no effect)
+// in FP64 FMAs, p = 1..4
 extern "C" dg_status dg_set_tensor_contractions(dg_solver *s, int on) {
   if (!s) return fail(DG_BAD_ARG, "null solver");
   s->tr_valid = false;
-  if (on && (s->eq != DG_EULER || s->fximg.empty()))
+  if (on && !fx_switched(s))
     return fail(DG_UNSUPPORTED, "exact-slice contractions are switched for Euler, p = 1..4");
   CK(cudaSetDevice(s->device));
   CK(cudaStreamSynchronize(s->st));
@@ -2258,7 +2256,13 @@ extern "C" dg_status dg_set_tensor_contractions(dg_solver *s, int on) {
 
 extern "C" dg_status dg_get_tensor_contractions(dg_solver *s, int *on) {
   if (!s || !on) return fail(DG_BAD_ARG, "null argument");
-  *on = s->eq == DG_EULER && !s->fximg.empty() && s->tensor;
+  *on = fx_switched(s) && (s->tensor > 0 || (s->tensor < 0 && s->p > 1));
+  return DG_OK;
+}
+
+extern "C" dg_status dg_get_element_stage(const dg_solver *s, int *stage) {
+  if (!s || !stage) return fail(DG_BAD_ARG, "null argument");
+  *stage = s->ctx.fx ? 2 : 1;
   return DG_OK;
 }
 

@@ -226,13 +226,17 @@ dg_status dg_set_inflow_series(dg_solver *s, int n, const double *amp, const dou
 /* The element stage computes its basis contractions (area values, volume
  * and surface projections, next-stage traces) at p = 1..4 as exact integer
  * slices off the FP64 pipe (56-bit fixed point, per-output error below an
- * FP64 dot product's rounding).  For Euler at p = 2..4 this can be
- * switched: off, the contractions are FP64 FMAs; on by default.  At p = 1 the
- * switch (off by default) is kept and has no effect: the slices are the
- * faster stage there too.  DG_UNSUPPORTED for other equations and orders.
+ * FP64 dot product's rounding).  For Euler at p = 1..4 this can be
+ * switched: off, the contractions are FP64 FMAs.  DG_UNSUPPORTED for other
+ * equations and orders.  Until it is called a solver takes the slices, the
+ * faster stage at every order; dg_get_tensor_contractions then says 1 at p =
+ * 2..4 and 0 at p = 1, where the switch's default was off, and afterwards what
+ * was set.  dg_get_element_stage says which stage runs.
  * (The name is from an earlier form of the slices, f16 digits on the tensor
  * cores.)  No reference counterpart. */
 dg_status dg_set_tensor_contractions(dg_solver *s, int on);
+/* the element stage that runs: 1 the FP64-FMA one, 2 the fixed-point one */
+dg_status dg_get_element_stage(const dg_solver *s, int *stage);
 /* the basis tables of order p = 1..4 as f16 digit slices, built on the host from
  * the library's basis tables (for checks; no GPU needed): 2240 pairs of
  * 32-bit words, each two f16 digits, then 3 x 16 int column exponents and 16
@@ -276,8 +280,8 @@ dg_status dg_bathymetry_project(dg_solver *s, int kind, const double *prm);
 dg_status dg_autotune(dg_solver *s, int *block);
 /* dg_autotune that also chooses the element stage, where a solver has two:
  * the FP64-FMA kernel, one thread per element (1), or the fixed-point kernel
- * with one thread per element and variable (2; Euler, p = 2..4 -- at p = 1, and
- * for the other equations at p = 1..4, there is only the latter).
+ * with one thread per element and variable (2; Euler, p = 1..4 -- for the
+ * other equations at p = 1..4 there is only the latter).
  * *threads_per_element receives 1 or 2.  The two agree to FP64
  * rounding, not bit for bit, so a run's last bits follow the choice. */
 dg_status dg_autotune_stage(dg_solver *s, int *block, int *threads_per_element);
