@@ -723,19 +723,22 @@ extern "C" dg_status dg_solver_sizes(const dg_solver *s, int *N, int *n_p, int *
 extern "C" void *dg_solver_stream(dg_solver *s) { return s ? (void *)s->st : nullptr; }
 
 // ---- shallow-water bed ---------------------------------------------------
-// the bed's slopes at the area points, which the fixed-point stage reads in
-// place of the bed's modes (they change only with the bed and the tables)
+// memory for a bed's modes and for its slopes at the area points, which the
+// fixed-point stage reads in their place: both before a bed is set, so that a
+// failure leaves the solver as it was and never a bed without its slopes
+static dg_status alloc_bed(dg_solver *s) {
+  dg_status st = DG_OK;
+  if (!s->bathy) st = dalloc(s, &s->bathy, (size_t)s->np * s->m.Kp);
+  if (st == DG_OK && s->ctx.fx && !s->bslope)
+    st = dalloc(s, &s->bslope, (size_t)2 * dg::nq_of(s->p) * s->m.Kp);
+  return st;
+}
+
+// the slopes of the bed in place (they change only with the bed and the tables)
 static dg_status set_bed_slopes(dg_solver *s) {
-  s->m.bslope = nullptr;
-  if (s->m.bathy && s->ctx.fx) {
-    if (!s->bslope) {
-      dg_status st = dalloc(s, &s->bslope, (size_t)2 * dg::nq_of(s->p) * s->m.Kp);
-      if (st != DG_OK) return st;
-    }
-    s->ops->bed_slopes(s->ctx, s->bslope);
-    s->m.bslope = s->bslope;
-  }
+  s->m.bslope = s->m.bathy && s->ctx.fx ? s->bslope : nullptr;
   s->ctx.m.bslope = s->m.bslope;
+  if (s->m.bslope) s->ops->bed_slopes(s->ctx, s->bslope);
   return sync_check(s);
 }
 
@@ -1024,10 +1027,8 @@ extern "C" dg_status dg_set_bathymetry(dg_solver *s, const double *b) {
   if (!b) {
     s->m.bathy = nullptr;
   } else {
-    if (!s->bathy) {
-      dg_status st = dalloc(s, &s->bathy, (size_t)s->np * s->m.Kp);
-      if (st != DG_OK) return st;
-    }
+    dg_status st = alloc_bed(s);
+    if (st != DG_OK) return st;
     CK(cudaMemcpyAsync(s->ubuf, b, (size_t)s->np * s->K * sizeof(double),
                        cudaMemcpyHostToDevice, s->st));
     dg::launch_permute_in(s->st, s->ubuf, s->bathy, s->m.perm, s->np, s->K, s->m.Kp);
