@@ -753,6 +753,7 @@ extern "C" dg_status dg_solver_set_tables(dg_solver *s, int n_q, int n_1, const 
   s->tr_valid = false;
   if (n_q != dg::nq_of(s->p) || n_1 != s->p + 1)
     return fail(DG_BAD_ARG, "table sizes do not match the order p");
+  CK(cudaSetDevice(s->device));  // a bed's slopes are formed again on it
   dg_order_tables t{};
   int np = s->np;
   t.n_p = np;

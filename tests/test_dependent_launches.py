@@ -1,7 +1,8 @@
-"""Kernels launched with programmatic dependence live beside their
-predecessor's last stores: what a step computes must not reach them through
-read-only loads or __restrict__ pointers, which the compiler may take across
-the wait at their start.  Read off the sources (no GPU needed)."""
+"""Read off the sources (no GPU needed).  Kernels launched with programmatic
+dependence live beside their predecessor's last stores: what a step computes
+must not reach them through read-only loads or __restrict__ pointers, which
+the compiler may take across the wait at their start.  And the C entries
+launch on their solver's device."""
 import glob
 import os
 import re
@@ -47,3 +48,17 @@ def test_their_device_functions_take_no_restrict_pointer_and_no_read_only_load()
     for f, text in src.items():
         for m in re.finditer(r"__ldg\((.{0,12})", text):
             assert m.group(1).startswith("a.vtx"), (f, m.group(0))
+
+
+def test_entry_points_that_launch_set_their_device_first():
+    """A solver's work runs on its own GPU whichever the thread's current one
+    is: the C entries make it current before their first launch."""
+    work = re.compile(r"->ops->|dg::launch_|set_bed_slopes\(|\brun\(s|run_steps\(|put_rows\(")
+    text = open(os.path.join(CSRC, "dg_solver.cpp")).read()
+    seen = 0
+    for m in re.finditer(r'extern "C" [\w ]+\*?\b(dg_\w+)\([^{;]*\)\s*\{\n(.*?)\n\}', text, re.S):
+        w = work.search(m.group(2))
+        if w:
+            seen += 1
+            assert "cudaSetDevice" in m.group(2)[:w.start()], m.group(1)
+    assert seen >= 10
