@@ -785,6 +785,18 @@ extern "C" dg_status dg_solver_set_tables(dg_solver *s, int n_q, int n_1, const 
     for (int j = 0; j < n_1; j++)
       if (t.E[f][j][0] != t.E[0][0][0])
         return fail(DG_BAD_ARG, "basis function 0 must take one value on every edge point");
+  // an infinity or a NaN has no limbs: the fixed-point stage would hand out numbers
+  if (s->p >= 1 && s->p <= 4) {
+    bool finite = true;
+    for (int i = 0; i < np; i++) {
+      for (int q = 0; q < n_q; q++)
+        finite = finite && std::isfinite(t.B[q][i]) && std::isfinite(t.GR[q][i]) &&
+                 std::isfinite(t.GS[q][i]);
+      for (int f = 0; f < 3; f++)
+        for (int j = 0; j < n_1; j++) finite = finite && std::isfinite(t.E[f][j][i]);
+    }
+    if (!finite) return fail(DG_BAD_ARG, "basis tables must be finite");
+  }
   s->tables = t;
   dg::build_tab(s->p, s->tables, s->tabimg.data());
   field_refresh(s);

@@ -38,3 +38,21 @@ def test_tables_set_after_a_bed_rebuild_its_slopes(dglib, oracle_mod, p):
     o.set_bathymetry(b)
     assert np.array_equal(out[0], out[1])
     assert relerr(out[0], o.rhs(c, 0.0), 3) <= 1e-12
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_tables_that_are_not_finite_are_refused(dglib, bad):
+    """And leave the tables before them."""
+    dg = dglib
+    mesh = dg.Mesh.square(4, 4, jitter=0.1, seed=3)
+    s = dg.Solver(mesh, dg.ADVECTION, 2, problem="adv_sine")
+    s.init_conditions()
+    c = s.get_state()
+    r = s.eval_rhs(c, 0.0)
+    for k in range(4):  # values, both slopes, edge values
+        tab = split_tables(ref_tables(2), 2)
+        tab[k] = tab[k].copy()
+        tab[k][-1] = bad
+        with pytest.raises(dg.DGError):
+            s.set_tables(*tab)
+    assert np.array_equal(s.eval_rhs(c, 0.0), r)
