@@ -317,8 +317,10 @@ __device__ __forceinline__ void load_F(const double *const (&Fp)[3], const bool 
 // The element stage (element_body's inputs, outputs and rules) of the tile of
 // 32 elements from e0.  MODE 0: no traces; 1: the traces of the output into
 // T, with the positivity rule where a.check is set; 2: the same with the
-// limiter (mode 0 of the output is the stored mean a.M); 3: as 1, and a.acc =
-// a.acc0 + a.ck dt L(us) beside the output (RK4).
+// limiter (mode 0 of the output is the stored mean a.M); 3: as 1, and the sum of
+// RK4's increments beside the output, a.acc = a.acc0 + a.ck dt L(us) (a.acc0 null:
+// zero).  MODE 0 with a.acc0, RK4's last stage: out = un + (a.acc0 + cc dt L(us)),
+// one rounding of the state for the four increments.
 template <class Eq, int P, int MODE>
 __device__ __forceinline__ void element_tile(const FxTab<P> &tab, const EqP &q, const ElemArgs &a,
                                              int e0, double *st, int *mxs, int *flag) {
@@ -521,8 +523,7 @@ __device__ __forceinline__ void element_tile(const FxTab<P> &tab, const EqP &q, 
       const double *in = a.acc0 + (size_t)(n * NP) * Kp + ec;
       double r[NP];
 #pragma unroll
-      for (int i = 0; i < NP; i++)  // a flattened stage input counts as its mean here too
-        r[i] = fma(sk, c[i], badv && i > 0 && a.acc0 == a.us ? 0.0 : in[(size_t)i * Kp]);
+      for (int i = 0; i < NP; i++) r[i] = a.acc0 ? fma(sk, c[i], in[(size_t)i * Kp]) : sk * c[i];
       if (live)
 #pragma unroll
         for (int i = 0; i < NP; i++) a.acc[(size_t)(n * NP + i) * Kp + e] = r[i];
@@ -534,6 +535,8 @@ __device__ __forceinline__ void element_tile(const FxTab<P> &tab, const EqP &q, 
       double v;
       if (MODE == 2 && i == 0) {
         v = a.M[(size_t)n * Kp + ec];
+      } else if (MODE == 0 && a.acc0) {
+        v = unn[(size_t)i * Kp] + fma(sc, c[i], a.acc0[(size_t)(n * NP + i) * Kp + ec]);
       } else {
         const double cin = (badv && i > 0) ? 0.0 : usn[(size_t)i * Kp];
         v = fma(sc, c[i], a.unit_cb ? cin : a.cb * cin);

@@ -342,7 +342,7 @@ struct ElemArgs {
   const double *bslope;     // its slopes at the area points (fixed-point stage) or null
   const double *vtx;        // element vertices (rows of Kp): positions for a velocity field
   double *T;                // traces of out (TR)
-  double *acc;              // RK4 (fixed-point stage): acc = acc0 + ck dt L(us) beside out
+  double *acc;              // RK4 (fixed-point stage): sum of the increments beside out
   const double *acc0;
   double ck;
   const double *M;          // fused limiter: the means of out (k_means), rows of Kp
@@ -1255,8 +1255,8 @@ struct Launch {
     DG_DISPATCH_P(if constexpr (fp64(P)) (
         launch(k_element<Eq, P, true>, nblk(c.m.K, c.blk), c.blk, c.st, tab<P>(c), *c.q, a)));
   }
-  // element_tr() with the positivity rule that also adds ck dt L(us) to acc0
-  // into acc (RK4's weighted sum of the increments); only with c.fx
+  // element_tr() with the positivity rule that also adds ck dt L(us) to acc0 (null:
+  // zero) into acc (RK4's weighted sum of the increments); only with c.fx
   static void element_acc(const Ctx &c, double *us, const double *un, double *out, double ca,
                           double cb, double cc, const double *dtp, double *acc,
                           const double *acc0, double ck) {
@@ -1266,6 +1266,14 @@ struct Launch {
     a.acc0 = acc0;
     a.ck = ck;
     fx::element<Eq>(c, a, 3);
+  }
+  // out = un + (acc0 + cc dt L(us)); only with c.fx
+  static void element_sum(const Ctx &c, double *us, const double *un, double *out, double cc,
+                          const double *dtp, const double *acc0) {
+    if (!c.m.K) return;
+    ElemArgs a = eargs(c, us, un, out, 1.0, 0.0, cc, dtp, nullptr, 0);
+    a.acc0 = acc0;
+    fx::element<Eq>(c, a, 0);
   }
   static void bed_slopes(const Ctx &c, double *out) {
     if (!c.m.K) return;
@@ -1319,7 +1327,7 @@ struct Launch {
 
   static const Ops &ops() {
     static const Ops o = {trace,  face,       element,  limit,  limit_trace, lambda, init, l2err,
-                          element_tr, limit_tr, element_acc, vertex, nullptr, nullptr, nullptr, nullptr};
+                          element_tr, limit_tr, element_acc, element_sum, vertex, nullptr, nullptr, nullptr, nullptr};
     return o;
   }
 

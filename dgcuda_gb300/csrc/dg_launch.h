@@ -174,11 +174,14 @@ struct Ops {
                      double cb, double cc, const double *dtp, int check);
   // limit() reading and updating the traces in T (after element_tr)
   void (*limit_tr)(const Ctx &, double *u);
-  // element_tr() with check that also stores acc = acc0 + ck dt (du/dt of us);
-  // acc may alias acc0 (only where Ctx::fx is set)
+  // element_tr() with check that also stores acc = acc0 + ck dt (du/dt of us), acc0
+  // null: zero; acc may alias acc0 (only where Ctx::fx is set)
   void (*element_acc)(const Ctx &, double *us, const double *un, double *out, double ca,
                       double cb, double cc, const double *dtp, double *acc, const double *acc0,
                       double ck);
+  // out = un + (acc0 + cc dt (du/dt of us)); out may alias un (only where Ctx::fx is set)
+  void (*element_sum)(const Ctx &, double *us, const double *un, double *out, double cc,
+                      const double *dtp, const double *acc0);
   // values of variable var at the three vertices, rows of Kp: out[v][elem]
   void (*vertex)(const Ctx &, const double *u, int var, int mode, double t, double *out);
   // a stage with the limiter in the element stage's epilogue (null where an

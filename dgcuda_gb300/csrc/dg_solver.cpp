@@ -226,8 +226,9 @@ void one_step(dg_solver *s, int scheme) {
   } else if (s->ctx.fx && !(s->prm.limiter && s->np >= 3)) {
     // RK4 and midpoint RK2 without the limiter: each stage writes the next
     // one's input and its traces in its epilogue, and RK4's sum of the
-    // increments beside it, so there are no increments, combinations and
-    // trace passes of their own (Euler p = 2, 60k triangles, RK4: 479 -> 373 us a step)
+    // increments beside it (added to the state once, as rk4_final does), so
+    // there are no increments, combinations and trace passes of their own
+    // (Euler p = 2, 60k triangles, RK4: 479 -> 373 us a step)
     double *in = s->k[0], *acc = s->k[1];
     run(s, K_TRACE, [&] { s->ops->trace(s->ctx, s->U); });
     auto rk = [&](double *us, double cb, double cc, double tcoef, const double *acc0, double ck) {
@@ -237,12 +238,12 @@ void one_step(dg_solver *s, int scheme) {
       });
     };
     if (scheme == DG_RK4) {  // inputs U + k1 / 2, U + k2 / 2, U + k3
-      rk(s->U, 1.0, 0.5, 0.0, s->U, 1.0 / 6.0);
+      rk(s->U, 1.0, 0.5, 0.0, nullptr, 1.0 / 6.0);
       rk(in, 0.0, 0.5, 0.5, acc, 1.0 / 3.0);
       rk(in, 0.0, 1.0, 0.5, acc, 1.0 / 3.0);
       run(s, K_FACE, [&] { s->ops->face(s->ctx, &s->ds->t, 1.0); });
       run(s, K_ELEMENT, [&] {
-        s->ops->element(s->ctx, in, acc, s->U, 1.0, 0.0, 1.0 / 6.0, dt);
+        s->ops->element_sum(s->ctx, in, s->U, s->U, 1.0 / 6.0, dt, acc);
       });
     } else {
       run(s, K_FACE, [&] { s->ops->face(s->ctx, &s->ds->t, 0.0); });

@@ -103,3 +103,28 @@ def test_flattened_elements_match_the_oracle(dglib, oracle_mod, p, scheme, where
     assert o.flattened() >= sel.sum()
     assert n == 1 and abs(t - to) <= 1e-12 * to
     assert relerr(s.get_state(), c, s.N) <= STATE_TOL
+
+
+@pytest.mark.parametrize("scheme", ["RK4", "RK2", "SSP_RK3"])
+@pytest.mark.parametrize("p", [1, 3])
+@pytest.mark.parametrize("case", ["euler_vortex", "maxwell_plane"])
+def test_small_increments_reach_the_state_whole(dglib, oracle_mod, case, p, scheme):
+    """A time step so short that the whole increment is about an ulp of the
+    state: RK4 and RK2 round the state once, to u + dt L(u), where parts added
+    one after another would be lost; SSP-RK3 combines states and may be two
+    roundings off."""
+    dg = dglib
+    s, _ = pair(dg, oracle_mod, case, p)
+    c = s.get_state()
+    L = s.eval_rhs(c, 0.0)
+    big = np.abs(c) > 1e-3
+    dt = 0.8 * np.median(np.spacing(np.abs(c[big])) / np.abs(L[big]))
+    s.step(1, getattr(dg, scheme), 0.0, dt=dt)
+    u, ref = s.get_state(), c + dt * L
+    part = np.abs(dt * L / np.spacing(np.abs(c))) % 1
+    clear = big & (np.abs(part - 0.5) > 0.05)  # not a matter of the last rounding
+    assert clear.sum() > big.sum() // 2 and (ref != c)[clear].mean() > 0.2
+    if scheme == "SSP_RK3":
+        assert (np.abs(u - ref) <= 2 * np.spacing(np.abs(ref)))[clear].all()
+    else:
+        assert np.array_equal(u[clear], ref[clear])
