@@ -30,7 +30,7 @@ Limb limb(double t, int M) {
 
 // The unit of the projection's tables, 2^(M - 1078): the smallest with every |T|
 // <= 2^58 and the |T| that meet in one sum adding up to 2^61 at most, so that sums of
-// at most 63 products with inputs below 2^56 stay in 64 bits.  For the library's
+// at most 63 products with inputs below 2^57 stay in 64 bits.  For the library's
 // tables two bits below the largest entry's exponent, the unit of the other
 // tables: the product that the sums leave out, l tl, is what their error was made
 // of (the header of dg_fixed.cuh has the figures).

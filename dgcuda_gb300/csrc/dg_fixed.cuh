@@ -10,25 +10,25 @@
 // product are still five times the FP64 rate:
 //
 //  * a row of inputs (one element and variable) shares the exponent of its
-//    largest entry; each entry becomes a 56-bit integer X (three bits more
-//    than a double's significand, so entries down to 1/8 of the largest are
-//    exact) in two limbs X = h 2^28 + l, each with x's sign;
+//    largest entry; each entry becomes a 57-bit integer X (four bits more
+//    than a double's significand, so entries down to 1/16 of the largest are
+//    exact) in two limbs X = h 2^28 + l, l in [-2^27, 2^27];
 //  * the tables are rounded on the host to T = th 2^28 + tl, tl in [-2^27, 2^27),
 //    one exponent per table: |T| < 2^56, the projection's, which are the larger
 //    ones, |T| <= 2^58 with the |T| of a sum below 2^61 together (dg_fixed.cu);
 //  * three multiply-adds per product into two 64-bit sums: H += h th, M += h
 //    tl + l th.  At most 63 products meet in one sum (p = 4 with a bed: 3 x 16
-//    area and 15 edge points), so |H| < 2^62 and |M| < 2^63.  The product
-//    l tl is left out: below 2^55 against 2^112 (2^114) of full scale;
+//    area and 15 edge points), so |H| <= 2^62 and |M| < 2^63.  The product
+//    l tl is left out: below 2^54 against 2^113 (2^115) of full scale;
 //  * H + (M >> 28) is the dot product in units of 2^56 of the products' own; it
 //    is normalised and rounded to a double with integer instructions.
-//  The error is the inputs' truncation, at most 2^-55 of the row's largest
-//  entry times max |T| per product: an FP64 dot product rounds each of its
-//  additions at 2^-53 of the running sum.  RMS errors against rational
-//  arithmetic for modes that decay from a mean of 1 to 2, p = 1 to 4 (FP64 FMAs):
-//  area values 1.1, 1.3, 2.0, 2.2e-16 (1.7, 2.7, 3.2, 3.5e-16), traces 1.3, 1.8, 2.3,
-//  3.3e-16 (1.9, 2.4, 3.3, 3.7e-16), the projection of their advection 0.4, 1.0, 1.7,
-//  2.6e-16 (3.6, 4.3, 6.4, 8.0e-16; 8.4e-16 at p = 4 with |T| < 2^56).
+//  RMS errors against rational arithmetic for modes that decay from a mean of 1 to
+//  2, p = 1 to 4 (FP64 FMAs): area values 1.0, 1.2, 1.2, 1.3e-16 (1.7, 2.7, 3.2, 3.5e-16),
+//  traces 1.1, 1.3, 1.2, 1.6e-16 (1.9, 2.4, 3.3, 3.8e-16), the projection of their
+//  advection 0.2, 0.3, 0.5, 0.7e-16 (3.6, 4.3, 6.4, 8.4e-16).  Whole runs against
+//  113-bit arithmetic (10 steps, all equations and schemes): no farther than with
+//  FP64 contractions at p = 1, where the state's own rounding is all, and down to a
+//  fifth of its distance for Euler at p = 4.
 //
 // Layout: a block is 32 elements (one per lane) and one warp per variable, so
 // a row's exponent, limbs and sums stay in one thread, every state row is

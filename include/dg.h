@@ -225,7 +225,7 @@ dg_status dg_set_inflow_series(dg_solver *s, int n, const double *amp, const dou
 
 /* The element stage computes its basis contractions (area values, volume
  * and surface projections, next-stage traces) at p = 1..4 as exact integer
- * slices off the FP64 pipe (56-bit fixed point, per-output error below an
+ * slices off the FP64 pipe (57-bit fixed point, per-output error below an
  * FP64 dot product's rounding).  For Euler at p = 1..4 this can be
  * switched: off, the contractions are FP64 FMAs.  DG_UNSUPPORTED for other
  * equations and orders.  Until it is called a solver takes the slices, the

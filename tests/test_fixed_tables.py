@@ -53,14 +53,13 @@ def test_limbs_reproduce_the_tables_and_no_sum_leaves_64_bits(dglib, p):
         assert a.shape == b.shape
         assert np.abs(a - b).max() <= float(unit(M)) / 2 + 2.0 ** -53 * np.abs(b).max()
     assert np.abs(val["Q"] - val["B"]).max() <= float(unit(max(t["eB"], t["eP"])))
-    X = 2 ** 56 - 1  # the largest input, and its largest limbs
-    xh, xl = X >> LOW, 2 ** LOW - 1
+    xh, xl = 2 ** 29, 2 ** 27  # the largest limbs of the 57-bit inputs
     for T, _ in sums(p, t):
         th, tl = limbs(T)
         assert np.abs(th).max() < 2 ** 31
         H = sum(xh * abs(int(v)) for v in th)
         M = sum(xh * abs(int(v)) for v in tl) + sum(xl * abs(int(v)) for v in th)
-        assert H < 2 ** 62 and M + 2 ** (LOW - 1) < 2 ** 63
+        assert H < 2 ** 62.5 and M + 2 ** (LOW - 1) < 2 ** 63
         assert H + (M >> LOW) < 2 ** 63 - 1
 
 
@@ -69,13 +68,14 @@ def fixed_dot(x, T, M):
     ex = int(np.frexp(np.abs(x).max())[1]) - 1
     H, Mm = 0, 1 << (LOW - 1)
     for v, t in zip(x, T):
-        a = int(abs(Fraction(v)) * Fraction(2) ** (55 - ex))
+        a = int(abs(Fraction(v)) * Fraction(2) ** (56 - ex))
         s = 1 if v >= 0 else -1
-        h, l = s * (a >> LOW), s * (a & (2 ** LOW - 1))
+        h = (a + 2 ** (LOW - 1)) >> LOW
+        h, l = s * h, s * (a - (h << LOW))
         th, tl = limbs(int(t))
         H += h * th
         Mm += h * tl + l * th
-    return float((H + (Mm >> LOW)) * Fraction(2) ** (2 * LOW + ex - 55) * unit(M))
+    return float((H + (Mm >> LOW)) * Fraction(2) ** (2 * LOW + ex - 56) * unit(M))
 
 
 def fp64_dot(x, t):
