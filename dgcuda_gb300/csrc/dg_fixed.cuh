@@ -42,12 +42,12 @@
 // Measured, Euler with the limiter, ms per launch (before: the contractions
 // as f16 digit slices on the tensor cores, 34 MMAs per 7 x 7 digit product on
 // 16 x 8 x 16 blocks of which half is padding): p = 3, 2.1M triangles 5.41 ->
-// 2.72.  The other equations (before: FP64 FMAs), microseconds at 131k triangles
-// (p = 4: 80k; advection 131k), p = 1 to 4: shallow water with a bed 92 -> 40,
-// 268 -> 80, 676 -> 182, 891 -> 223; Maxwell 71 -> 37, 205 -> 65, 527 -> 135, 710
+// 2.80.  The other equations (before: FP64 FMAs), microseconds at 131k triangles
+// (p = 4: 80k; advection 131k), p = 1 to 4: shallow water with a bed 92 -> 39,
+// 268 -> 82, 676 -> 182, 891 -> 225; Maxwell 71 -> 33, 205 -> 62, 527 -> 135, 710
 // -> 164; advection with a velocity field 35 -> 23, 86 -> 37, 206 -> 71, 371 ->
-// 113.  At p = 3 (ncu, 524k) the FP64 pipe -- fluxes, RK combination, limiter --
-// is 58 % busy, the heavy FMA pipe 65 % and the integer ALU 36 %.
+// 114.  At p = 3 (ncu, 524k) the FP64 pipe -- fluxes, RK combination, limiter --
+// is 57 % busy, the heavy FMA pipe 66 % and the integer ALU 38 %.
 #pragma once
 #include "dg_kernels.cuh"
 namespace dg {
@@ -563,13 +563,13 @@ __device__ __forceinline__ void element_tile(const FxTab<P> &tab, const EqP &q, 
 // pipes, until spills cost more.  Measured (Euler p = 3, 2.1M triangles, ms at
 // 4 to 8 blocks): 3.59, 2.93, 2.79, 2.74, 2.78; Euler p = 4 (5 to 8): 1.24,
 // 1.21, 1.27, 1.39; shallow water p = 2, 131k (us at 5 to 12): 93 88 86 86 81 82
-// 80; Maxwell p = 3 (5 to 12): 156 150 138 139 135 135 139; advection p = 3 (14,
-// 18, 24, 32): 79 75 70 72.
+// 80; Maxwell p = 3 (5 to 12): 156 150 138 139 135 135 139; advection p = 3, 131k and
+// 35k (20, 22, 24, 28): 77 71 73 70 and 31.8 31.2 31.6 32.8.
 template <class Eq, int P>
 constexpr int min_blocks() {
   if (Eq::N == 4) return P <= 2 ? 8 : P == 3 ? 7 : 6;
   if (Eq::N == 3) return P <= 2 ? 12 : P == 4 ? 7 : Eq::kBathymetry ? 8 : 9;
-  return P == 1 ? 16 : P == 4 ? 20 : 24;
+  return P == 1 ? 16 : P == 4 ? 20 : P == 3 ? 22 : 24;
 }
 
 template <class Eq, int P, int MODE>
